@@ -18,7 +18,8 @@ LIB_PATH = os.environ.get("FUSEKIT_CUDA_LIB") or os.path.join(_HERE, "libfusekit
  TASK_SDPA_DECODE_QUANT, TASK_EMBED_ROWS, TASK_RESIDUAL_NORM_ROWS, TASK_LINEAR_ROWS, TASK_QK_NORM_STORE_ROWS, TASK_ATTENTION_ROWS,
  TASK_MOE_ROUTE_ROWS, TASK_NORM_LINEAR, TASK_ATTENTION_DECODE, TASK_MOE_UP, TASK_MOE_DOWN, TASK_ARGMAX_ROW, TASK_BLOCK_NORM_ROWS,
  TASK_BLOCK_LINEAR_ROWS, TASK_ROTARY_STORE_ROWS, TASK_WINDOW_ATTENTION_ROWS, TASK_WINDOW_ATTENTION_DECODE, TASK_RECURRENCE_ROWS,
- TASK_RECURRENCE_DECODE, TASK_NORM_GATE_ROWS, TASK_SEGMENT_LINEAR) = range(36)
+ TASK_RECURRENCE_DECODE, TASK_NORM_GATE_ROWS, TASK_SEGMENT_LINEAR, TASK_STAGE_ROWS, TASK_STAGED_LINEAR, TASK_STAGED_GATEUP,
+ TASK_EMBED_PROMPT, TASK_ROPE_STORE_PROMPT, TASK_ARGMAX_PROMPT) = range(42)
 ACT_SWIGLU, ACT_GEGLU_TANH = 0, 1
 ACT_NONE, ACT_RELU_SQUARED, ACT_SILU = 0, 2, 3
 

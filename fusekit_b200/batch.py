@@ -57,6 +57,8 @@ class BatchDecodeEngine:
         self.W: dict[str, int] = {}
         self.V: dict[str, int] = {}
         self.graph = 0
+        self.scratch: dict[str, int] = {}       # of whole prompts (PrefillEngine)
+        self.portions: dict[tuple, object] = {}     # task lists by (rows, last portion)
 
     def x_ptr(self, l): return self.X + l * self.rows * self.spec.hidden * 2
     def hb_ptr(self, l): return self.HB + l * self.rows * self.spec.hidden * 2
@@ -189,12 +191,91 @@ class PrefillEngine(BatchDecodeEngine):
     to fill the caches that engine then decodes from."""
     consecutive = True
 
+    PORTION, HEAD_ROWS = 1024, 256          # positions of a prompt taken together; rows of logits kept while their greedy tokens are found
+
+    @property
+    def _staged(self) -> bool:
+        """Whether prompts longer than a step go through the products of staged rows: not when a kernel was asked for by name, nor for
+        sizes that those do not take."""
+        s = self.spec
+        return self.qmm == 0 and s.head_dim % 64 == 0 and s.vocab % 8 == 0 and s.hidden % 64 == 0 and s.inter % 64 == 0 and max(s.hidden, s.inter, s.n_q * s.head_dim) <= 32768
+
+    def capture(self) -> int:
+        if self._staged and not self.scratch and self.capacity > self.rows:
+            s, P, rt = self.spec, min(self.PORTION, self.capacity), self.rt
+            H, A = s.hidden, s.n_q * s.head_dim
+            self.scratch = {k: rt.alloc(n) for k, n in {
+                "tokens": P * 4, "greedy": P * 4, "x": P * H * 2, "hb": P * H * 2, "qkv": P * self.nqkv * 2, "q": P * A * 2, "att": P * A * 2, "act": P * s.inter * 2,
+                "staged": P * max(-(-k // 512) for k in (H, A, s.inter)) * 1152, "factor": P * 4, "logits": min(P, self.HEAD_ROWS) * s.vocab * 2}.items()}
+        return super().capture()
+
+    def prompt_dispatches(self, rows: int, last: bool) -> list:
+        """One portion of a prompt, positions offset .. offset + rows - 1; with `last` the logits of its last step of `self.rows`
+        positions (counted from the prompt's start: portions before are whole steps) end up where a step leaves them."""
+        s, M, H, hd, I, S, V = self.spec, rows, self.spec.hidden, self.spec.head_dim, self.spec.inter, self.scratch, self.V
+        T, A = N.Task.make, self.spec.n_q * self.spec.head_dim
+
+        def product(l, src, norm, k, weight, n, out, residual=0, one=0, at=0, m=M):
+            return [T(N.TASK_STAGE_ROWS, l, {0: src + at * k * 2, 1: norm, 2: S["staged"], 3: S["factor"]}, [k, m], [s.eps]),
+                    T(N.TASK_STAGED_LINEAR, l, {0: S["staged"], 1: S["factor"], 2: weight, 3: residual, 4: out}, [k, n, m, one])]
+
+        tasks = [T(N.TASK_EMBED_PROMPT, -1, {0: V["embed_tokens"], 1: S["x"], 2: S["tokens"]}, [H, M, s.vocab])]
+        for l in range(s.n_layers):
+            (ck, cv), p = self.cache[l], f"layers.{l}."
+            tasks += product(l, S["x"], V[p + "input_norm"], H, self.W[p + "qkv"], self.nqkv, S["qkv"], V[p + "qkv_bias_rows"], 1)
+            tasks += [T(N.TASK_ROPE_STORE_PROMPT, l, {0: S["qkv"], 1: S["q"], 5: ck, 6: cv}, [s.n_q, s.n_kv, hd, self.capacity, M], [0.0, s.theta]),
+                      T(N.TASK_ATTENTION_ROWS, l, {0: S["q"], 1: ck, 2: cv, 3: S["att"]}, [s.n_q, s.n_kv, hd, hd, self.capacity, M, 1 << 8], [1.0 / math.sqrt(hd)])]
+            tasks += product(l, S["att"], 0, A, self.W[p + "o"], H, S["hb"], S["x"])
+            tasks += [T(N.TASK_STAGE_ROWS, l, {0: S["hb"], 1: V[p + "post_attention_norm"], 2: S["staged"], 3: S["factor"]}, [H, M], [s.eps]),
+                      T(N.TASK_STAGED_GATEUP, l, {0: S["staged"], 1: S["factor"], 2: self.W[p + "gateup"], 4: S["act"]}, [H, I, M, N.ACT_SWIGLU])]
+            tasks += product(l, S["act"], 0, I, self.W[p + "down"], H, S["x"], S["hb"])
+        final = (M - 1) // self.rows * self.rows if last else M
+        for r0 in list(range(0, final, self.HEAD_ROWS)) + ([final] if last else []):
+            m = min(self.HEAD_ROWS, final - r0) if r0 < final else M - final
+            out = S["logits"] if r0 < final else self.logits
+            tasks += product(-1, S["x"], V["final_norm"], H, self.W["lm_head"], s.vocab, out, at=r0, m=m)
+            tasks.append(T(N.TASK_ARGMAX_PROMPT, -1, {0: out, 1: S["greedy"] + r0 * 4}, [s.vocab, m]))
+        return tasks
+
+    def _prompt(self, toks, base_offset: int):
+        """A prompt of more than one step in portions of up to PORTION positions (whole steps but for the last)."""
+        rt, M, n, out = self.rt, self.rows, len(toks), []
+        ids = np.array(toks, np.int64)
+        if ids.min() < 0 or ids.max() >= self.spec.vocab:
+            raise N.FusekitError(f"fk_decode_chunk_rows: token id {int(ids[(ids < 0) | (ids >= self.spec.vocab)][0])} is outside the embedding table ({self.spec.vocab} rows)")
+        ids = ids.astype(np.uint32)
+        most = min(self.PORTION, self.capacity) // M * M
+        for c0 in range(0, n, most):
+            part = ids[c0:c0 + most]
+            key = (len(part), c0 + most >= n)
+            if key not in self.portions:
+                if len(self.portions) > 64:
+                    self.portions.clear()
+                tasks = self.prompt_dispatches(*key)
+                self.portions[key] = (N.Task * len(tasks))(*tasks)
+            arr = self.portions[key]
+            rt.upload(self.scratch["tokens"], part)
+            rt.state_set(0, base_offset + c0)
+            N.check(rt.L.fk_launch_batch(rt.h, arr, len(arr)), "fk_launch_batch")
+            out.append(rt.download(self.scratch["greedy"], (len(part),), np.uint32))
+            err = rt.state_get()[2]
+            if err:
+                raise N.FusekitError(f"device error word {err:#x}")
+        return np.concatenate(out)
+
     def prefill(self, tokens, base_offset: int = 0):
-        """Run `tokens` through the model in chunks of `rows` positions starting at `base_offset`; returns the greedy
-        prediction after every position, [len(tokens)].  A last partial chunk is padded with token 0: the padded rows write
-        cache rows beyond the prompt, which later positions overwrite before anything attends them."""
+        """Run `tokens` through the model from position `base_offset` on; returns the greedy prediction after every position,
+        [len(tokens)].  Up to `rows` tokens are one step, a partial one padded with token 0: the padded rows write cache rows beyond the
+        prompt, which later positions overwrite before anything attends them.  More go through the kernels of whole prompts, which
+        read the weights once per portion instead of once per step, or (see `_staged`) step by step."""
         toks = [int(t) for t in tokens]
         M, preds = self.rows, []
+        if len(toks) > M and self._staged:
+            if base_offset + (len(toks) + M - 1) // M * M > self.capacity:
+                raise ValueError("prefill chunk reaches beyond the cache capacity")
+            if not self.graph:
+                self.capture()
+            return self._prompt(toks, base_offset)
         for c0 in range(0, len(toks), M):
             chunk = toks[c0:c0 + M]
             if base_offset + c0 + M > self.capacity:

@@ -1,12 +1,11 @@
 // Device functions shared by the layered decoders' kernels.
 #pragma once
-#include "fk_common.cuh"
+#include "fk_layers.h"
 #include <math.h>
 
 #define FKL_MAX_EXPERTS 1024
 #define FKL_MAX_TOP 64
 #define FKL_GV_MAX_GROUPS 1024        // groups of a mixer's output norm
-#define FKL_ERR_TOKEN 0x20000u
 #define FKL_ERR_CAPACITY 0x100000u
 #define FKL_ERR_TC_WAIT 0x200000u
 

@@ -72,10 +72,9 @@ static cudaError_t launch_gemv(FklEnv &c, int mode, GemvArgs &a) {
     if (vec && a.k <= 4 * per) return launch(c, k_gemv<FKL_GV_LINEAR, 4>, g, b, smem, c.state, a);
     return launch(c, k_gemv<FKL_GV_LINEAR, 0>, g, b, smem, c.state, a);
 }
-// bf16 rows [rows, k] (row stride ld elements) in boxes of 64 columns x box_rows, 128-byte swizzle
 typedef CUresult (*EncodeTiled)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *, const cuuint32_t *, const cuuint32_t *,
                                 CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-static bool tensor_map(CUtensorMap *m, const void *p, long long rows, long long k, long long ld, int box_rows) {
+bool fkl_tensor_map(CUtensorMap *m, const void *p, long long rows, long long k, long long ld, int box_rows, bool half) {
     static EncodeTiled fn = nullptr;
     if (!fn) {
         void *f = nullptr; cudaDriverEntryPointQueryResult qr;
@@ -84,7 +83,7 @@ static bool tensor_map(CUtensorMap *m, const void *p, long long rows, long long 
     }
     const cuuint64_t dims[2] = {(cuuint64_t)k, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)ld * 2};
     const cuuint32_t box[2] = {FKL_TC_BK, (cuuint32_t)box_rows}, es[2] = {1, 1};
-    return fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (void *)p, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+    return fn(m, half ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (void *)p, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 // the widest tile that still gives (almost) every SM one
@@ -162,7 +161,7 @@ fk_status fkl_run(FklEnv &c, const fk_task &t, char *err, size_t ecap) {
             const long long tiles = mt * ((N + bn - 1) / bn);
             const int grid = tiles < c.sm_count ? (int)tiles : c.sm_count;
             CUtensorMap mx, mw;
-            if (!tensor_map(&mx, (const void *)b[0], M, w.k, ldx, 128) || !tensor_map(&mw, w.rows, w.n, w.k, w.k, bn)) return bad(err, ecap, "linear_rows: tensor map refused");
+            if (!fkl_tensor_map(&mx, (const void *)b[0], M, w.k, ldx, 128) || !fkl_tensor_map(&mw, w.rows, w.n, w.k, w.k, bn)) return bad(err, ecap, "linear_rows: tensor map refused");
             if (block) e = bn == 256 ? launch_tc<256, true>(c, grid, mx, mw, a) : bn == 128 ? launch_tc<128, true>(c, grid, mx, mw, a) : launch_tc<64, true>(c, grid, mx, mw, a);
             else e = bn == 256 ? launch_tc<256, false>(c, grid, mx, mw, a) : bn == 128 ? launch_tc<128, false>(c, grid, mx, mw, a) : launch_tc<64, false>(c, grid, mx, mw, a);
             break;

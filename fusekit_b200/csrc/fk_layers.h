@@ -3,6 +3,9 @@
 #pragma once
 #include "../../include/fusekit_cuda.h"
 #include "fk_common.cuh"
+#include <cuda.h>
+
+#define FKL_ERR_TOKEN 0x20000u
 
 struct FklWeight { const uint16_t *rows; long long n, k; };       // bf16 rows [n, k] as uploaded (fk_weight_keep_rows)
 struct FklEnv {
@@ -15,3 +18,5 @@ fk_status fkl_run(FklEnv &env, const fk_task &t, char *err, size_t cap);
 cudaError_t fkl_init();                                            // shared-memory limits of the kernels, once per context
 fk_status fkb_run(FklEnv &env, const fk_task &t, char *err, size_t cap);      // the kinds of fk_blocks.cu
 cudaError_t fkb_init();
+// 16-bit rows [rows, k] (row stride ld elements) in boxes of 64 columns x box_rows, 128-byte swizzle
+bool fkl_tensor_map(CUtensorMap *m, const void *p, long long rows, long long k, long long ld, int box_rows, bool half = false);

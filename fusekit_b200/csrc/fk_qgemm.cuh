@@ -1,0 +1,498 @@
+// Quantised matrix product on the 5th-generation tensor cores for any number of rows: Y[M, N] = T(X[M, K] . dequant(W)^T + residual)
+// or the gated activation of gate/up pairs, 4-bit weights in the streaming layout (units of 16 rows x 8 groups, fk_stream.cuh).
+//
+// Arithmetic: one pass of kind::f16 (fp16 operands, fp32 accumulation over all of K in tensor memory), with operands that are exact.
+//   * A weight is (q - 8) s + e, e = b + 8 s.  (q - 8) s has 3 + 8 significant bits, fp16's 11; scaled by one power of two per weight
+//     (k_weight_peak: the largest of 16 |s| and |e| lands in [2^14, 2^15)) it is exact for every s down to 2^-28 of that.
+//   * An activation is bf16: 8 bits, exact in fp16 after a power of two per row (k_stage_rows: the row's largest lands in [2^8, 2^9))
+//     for everything down to 2^-25 of the row's largest, rounded to 2^-33 of it below.
+//   * e enters as three extra k slots per group, (e_hi, e_hi, e_lo) . (X_hi, X_lo, X_hi), X the sum of the group's activations: 22 bits
+//     of both, a fourth slot is zero.  A super-block of 8 groups is 8 k-blocks of 64 slots and one of 32.
+// Scales inside the operand leave nothing to do per group after the product: accumulators stay in tensor memory until a tile is done.
+//
+// A block owns 256 weight rows (two M = 128 accumulators) x BN rows of X.  16 warps turn one unit each (16 weight rows) into fp16
+// and write it straight into tensor memory as the A operand (tcgen05.st .16x256b: the lane layout of the units is its lane layout; a ring
+// of four k-blocks); through shared memory the expanded operand costs two more crossings of it than the packed weights.  One warp
+// fetches X by TMA (128-byte swizzle), one thread issues the MMAs, 8 warps store finished tiles.  Weight rings are filled before
+// griddepcontrol.wait.  Every wait is bounded; when one runs out the kernel sets an error bit, waits (bounded) for its copies, frees
+// its tensor memory and returns.
+//
+// Work split: `whole` = tiles dealt whole in turn, else all (tile, super-block) steps dealt in equal runs; a run that covers part of a
+// tile leaves fp32 sums in the scratch area, and of the warps that hold the same rows the last to arrive adds the parts in K order.
+#pragma once
+#include "fk_stream.cuh"
+#include "fk_layers.h"
+#include <cuda_fp16.h>
+
+#define FKQ_SB 576                      // staged halves per super-block: 512 activations, 32 slots for the sums, 32 unused
+#define FKQ_DEQ 16                      // dequantising warps: one unit each
+#define FKQ_EPI 8                       // storing warps
+#define FKQ_THREADS ((FKQ_DEQ + FKQ_EPI + 2) * 32)
+#define FKQ_ROWS 256                    // weight rows of a block
+#define FKQ_AS 4                        // k-blocks of A operand in tensor memory (64 columns each)
+#define FKQ_SPIN (1u << 21)
+#define FKQ_MAX_K 32768                 // a row is staged from registers: 1024 threads x 4 vectors of 8
+#define FKQ_ERR_WAIT 0x400000u
+#define FKQ_COUNTERS 65536              // ticket words: 8 per tile that is split
+template <int BN> struct QgTile {
+    static constexpr int XS = BN >= 128 ? 4 : BN == 64 ? 8 : 12, XBYTES = BN * 128, NBUF = BN <= 64 ? 2 : 1;
+    static constexpr size_t SMEM = 1024 + (size_t)XS * XBYTES + (size_t)FKQ_DEQ * FK_STAGES * FK_UNIT_BYTES;
+};
+__host__ __device__ inline size_t fkq_part_floats(int bn) { return (size_t)bn * FKQ_ROWS; }
+
+struct QGemmArgs { TiledW W; const float *xscale; const uint16_t *residual; uint16_t *y; float *scratch; unsigned int *counters; int m, n, ldr, act, whole, mtiles, tiles; float wmul, wscale; };
+
+__device__ __forceinline__ bool qg_wait(uint32_t bar, uint32_t parity) {
+    for (uint32_t i = 0; i < FKQ_SPIN; ++i) {
+        uint32_t ok;
+        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+        if (ok) return true;
+    }
+    return false;
+}
+__device__ __forceinline__ void qg_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
+__device__ __forceinline__ void qg_expect(uint32_t bar, uint32_t bytes) { asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory"); }
+__device__ __forceinline__ void qg_commit(uint32_t bar) { asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory"); }
+__device__ __forceinline__ uint32_t h2_sub(uint32_t a, uint32_t b) { __half2 r = __hsub2(*reinterpret_cast<__half2 *>(&a), *reinterpret_cast<__half2 *>(&b)); return *reinterpret_cast<uint32_t *>(&r); }
+__device__ __forceinline__ uint32_t h2_mul(uint32_t a, uint32_t b) { __half2 r = __hmul2(*reinterpret_cast<__half2 *>(&a), *reinterpret_cast<__half2 *>(&b)); return *reinterpret_cast<uint32_t *>(&r); }
+__device__ __forceinline__ uint32_t h2_pack(float lo, float hi) { __half2 r = __floats2half2_rn(lo, hi); return *reinterpret_cast<uint32_t *>(&r); }
+__device__ __forceinline__ void qg_st16(uint32_t addr, const uint32_t (&r)[16]) {
+    asm volatile("tcgen05.st.sync.aligned.16x256b.x4.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+                 ::"r"(addr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+                   "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
+}
+__device__ __forceinline__ void qg_ld16(uint32_t (&d)[16], uint32_t addr) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+                 : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]), "=r"(d[4]), "=r"(d[5]), "=r"(d[6]), "=r"(d[7]),
+                   "=r"(d[8]), "=r"(d[9]), "=r"(d[10]), "=r"(d[11]), "=r"(d[12]), "=r"(d[13]), "=r"(d[14]), "=r"(d[15]) : "r"(addr) : "memory");
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
+// The v-th piece of work of block `b` of `G`: super-blocks [k0, k1) of a tile.
+struct QWork { int tile, k0, k1; };
+__host__ __device__ inline bool fkq_work(int whole, int tiles, int nsb, int b, int G, int v, QWork &w) {
+    if (whole) { w.tile = b + v * G; w.k0 = 0; w.k1 = nsb; return w.tile < tiles; }
+    const long long T = (long long)tiles * nsb;
+    const int s0 = (int)(b * T / G), s1 = (int)((b + 1) * T / G);
+    w.tile = s0 / nsb + v;
+    const int t0 = w.tile * nsb, a = s0 > t0 ? s0 : t0, e = s1 < t0 + nsb ? s1 : t0 + nsb;
+    if (w.tile >= tiles || a >= e) return false;
+    w.k0 = a - t0; w.k1 = e - t0;
+    return true;
+}
+// the block whose run holds step s, and the scratch slot of block b's part of `tile` (two slots a block: the tile its run begins in, the one it ends in)
+__host__ __device__ inline int fkq_owner(int tiles, int nsb, int G, int s) { return (int)((((long long)s + 1) * G - 1) / ((long long)tiles * nsb)); }
+__host__ __device__ inline int fkq_slot(int tiles, int nsb, int G, int b, int tile) { return 2 * b + ((int)((long long)b * tiles * nsb / G) / nsb == tile ? 0 : 1); }
+
+// Rows of X per tile, blocks and split of a product of m rows: the widest tile that the rows fill; up to 32 rows the steps are dealt in
+// equal runs (a part's sums are small, and the product is bound by the weights), from 33 on only while less than half of the blocks have a tile.
+struct QPlan { int bn, mtiles, tiles, grid, whole; };
+inline QPlan fkq_plan(int m, int ntiles, int nsb, int sm) {
+    QPlan p;
+    p.bn = m <= 16 ? 16 : m <= 32 ? 32 : m <= 64 ? 64 : 128;
+    p.mtiles = (m + p.bn - 1) / p.bn; p.tiles = (ntiles + 15) / 16 * p.mtiles; p.whole = 1; p.grid = p.tiles < sm ? p.tiles : sm;
+    if (p.tiles > FKQ_COUNTERS / FKQ_EPI) return p;
+    if (p.bn <= 32) {
+        if (p.tiles % sm) { const long long steps = (long long)p.tiles * nsb; p.whole = 0; p.grid = steps < sm ? (int)steps : sm; }
+    } else if (2 * p.tiles <= sm && nsb > 1) {
+        const int parts = sm / p.tiles < nsb ? sm / p.tiles : nsb;
+        p.whole = 0; p.grid = p.tiles * parts;
+    }
+    return p;
+}
+
+template <int BN, bool GATEUP>
+__global__ void __launch_bounds__(FKQ_THREADS, 1) k_qgemm(FkState *st, const __grid_constant__ CUtensorMap mx, QGemmArgs a) {
+    using T = QgTile<BN>;
+    constexpr int XS = T::XS, NBUF = T::NBUF;
+    extern __shared__ unsigned char qg_smem[];
+    __shared__ __align__(8) uint64_t bars[FKQ_DEQ * FK_STAGES + 2 * XS + 2 * FKQ_AS + 2 * NBUF];
+    __shared__ uint32_t tmem_slot;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const uint32_t base = (smem_u32(qg_smem) + 1023u) & ~1023u, ring = base + XS * T::XBYTES;
+    const uint32_t wfull = smem_u32(bars), xfull = wfull + 8 * FKQ_DEQ * FK_STAGES, xempty = xfull + 8 * XS, afull = xempty + 8 * XS, aempty = afull + 8 * FKQ_AS,
+                   dfull = aempty + 8 * FKQ_AS, dempty = dfull + 8 * NBUF;
+    pdl_launch_dependents();
+    if (tid == 0) {
+        for (int i = 0; i < FKQ_DEQ * FK_STAGES; ++i) mbar_init(bars + i, 1);
+        uint64_t *b = bars + FKQ_DEQ * FK_STAGES;
+        for (int i = 0; i < 2 * XS; ++i) mbar_init(b + i, 1);
+        b += 2 * XS;
+        for (int i = 0; i < FKQ_AS; ++i) { mbar_init(b + i, FKQ_DEQ); mbar_init(b + FKQ_AS + i, 1); }
+        b += 2 * FKQ_AS;
+        for (int i = 0; i < NBUF; ++i) { mbar_init(b + i, 1); mbar_init(b + NBUF + i, FKQ_EPI); }
+        mbar_fence_init();
+    }
+    if (wid == FKQ_DEQ) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(512u) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = tmem_slot, tmem_a = tmem + 256;
+    const int nsb = a.W.nsb, G = gridDim.x, me = blockIdx.x;
+    bool ok = true;
+    QWork w;
+    if (wid < FKQ_DEQ) {
+        // ---------------------------------------------------------------- weights: packed ring -> fp16 in tensor memory
+        const int q = wid & 3, sub = wid >> 3, half = (wid >> 2) & 1, mine = sub * 8 + q * 2 + half;
+        const uint32_t bar0 = wfull + 8 * FK_STAGES * wid, ring0 = ring + (uint32_t)(wid * FK_STAGES * FK_UNIT_BYTES);
+        const uint32_t dst0 = tmem_a + ((uint32_t)(32 * q + 16 * half) << 16) + (uint32_t)(sub * 32);
+        int iv = 0, ikb = 0, issued = 0, used = 0, it = 0;
+        QWork iw; bool more = fkq_work(a.whole, a.tiles, nsb, me, G, 0, iw);
+        ikb = more ? iw.k0 : 0;
+        // the next unit of this warp in the block's order of steps (tiles past the last row tile have none)
+        auto issue = [&]() {
+            while (more && (iw.tile / a.mtiles) * 16 + mine >= a.W.ntiles) { more = fkq_work(a.whole, a.tiles, nsb, me, G, ++iv, iw); ikb = more ? iw.k0 : 0; }
+            if (!more) return;
+            if (lane == 0) {
+                const int s = issued & (FK_STAGES - 1);
+                qg_expect(bar0 + 8 * s, FK_UNIT_BYTES);
+                asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                             ::"r"(ring0 + (uint32_t)(s * FK_UNIT_BYTES)), "l"(a.W.units + ((size_t)((iw.tile / a.mtiles) * 16 + mine) * nsb + ikb) * FK_UNIT_VEC),
+                               "r"((uint32_t)FK_UNIT_BYTES), "r"(bar0 + 8 * s) : "memory");
+            }
+            ++issued;
+            if (++ikb == iw.k1) { more = fkq_work(a.whole, a.tiles, nsb, me, G, ++iv, iw); ikb = more ? iw.k0 : 0; }
+        };
+        for (int s = 0; s < FK_STAGES; ++s) issue();
+        auto slot = [&]() {                             // the next A stage is free
+            if (it >= FKQ_AS && !qg_wait(aempty + 8 * (it % FKQ_AS), (uint32_t)(it / FKQ_AS - 1) & 1u)) { ok = false; return false; }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            return true;
+        };
+        auto publish = [&]() {
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) qg_arrive(afull + 8 * (it % FKQ_AS));
+            ++it;
+        };
+        for (int v = 0; ok && fkq_work(a.whole, a.tiles, nsb, me, G, v, w); ++v) {
+            const bool have = (w.tile / a.mtiles) * 16 + mine < a.W.ntiles;
+            for (int kb = w.k0; kb < w.k1 && ok; ++kb) {
+                const int s = used & (FK_STAGES - 1);
+                if (have && !qg_wait(bar0 + 8 * s, (uint32_t)(used / FK_STAGES) & 1u)) { ok = false; break; }
+                const uint32_t u = ring0 + (uint32_t)(s * FK_UNIT_BYTES);
+                // scales and biases of rows g and g + 8, groups 2t and 2t + 1
+                uint4 sb = make_uint4(0, 0, 0, 0);
+                if (have) sb = lds128(u + 4096 + (uint32_t)lane * 16u);
+                const float s0 = bf_lo(sb.x) * a.wmul, s1 = bf_hi(sb.x) * a.wmul, s8 = bf_lo(sb.y) * a.wmul, s9 = bf_hi(sb.y) * a.wmul;
+                const uint32_t pg = h2_pack(s0, s1), pg8 = h2_pack(s8, s9);
+#pragma unroll 2
+                for (int j = 0; j < 8; ++j) {
+                    uint4 p = make_uint4(0, 0, 0, 0);
+                    if (have) p = lds128(u + (uint32_t)(j * 512 + lane * 16));
+                    const int src = (lane & ~3) | (j >> 1);
+                    const uint32_t c = __shfl_sync(0xffffffffu, pg, src), c8 = __shfl_sync(0xffffffffu, pg8, src);
+                    const uint32_t sel = (j & 1) ? 0x3232u : 0x1010u, sg = __byte_perm(c, c, sel), sg8 = __byte_perm(c8, c8, sel);
+                    const uint32_t hg = h2_mul(sg, 0x2C002C00u), hg8 = h2_mul(sg8, 0x2C002C00u);      // scale / 16: odd nibbles stay at their place
+                    uint32_t r[16];
+                    auto expand = [&](uint32_t word, uint32_t sc, uint32_t sc16, int i) {            // pairs (0,4) (1,5) | (2,6) (3,7)
+                        const uint32_t hi = word >> 8;
+                        r[i] = h2_mul(h2_sub((word & 0x000F000Fu) | 0x64006400u, 0x64086408u), sc);
+                        r[i + 1] = h2_mul(h2_sub((word & 0x00F000F0u) | 0x64006400u, 0x64806480u), sc16);
+                        r[i + 4] = h2_mul(h2_sub((hi & 0x000F000Fu) | 0x64006400u, 0x64086408u), sc);
+                        r[i + 5] = h2_mul(h2_sub((hi & 0x00F000F0u) | 0x64006400u, 0x64806480u), sc16);
+                    };
+                    expand(p.x, sg, hg, 0); expand(p.z, sg8, hg8, 2); expand(p.y, sg, hg, 8); expand(p.w, sg8, hg8, 10);
+                    if (!slot()) break;
+                    qg_st16(dst0 + (uint32_t)((it % FKQ_AS) * 64), r);
+                    publish();
+                }
+                if (!ok) break;
+                {                                       // the sums' slots: columns 8b + 2t (e_hi, e_hi) and 8b + 2t + 1 (e_lo, 0) of group 2t + b
+                    uint32_t r[8];
+                    auto edge = [&](float e, uint32_t &hi, uint32_t &lo) {
+                        const float h = __half2float(__float2half_rn(e));
+                        hi = h2_pack(h, h); lo = h2_pack(e - h, 0.0f);
+                    };
+                    edge(fmaf(bf_lo(sb.z), a.wmul, 8.0f * s0), r[0], r[1]); edge(fmaf(bf_lo(sb.w), a.wmul, 8.0f * s8), r[2], r[3]);
+                    edge(fmaf(bf_hi(sb.z), a.wmul, 8.0f * s1), r[4], r[5]); edge(fmaf(bf_hi(sb.w), a.wmul, 8.0f * s9), r[6], r[7]);
+                    if (!slot()) break;
+                    asm volatile("tcgen05.st.sync.aligned.16x256b.x2.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
+                                 ::"r"(dst0 + (uint32_t)((it % FKQ_AS) * 64)), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
+                    publish();
+                }
+                if (have) { ++used; __syncwarp(); issue(); }
+            }
+        }
+        // what is still in flight lands, and the MMAs that read the last stages have been counted, before the block may leave
+        for (; used < issued; ++used) if (!qg_wait(bar0 + 8 * (used & (FK_STAGES - 1)), (uint32_t)(used / FK_STAGES) & 1u)) ok = false;
+        if (ok) for (int j = it > FKQ_AS ? it - FKQ_AS : 0; j < it; ++j) if (!qg_wait(aempty + 8 * (j % FKQ_AS), (uint32_t)(j / FKQ_AS) & 1u)) ok = false;
+        if (!ok && lane == 0) atomicOr(&st->error, FKQ_ERR_WAIT);
+    } else if (wid == FKQ_DEQ + FKQ_EPI) {
+        // ---------------------------------------------------------------- X
+        pdl_wait();
+        if (lane == 0) {
+            int it = 0;
+            for (int v = 0; ok && fkq_work(a.whole, a.tiles, nsb, me, G, v, w); ++v) {
+                const int m0 = (w.tile % a.mtiles) * BN;
+                for (int kb = w.k0 * 9; kb < w.k1 * 9; ++kb, ++it) {
+                    const int s = it % XS;
+                    if (it >= XS && !qg_wait(xempty + 8 * s, (uint32_t)(it / XS - 1) & 1u)) { ok = false; break; }
+                    qg_expect(xfull + 8 * s, (uint32_t)T::XBYTES);
+                    asm volatile("cp.async.bulk.tensor.2d.shared::cta.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+                                 ::"r"(base + s * T::XBYTES), "l"(&mx), "r"(kb * 64), "r"(m0), "r"(xfull + 8 * s) : "memory");
+                }
+            }
+            for (int j = it > XS ? it - XS : 0; j < it; ++j) if (!qg_wait((ok ? xempty : xfull) + 8 * (j % XS), (uint32_t)(j / XS) & 1u)) ok = false;
+            if (!ok) atomicOr(&st->error, FKQ_ERR_WAIT);
+        }
+    } else if (wid == FKQ_DEQ + FKQ_EPI + 1) {
+        // ---------------------------------------------------------------- MMA issue
+        pdl_wait();
+        if (lane == 0) {
+            const uint32_t idesc = (1u << 4) | ((uint32_t)(BN >> 3) << 17) | ((128u >> 4) << 24);          // fp16 x fp16 -> fp32
+            int it = 0;
+            for (int v = 0; ok && fkq_work(a.whole, a.tiles, nsb, me, G, v, w); ++v) {
+                const int d = v % NBUF, steps = (w.k1 - w.k0) * 9;
+                if (v >= NBUF && !qg_wait(dempty + 8 * d, (uint32_t)(v / NBUF - 1) & 1u)) { ok = false; break; }
+                int kk = 0;
+                for (int kb = 0; kb < steps; ++kb, ++it) {
+                    const int s = it % XS, as = it % FKQ_AS;
+                    if (!qg_wait(xfull + 8 * s, (uint32_t)(it / XS) & 1u) || !qg_wait(afull + 8 * as, (uint32_t)(it / FKQ_AS) & 1u)) { ok = false; break; }
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const uint32_t xb = base + s * T::XBYTES;
+                    const uint64_t db = (uint64_t)((xb >> 4) & 0x3FFFu) | (1ull << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
+                    const int nk = kk == 8 ? 2 : 4;
+                    kk = kk == 8 ? 0 : kk + 1;
+#pragma unroll
+                    for (int sub = 0; sub < 2; ++sub)
+#pragma unroll
+                        for (int k = 0; k < 4; ++k)
+                            if (k < nk)
+                                asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+                                             ::"r"(tmem + (uint32_t)((d * 2 + sub) * BN)), "r"(tmem_a + (uint32_t)(as * 64 + sub * 32 + k * 8)), "l"(db + (uint64_t)(k * 2)),
+                                               "r"(idesc), "r"(kb | k) : "memory");
+                    qg_commit(aempty + 8 * as); qg_commit(xempty + 8 * s);
+                }
+                if (ok) qg_commit(dfull + 8 * d);
+            }
+            if (!ok) atomicOr(&st->error, FKQ_ERR_WAIT);
+        }
+    } else {
+        // ---------------------------------------------------------------- finished tiles: lane = weight row, registers = rows of X
+        pdl_wait();
+        const int ew = wid - FKQ_DEQ, q = ew & 3, sub = ew >> 2;
+        for (int v = 0; ok && fkq_work(a.whole, a.tiles, nsb, me, G, v, w); ++v) {
+            const int d = v % NBUF, rt = w.tile / a.mtiles, m0 = (w.tile - rt * a.mtiles) * BN, row0 = rt * FKQ_ROWS + sub * 128 + q * 32;
+            if (!qg_wait(dfull + 8 * d, (uint32_t)(v / NBUF) & 1u)) { ok = false; break; }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t src = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)((d * 2 + sub) * BN);
+            const bool part = w.k0 != 0 || w.k1 != nsb;
+            bool finish = !part;
+            int first = 0, last = 0;
+            if (part) {
+                float *mine = a.scratch + (size_t)fkq_slot(a.tiles, nsb, G, me, w.tile) * fkq_part_floats(BN) + sub * 128 + q * 32 + lane;
+#pragma unroll 1
+                for (int c = 0; c < BN; c += 16) {
+                    uint32_t r[16]; qg_ld16(r, src + (uint32_t)c);
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) __stcg(mine + (size_t)(c + i) * FKQ_ROWS, __uint_as_float(r[i]));
+                }
+                first = fkq_owner(a.tiles, nsb, G, w.tile * nsb); last = fkq_owner(a.tiles, nsb, G, (w.tile + 1) * nsb - 1);
+                __threadfence();
+                __syncwarp();
+                unsigned int ticket = 0;
+                if (lane == 0) {
+                    ticket = atomicAdd(a.counters + (size_t)w.tile * FKQ_EPI + ew, 1u);
+                    if (ticket == (unsigned int)(last - first)) a.counters[(size_t)w.tile * FKQ_EPI + ew] = 0u;      // all parts are in: ready for the next launch
+                }
+                finish = __shfl_sync(0xffffffffu, ticket, 0) == (unsigned int)(last - first);
+                __threadfence();
+            }
+            if (finish) {
+#pragma unroll 1
+                for (int c = 0; c < BN && m0 + c < a.m; c += 16) {
+                    float acc[16];
+                    if (!part) {
+                        uint32_t r[16]; qg_ld16(r, src + (uint32_t)c);
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) acc[i] = __uint_as_float(r[i]);
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) acc[i] = 0.0f;
+                        for (int p = first; p <= last; ++p) {
+                            const float *from = a.scratch + (size_t)fkq_slot(a.tiles, nsb, G, p, w.tile) * fkq_part_floats(BN) + sub * 128 + q * 32 + lane;
+#pragma unroll
+                            for (int i = 0; i < 16; ++i) acc[i] += __ldcg(from + (size_t)(c + i) * FKQ_ROWS);
+                        }
+                    }
+                    const float xs = lane < 16 && m0 + c + lane < a.m ? __ldcg(a.xscale + m0 + c + lane) * a.wscale : 0.0f;
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) acc[i] *= __shfl_sync(0xffffffffu, xs, i);
+                    if (GATEUP) {
+                        // lanes 0-7 / 16-23 hold gate rows, 8-15 / 24-31 the up rows of the same outputs: the lower half takes the even row of X of a
+                        // pair, the upper half the odd one
+                        const bool up = lane & 8;
+                        const int out = (row0 >> 4) * 8 + (lane >> 4) * 8 + (lane & 7);
+#pragma unroll
+                        for (int i = 0; i < 16; i += 2) {
+                            const float other = __shfl_xor_sync(0xffffffffu, up ? acc[i] : acc[i + 1], 8);
+                            const float gate = up ? other : acc[i], upv = up ? acc[i + 1] : other;
+                            const int m = m0 + c + i + (up ? 1 : 0);
+                            if (m < a.m && out < a.n) a.y[(size_t)m * a.n + out] = a.act == 1 ? s_act_geglu(gate, upv) : s_act_swiglu(gate, upv);
+                        }
+                    } else {
+                        const int n = row0 + lane;
+                        if (n < a.n) {
+                            if (a.residual) {
+                                uint16_t r[16];
+#pragma unroll
+                                for (int i = 0; i < 16; ++i) r[i] = m0 + c + i < a.m ? __ldcg(a.residual + (size_t)(m0 + c + i) * a.ldr + n) : (uint16_t)0;
+#pragma unroll
+                                for (int i = 0; i < 16; ++i) acc[i] += bf2f(r[i]);
+                            }
+#pragma unroll
+                            for (int i = 0; i < 16; ++i) if (m0 + c + i < a.m) a.y[(size_t)(m0 + c + i) * a.n + n] = f2bf(acc[i]);
+                        }
+                    }
+                    __syncwarp();
+                }
+            }
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) qg_arrive(dempty + 8 * d);
+        }
+        if (!ok && lane == 0) atomicOr(&st->error, FKQ_ERR_WAIT);
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (wid == FKQ_DEQ) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
+}
+
+// The largest of 16 |s| and |b + 8 s| of a weight (non-finite ones left out), as the bits of a non-negative float: what its common
+// power of two is chosen from.  Once per weight, when it is laid out.
+__global__ void k_weight_peak(const uint4 *units, long long nunits, unsigned int *peak) {
+    float top = 0.0f;
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nunits * 32; i += (long long)gridDim.x * blockDim.x) {
+        const uint4 v = units[(i >> 5) * FK_UNIT_VEC + 256 + (i & 31)];
+        const uint32_t s[2] = {v.x, v.y}, b[2] = {v.z, v.w};
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const float c[4] = {16.0f * fabsf(bf_lo(s[h])), 16.0f * fabsf(bf_hi(s[h])), fabsf(fmaf(8.0f, bf_lo(s[h]), bf_lo(b[h]))), fabsf(fmaf(8.0f, bf_hi(s[h]), bf_hi(b[h])))};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) if (c[j] <= 3.0e38f) top = fmaxf(top, c[j]);
+        }
+    }
+    top = warp_max(top);
+    if ((threadIdx.x & 31) == 0) atomicMax(peak, __float_as_uint(top));
+}
+
+// Rows of X as the product reads them: fp16 scaled by a power of two per row, in the k order in which the nibble pairs come out of
+// their words (slot 16 b + 4 t + 2 h + e of a group is k = 32 (b / 2) + 8 t + 2 (b & 1) + h + 4 e), the group sums after every 8 groups;
+// optionally normalised first (the two roundings of the one-row kernels).  A block per row, the row in registers: bound by the
+// latency of one pass over it.
+struct StageRowsArgs { const uint16_t *x, *w; __half *out; float *scale; int k, nsb; float eps; };
+template <int NT>
+__global__ void __launch_bounds__(NT) k_stage_rows(const FkState *st, StageRowsArgs a) {
+    __shared__ float red[40];
+    const int tid = threadIdx.x, row = blockIdx.x, chunks = a.nsb * 64;
+    constexpr int NV = 4;
+    uint4 x[NV];
+    pdl_wait(); pdl_launch_dependents();
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+        const int c = v * NT + tid;
+        x[v] = c * 8 < a.k ? __ldcg(reinterpret_cast<const uint4 *>(a.x + (size_t)row * a.k) + c) : make_uint4(0, 0, 0, 0);
+    }
+    if (a.w) {
+        float ss = 0.0f;
+#pragma unroll
+        for (int v = 0; v < NV; ++v) {
+            float f[8]; unpack8(x[v], f);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) ss = fmaf(f[j], f[j], ss);
+        }
+        const float r = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(block_sum(ss, red), (float)a.k), a.eps)));
+#pragma unroll
+        for (int v = 0; v < NV; ++v) {
+            const int c = v * NT + tid;
+            if (c * 8 >= a.k) continue;
+            const uint4 wv = __ldg(reinterpret_cast<const uint4 *>(a.w) + c);
+            float f[8], n[8]; unpack8(x[v], f); unpack8(wv, n);
+            uint32_t o[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) o[j] = (uint32_t)f2bf(n[2 * j] * rT(f[2 * j] * r)) | ((uint32_t)f2bf(n[2 * j + 1] * rT(f[2 * j + 1] * r)) << 16);
+            x[v] = make_uint4(o[0], o[1], o[2], o[3]);
+        }
+    }
+    uint32_t top = 0;                                   // largest magnitude as bf16 bits; infinities and NaN do not set the scale
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+        const uint32_t h[4] = {x[v].x, x[v].y, x[v].z, x[v].w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const uint32_t lo = h[j] & 0x7fffu, hi = (h[j] >> 16) & 0x7fffu;
+            if (lo < 0x7f80u && lo > top) top = lo;
+            if (hi < 0x7f80u && hi > top) top = hi;
+        }
+    }
+    top = __reduce_max_sync(0xffffffffu, top);
+    __syncthreads();
+    if ((tid & 31) == 0) red[tid >> 5] = __uint_as_float(top);
+    __syncthreads();
+    top = 0;
+#pragma unroll
+    for (int i = 0; i < NT / 32; ++i) top = max(top, __float_as_uint(red[i]));
+    int e = top ? (int)(top >> 7) - 127 : 8;
+    if (e < -118) e = -118;                             // the factor and its inverse stay normal numbers
+    const float mul = __uint_as_float((uint32_t)(127 + 8 - e) << 23);
+    if (tid == 0) a.scale[row] = __uint_as_float((uint32_t)(127 - 8 + e) << 23);
+    __half *out = a.out + (size_t)row * a.nsb * FKQ_SB;
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+        const int c = v * NT + tid;
+        if (c >= chunks) break;                         // chunks is a multiple of 64: uniform over a warp
+        float f[8]; unpack8(x[v], f);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) f[j] *= mul;
+        float sum = ((f[0] + f[1]) + (f[2] + f[3])) + ((f[4] + f[5]) + (f[6] + f[7]));
+        sum += __shfl_xor_sync(0xffffffffu, sum, 1); sum += __shfl_xor_sync(0xffffffffu, sum, 2); sum += __shfl_xor_sync(0xffffffffu, sum, 4);
+        const int cc = c & 63, j = cc >> 3, b = (cc >> 2) & 1, t = cc & 3;
+        __half *block = out + (size_t)(c >> 6) * FKQ_SB, *dst = block + j * 64 + 32 * b + 4 * t;
+        *reinterpret_cast<uint2 *>(dst) = make_uint2(h2_pack(f[0], f[4]), h2_pack(f[1], f[5]));
+        *reinterpret_cast<uint2 *>(dst + 16) = make_uint2(h2_pack(f[2], f[6]), h2_pack(f[3], f[7]));
+        if ((cc & 7) == 0) {
+            const float hi = __half2float(__float2half_rn(sum));
+            *reinterpret_cast<uint2 *>(block + 512 + 16 * (j & 1) + 4 * (j >> 1)) = make_uint2(h2_pack(hi, sum - hi), h2_pack(hi, 0.0f));
+        }
+    }
+}
+
+// ---------------------------------------------------------------- the other kernels of a prompt
+struct EmbedPromptArgs { const uint16_t *table; uint16_t *x; const uint32_t *tokens; int h, vocab; };
+__global__ void __launch_bounds__(256) k_embed_prompt(FkState *st, EmbedPromptArgs a) {        // rows of h (a multiple of 8) values
+    pdl_wait(); pdl_launch_dependents();
+    uint32_t tok = __ldcg(a.tokens + blockIdx.x);
+    if (tok >= (uint32_t)a.vocab) { if (threadIdx.x == 0) atomicOr(&st->error, FKL_ERR_TOKEN); tok = 0; }
+    const uint4 *src = reinterpret_cast<const uint4 *>(a.table + (size_t)tok * a.h);
+    uint4 *dst = reinterpret_cast<uint4 *>(a.x + (size_t)blockIdx.x * a.h);
+    for (int i = threadIdx.x; i < a.h / 8; i += blockDim.x) dst[i] = __ldg(src + i);
+}
+// greedy token after every row, ties to the lowest index; eight logits per load (v a multiple of 8)
+__global__ void __launch_bounds__(512) k_argmax_prompt(const FkState *st, const uint16_t *logits, uint32_t *out, int v) {
+    __shared__ unsigned long long best_of[16];
+    pdl_wait(); pdl_launch_dependents();
+    const uint4 *lg = reinterpret_cast<const uint4 *>(logits + (size_t)blockIdx.x * v);
+    unsigned long long best = 0ull;
+    for (int i = threadIdx.x; i < v / 8; i += blockDim.x) {
+        const uint4 p = __ldcg(lg + i);
+        const uint32_t h[4] = {p.x, p.y, p.z, p.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const unsigned long long k0 = argmax_key((uint16_t)(h[j] & 0xffffu), (uint32_t)(i * 8 + 2 * j)), k1 = argmax_key((uint16_t)(h[j] >> 16), (uint32_t)(i * 8 + 2 * j + 1));
+            best = k0 > best ? k0 : best; best = k1 > best ? k1 : best;
+        }
+    }
+    best = warp_max_u64(best);
+    if ((threadIdx.x & 31) == 0) best_of[threadIdx.x >> 5] = best;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int i = 1; i < (int)(blockDim.x >> 5); ++i) best = best_of[i] > best ? best_of[i] : best;
+        out[blockIdx.x] = 0xffffffffu - (uint32_t)(best & 0xffffffffull);
+    }
+}

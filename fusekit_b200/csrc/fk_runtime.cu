@@ -10,6 +10,7 @@
 #include "fk_qmm_tc.cuh"
 #include "fk_json.h"
 #include "fk_layers.h"
+#include "fk_qgemm.cuh"
 #include <chrono>
 #include <thread>
 
@@ -72,6 +73,7 @@ struct Weight {
     // tiled layout (fk_stream.cuh): set by fk_weight_finalize / fk_weight_pair for 4- and 8-bit weights
     bool tiled = false; uint4 *units = nullptr; int ntiles = 0, nsb = 0; size_t unit_bytes = 0;
     int rows_kind = FK_ROWS_PLAIN, hd = 0, n_rot = 0;
+    float peak = 0.0f;                          // 4-bit streaming layout: what the fp16 operand's power of two is chosen from (k_weight_peak)
     WView view() const { WView v; v.w = w; v.s = s; v.b = b; v.n = n; v.k = k; v.bits = bits; return v; }
     TiledW tview() const { TiledW t; t.units = units; t.ntiles = ntiles; t.nsb = nsb; t.n = (int)n; t.k = (int)k; t.bits = bits;
                            t.rows_kind = rows_kind; t.hd = hd; t.n_rot = n_rot; return t; }
@@ -88,6 +90,7 @@ struct Ctx {
     uint32_t *pinned = nullptr;                 // host staging for state / history
     std::vector<Weight> weights; std::vector<Graph> graphs; std::vector<void *> allocs;
     bool pending = false; bool pdl = true; int sm_count = 148;
+    float *qg_scratch = nullptr; unsigned int *qg_counters = nullptr; unsigned int *qg_peak = nullptr;      // of the staged products
     float *qmm_scratch = nullptr; unsigned int *qmm_counters = nullptr;   // K-split partial sums and tickets of the several-row projection
     bool use_tiled = true; int stages = FK_STAGES; int force_warps = 0; int force_split = -1; bool qmm_tc = false; int wide_upto = 3; bool sdpa_cluster = true; bool sdpa_mma = true; int sdpa_cl = 0;
     ncclComm_t comm = nullptr; int rank = 0, world = 1;
@@ -136,6 +139,9 @@ extern "C" fk_status fk_open(int device, fk_handle *out) {
     c->hist_cap = FK_HIST_CAP;
     CU(cudaMalloc(&c->qmm_scratch, sizeof(float) * 2 * c->sm_count * FK_QMM_PART_FLOATS));
     CU(cudaMalloc(&c->qmm_counters, sizeof(unsigned int) * 2 * c->sm_count)); CU(cudaMemset(c->qmm_counters, 0, sizeof(unsigned int) * 2 * c->sm_count));
+    CU(cudaMalloc(&c->qg_scratch, sizeof(float) * 2 * c->sm_count * fkq_part_floats(128)));
+    CU(cudaMalloc(&c->qg_counters, sizeof(unsigned int) * (FKQ_COUNTERS + 1))); CU(cudaMemset(c->qg_counters, 0, sizeof(unsigned int) * (FKQ_COUNTERS + 1)));
+    c->qg_peak = c->qg_counters + FKQ_COUNTERS;
     CU(cudaMalloc(&c->history, sizeof(uint32_t) * c->hist_cap)); CU(cudaMemset(c->history, 0, sizeof(uint32_t) * c->hist_cap));
     CU(cudaMallocHost(&c->pinned, sizeof(uint32_t) * (c->hist_cap + 64)));
     const char *e = getenv("FK_PDL"); if (e && e[0] == '0') c->pdl = false;
@@ -164,6 +170,9 @@ extern "C" fk_status fk_open(int device, fk_handle *out) {
     CU(big_smem(k_linear_residual<4>)); CU(big_smem(k_linear_residual<8>)); CU(big_smem(k_linear_residual<16>));
     CU(big_smem(k_rmsnorm_gateup_act<4>)); CU(big_smem(k_rmsnorm_gateup_act<8>)); CU(big_smem(k_rmsnorm_gateup_act<16>));
     CU(big_smem(k_final_head<4>)); CU(big_smem(k_final_head<8>)); CU(big_smem(k_final_head<16>));
+#define QG(BN) CU(cudaFuncSetAttribute(k_qgemm<BN, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)QgTile<BN>::SMEM)); CU(cudaFuncSetAttribute(k_qgemm<BN, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)QgTile<BN>::SMEM))
+    QG(16); QG(32); QG(64); QG(128);
+#undef QG
     CU(fkl_init());
     c->open = true;
     std::lock_guard<std::mutex> lk(g_mu);
@@ -182,6 +191,7 @@ extern "C" fk_status fk_close(fk_handle h) {
     for (unsigned char *p : c->loop_arenas) cudaFree(p);
     if (c->arena) cudaFree(c->arena);
     c->ipc_open.clear(); c->loop_arenas.clear(); c->arena = nullptr; c->peer_ready = false; c->comm = nullptr;
+    cudaFree(c->qg_scratch); cudaFree(c->qg_counters);
     cudaFree(c->qmm_scratch); cudaFree(c->qmm_counters);
     cudaFree(c->state); cudaFree(c->history); cudaFreeHost(c->pinned);
     cudaEventDestroy(c->ev0); cudaEventDestroy(c->ev1); cudaStreamDestroy(c->stream);
@@ -208,7 +218,8 @@ static const char *kKernelNames[FK_TASK_KIND_COUNT] = {
     "fusekit_linear_rows", "fusekit_qk_norm_store_rows", "fusekit_attention_rows", "fusekit_moe_route_rows", "fusekit_norm_linear",
     "fusekit_attention_decode", "fusekit_moe_up", "fusekit_moe_down", "fusekit_argmax_row", "fusekit_block_norm_rows",
     "fusekit_block_linear_rows", "fusekit_rotary_store_rows", "fusekit_window_attention_rows", "fusekit_window_attention_decode", "fusekit_recurrence_rows",
-    "fusekit_recurrence_decode", "fusekit_norm_gate_rows", "fusekit_segment_linear"};
+    "fusekit_recurrence_decode", "fusekit_norm_gate_rows", "fusekit_segment_linear", "fusekit_stage_rows", "fusekit_staged_linear",
+    "fusekit_staged_gateup", "fusekit_embed_prompt", "fusekit_rope_store_prompt", "fusekit_argmax_prompt"};
 extern "C" fk_status fk_kernel_names(char *buf, size_t cap) {
     if (!buf || cap == 0) return fail(FK_ERR_VALUE, "buf is null");
     std::string s;
@@ -317,6 +328,15 @@ static fk_status repack(Ctx *c, Weight *dstw, const Weight *a, const Weight *b2)
     k_repack_tiled<<<(unsigned)((tot + 255) / 256), 256, 0, c->stream>>>(sa, sb, dstw->units, a->n, (int)a->k, a->bits, dstw->ntiles, dstw->nsb,
                                                                         dstw->rows_kind, dstw->hd, dstw->n_rot);
     CU(cudaGetLastError());
+    if (a->bits == 4) {
+        unsigned int peak = 0;
+        CU(cudaMemsetAsync(c->qg_peak, 0, sizeof peak, c->stream));
+        k_weight_peak<<<2 * c->sm_count, 256, 0, c->stream>>>(dstw->units, (long long)dstw->ntiles * dstw->nsb, c->qg_peak);
+        CU(cudaGetLastError());
+        CU(cudaMemcpyAsync(&peak, c->qg_peak, sizeof peak, cudaMemcpyDeviceToHost, c->stream));
+        CU(cudaStreamSynchronize(c->stream));
+        memcpy(&dstw->peak, &peak, sizeof peak);
+    }
     CU(cudaStreamSynchronize(c->stream));
     dstw->tiled = true;
     return FK_OK;
@@ -438,6 +458,24 @@ static cudaError_t launch_qmm(Ctx *c, const Weight *w, QmmArgs &qa, bool gateup)
     qa.kparts = kparts;
     if (gateup) return launch(c, k_qmm4<true>, dim3(qg), dim3(FK_QMM_WARPS * 32), qmm_smem_bytes(), c->state, qa);
     return launch(c, k_qmm4<false>, dim3(qg), dim3(FK_QMM_WARPS * 32), qmm_smem_bytes(), c->state, qa);
+}
+template <int BN> static cudaError_t launch_qgemm(Ctx *c, const QPlan &p, bool gateup, const CUtensorMap &mx, const QGemmArgs &a) {
+    if (gateup) return launch(c, k_qgemm<BN, true>, dim3(p.grid), dim3(FKQ_THREADS), QgTile<BN>::SMEM, c->state, mx, a);
+    return launch(c, k_qgemm<BN, false>, dim3(p.grid), dim3(FKQ_THREADS), QgTile<BN>::SMEM, c->state, mx, a);
+}
+// a product of staged rows (fk_qgemm.cuh): plain rows with a residual, or gate/up pairs with the activation
+static fk_status run_staged(Ctx *c, const Weight *w, bool gateup, const void *xs, const float *xscale, const uint16_t *residual, int ldr, uint16_t *y, int k, int n, int m, int act, cudaError_t *e) {
+    if (!w || !w->finalized || !w->tiled || w->bits != 4 || w->rows_kind != (gateup ? FK_ROWS_GATE_UP : FK_ROWS_PLAIN)) return fail(FK_ERR_VALUE, "staged product: takes streamed 4-bit weights (plain rows, or gate/up pairs)");
+    if (w->k != k || w->n != (gateup ? 2LL : 1LL) * n || m <= 0 || !xs || !xscale || !y || ((uintptr_t)xs & 15)) return fail(FK_ERR_VALUE, "staged product: shape mismatch");
+    if (k > FKQ_MAX_K) return fail(FK_ERR_VALUE, "staged product: at most %d columns", FKQ_MAX_K);
+    const QPlan p = fkq_plan(m, w->ntiles, w->nsb, c->sm_count);
+    int ex = 0;
+    if (w->peak > 0.0f) { frexpf(w->peak, &ex); ex = ex < -100 ? -100 : ex > 110 ? 110 : ex; } else ex = 15;      // peak in [2^(ex-1), 2^ex)
+    QGemmArgs a{w->tview(), xscale, residual, y, c->qg_scratch, c->qg_counters, m, n, ldr, act, p.whole, p.mtiles, p.tiles, ldexpf(1.0f, 15 - ex), ldexpf(1.0f, ex - 15)};
+    CUtensorMap mx;
+    if (!fkl_tensor_map(&mx, xs, m, (long long)w->nsb * FKQ_SB, (long long)w->nsb * FKQ_SB, p.bn, true)) return fail(FK_ERR_VALUE, "staged product: tensor map refused");
+    *e = p.bn == 16 ? launch_qgemm<16>(c, p, gateup, mx, a) : p.bn == 32 ? launch_qgemm<32>(c, p, gateup, mx, a) : p.bn == 64 ? launch_qgemm<64>(c, p, gateup, mx, a) : launch_qgemm<128>(c, p, gateup, mx, a);
+    return FK_OK;
 }
 #define BITS_SWITCH(bits, CALL)                  \
     switch (bits) {                              \
@@ -830,6 +868,44 @@ static fk_status run_task(Ctx *c, const fk_task &t, const Weight *nextw = nullpt
         if (!b[0] || !b[5] || i[0] <= 0 || i[1] <= 0 || i[1] > FK_MAX_ROWS) return fail(FK_ERR_VALUE, "argmax_rows: bad arguments");
         ArgmaxRowsArgs a{(const uint16_t *)b[0], (uint32_t *)b[5], c->history, i[0], i[1], i[2] > 0 ? i[2] : 1};
         e = launch(c, k_argmax_rows, dim3(i[1]), dim3(1024), 0, c->state, a);
+        break;
+    }
+    case FK_TASK_STAGE_ROWS: {
+        const int k = i[0], m = i[1];
+        if (!b[0] || !b[2] || !b[3] || k <= 0 || k % 64 || k > FKQ_MAX_K || m <= 0 || ((b[0] | b[1] | b[2]) & 15)) return fail(FK_ERR_VALUE, "stage_rows: bad arguments (K a multiple of 64 up to %d, 16-byte aligned buffers)", FKQ_MAX_K);
+        StageRowsArgs a{(const uint16_t *)b[0], (const uint16_t *)b[1], (__half *)b[2], (float *)b[3], k, (k + 511) / 512, f[0]};
+        if (k <= 4096) e = launch(c, k_stage_rows<128>, dim3(m), dim3(128), 0, (const FkState *)c->state, a);
+        else if (k <= 8192) e = launch(c, k_stage_rows<256>, dim3(m), dim3(256), 0, (const FkState *)c->state, a);
+        else e = launch(c, k_stage_rows<1024>, dim3(m), dim3(1024), 0, (const FkState *)c->state, a);
+        break;
+    }
+    case FK_TASK_STAGED_LINEAR: {
+        fk_status s = run_staged(c, get_w(c, b[2]), false, (const void *)b[0], (const float *)b[1], (const uint16_t *)b[3], i[3] ? 0 : i[1], (uint16_t *)b[4], i[0], i[1], i[2], 0, &e);
+        if (s) return s;
+        break;
+    }
+    case FK_TASK_STAGED_GATEUP: {
+        if (i[3] != FK_ACT_SWIGLU && i[3] != FK_ACT_GEGLU_TANH) return fail(FK_ERR_VALUE, "staged_gateup: unknown activation");
+        fk_status s = run_staged(c, get_w(c, b[2]), true, (const void *)b[0], (const float *)b[1], nullptr, 0, (uint16_t *)b[4], i[0], i[1], i[2], i[3], &e);
+        if (s) return s;
+        break;
+    }
+    case FK_TASK_EMBED_PROMPT: {
+        if (!b[0] || !b[1] || !b[2] || i[0] <= 0 || i[0] % 8 || i[1] <= 0 || i[2] <= 0 || ((b[0] | b[1]) & 15)) return fail(FK_ERR_VALUE, "embed_prompt: bad arguments");
+        EmbedPromptArgs a{(const uint16_t *)b[0], (uint16_t *)b[1], (const uint32_t *)b[2], i[0], i[2]};
+        e = launch(c, k_embed_prompt, dim3(i[1]), dim3(256), 0, c->state, a);
+        break;
+    }
+    case FK_TASK_ROPE_STORE_PROMPT: {
+        const int nq = i[0], nkv = i[1], hd = i[2], cap = i[3], rows = i[4];
+        if (!b[0] || !b[1] || !b[5] || !b[6] || nq <= 0 || nkv <= 0 || hd <= 0 || (hd & 1) || hd > 2048 || cap <= 0 || rows <= 0 || rows > 65535) return fail(FK_ERR_VALUE, "rope_store_prompt: bad arguments");
+        RopeRowsArgs a{(const uint16_t *)b[0], (uint16_t *)b[1], (uint16_t *)b[5], (uint16_t *)b[6], nq, nkv, hd, cap, rows, (float)log2((double)f[1]), 1};
+        e = launch(c, k_rope_store_rows, dim3(nq + 2 * nkv, rows), dim3((hd / 2 + 31) / 32 * 32), 0, (const FkState *)c->state, a);
+        break;
+    }
+    case FK_TASK_ARGMAX_PROMPT: {
+        if (!b[0] || !b[1] || i[0] <= 0 || i[0] % 8 || i[1] <= 0 || (b[0] & 15)) return fail(FK_ERR_VALUE, "argmax_prompt: bad arguments");
+        e = launch(c, k_argmax_prompt, dim3(i[1]), dim3(512), 0, (const FkState *)c->state, (const uint16_t *)b[0], (uint32_t *)b[1], i[0]);
         break;
     }
     case FK_TASK_KV_STORE_QUANT: {

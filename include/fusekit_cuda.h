@@ -77,7 +77,14 @@ enum {
     FK_TASK_RECURRENCE_DECODE = 33,
     FK_TASK_NORM_GATE_ROWS = 34,
     FK_TASK_SEGMENT_LINEAR = 35,
-    FK_TASK_KIND_COUNT = 36
+    /* products of any number of rows with 4-bit weights on the tensor cores, and the rest of a prompt's passes */
+    FK_TASK_STAGE_ROWS = 36,
+    FK_TASK_STAGED_LINEAR = 37,
+    FK_TASK_STAGED_GATEUP = 38,
+    FK_TASK_EMBED_PROMPT = 39,
+    FK_TASK_ROPE_STORE_PROMPT = 40,
+    FK_TASK_ARGMAX_PROMPT = 41,
+    FK_TASK_KIND_COUNT = 42
 };
 
 /* activation selector for FK_TASK_RMSNORM_GATEUP_ACT */
@@ -224,6 +231,14 @@ enum { FK_ACT_NONE = 0, FK_ACT_RELU_SQUARED = 2, FK_ACT_SILU = 3 };
  * SEGMENT_LINEAR       one row, up to three products y_s = W_s x_s of i0 rows: buf(2s) x_s f32, buf(2s + 1) weight  buf6 y f32[i1][i0]  buf7 w T, buf8
  *                      gate f32: input i5 is staged as norm(x) * w * sigmoid(gate), the norm over groups of i6 (i5 = -1: none)
  *                      i0 rows  i1 products  i2..i4 values of x_s   f0 eps
+ * STAGE_ROWS           buf0 x T[M, K]  buf1 norm_w T[K]|0 (RMSNorm first)  buf2 staged rows, 1152 * ceil(K / 512) bytes each (16-byte aligned)
+ *                      buf3 row factors f32[M]   i0 K (a multiple of 64, at most 32768)  i1 M   f0 eps
+ * STAGED_LINEAR        buf0 staged rows  buf1 row factors  buf2 weight (streamed 4-bit, plain rows)  buf3 residual T[M, N]|0  buf4 y T[M, N]
+ *                      i0 K  i1 N  i2 M (any number)  i3 = 1: one residual row T[N] for all.  Row m is LINEAR_RESIDUAL's for x[m]
+ * STAGED_GATEUP        buf0 staged rows  buf1 row factors  buf2 weight (fk_weight_pair)  buf4 act_out T[M, I]   i0 H  i1 I  i2 M  i3 act
+ * EMBED_PROMPT         buf0 table T[V, H]  buf1 x T[M, H]  buf2 token ids u32[M] (a device buffer)   i0 H  i1 M  i2 V
+ * ROPE_STORE_PROMPT    ROPE_STORE_ROWS for any number of consecutive positions (the cache does not wrap within them)
+ * ARGMAX_PROMPT        buf0 logits T[M, V]  buf1 greedy ids u32[M]   i0 V (a multiple of 8)  i1 M; the decode state is left alone
  *
  * Batch decode (M = 2..16 independent sequences at one position): EMBED with i1 = M, LINEAR_RESIDUAL / RMSNORM_GATEUP_ACT
  * with their row counts, SDPA_DECODE with i5 = M (q and out T[M, n_q*hd], caches [M, n_kv, capacity, hd]).

@@ -1,0 +1,162 @@
+"""Products of staged rows (any number of rows, 4-bit weights, tcgen05) and the whole-prompt path built on them."""
+import numpy as np
+import pytest
+
+from fusekit_b200 import _native as N
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+T = N.Task.make
+
+
+def _weight(rt, w):
+    wid = rt.weight_alloc(w.n, w.k, 4)
+    rt.weight_upload_rows(wid, 0, w.packed, w.scales, w.biases)
+    return wid
+
+
+def _gen(name, n, k, wide=False):
+    """A synthetic weight; ``wide``: scales over six orders of magnitude, groups far from zero and groups of one value."""
+    w = O.gen_weight(hash_stream(name), n, k, 4)
+    if wide:
+        rng = np.random.default_rng(n + k)
+        s = O.bf16_to_f32(w.scales) * np.float32(10.0) ** rng.uniform(-4, 2, w.scales.shape).astype(np.float32)
+        s[rng.random(s.shape) < 0.1] = 0.0
+        b = np.where(rng.random(s.shape) < 0.2, rng.normal(size=s.shape), O.bf16_to_f32(w.biases)).astype(np.float32)
+        w.scales, w.biases = O.f32_to_bf16(s), O.f32_to_bf16(b)
+    return w
+
+
+def hash_stream(name):
+    from fusekit_b200.model_spec import stream_id
+    return stream_id(5, name)
+
+
+def _values(w):
+    """The numbers a weight stands for, in 64 bits."""
+    q = (np.asarray(w.packed, np.uint32)[..., None] >> (4 * np.arange(8, dtype=np.uint32))) & 15
+    q = q.reshape(w.n, w.k // 64, 64).astype(np.float64)
+    s, b = (O.bf16_to_f32(a).astype(np.float64).reshape(w.n, w.k // 64, 1) for a in (w.scales, w.biases))
+    return (q * s + b).reshape(w.n, w.k)
+
+
+def _rows(m, k, seed, spread=False):
+    rng = np.random.default_rng(seed)
+    x = rng.normal(size=(m, k)).astype(np.float32)
+    if spread:                                          # outliers, rows of other magnitudes, a row of zeros
+        x *= np.float32(2.0) ** rng.integers(-18, 4, (m, k)).astype(np.float32)
+        x *= np.float32(10.0) ** rng.uniform(-20, 20, (m, 1)).astype(np.float32)
+        x[m // 2] = 0.0
+    return O.f32_to_bf16(x)
+
+
+def _stage(rt, xd, m, k, norm=0, eps=1e-6):
+    staged, factor = rt.alloc(m * -(-k // 512) * 1152), rt.alloc(m * 4)
+    rt.launch(T(N.TASK_STAGE_ROWS, -1, {0: xd, 1: norm, 2: staged, 3: factor}, [k, m], [eps]))
+    return staged, factor
+
+
+def _check(got, want, size, what):
+    """One rounding to bf16 (2^-9 of the value), and fp32 sums: 2^-19 of the sum of magnitudes covers 32768 terms in any order
+    (n 2^-24 in the worst order of a sum of n / 64 blocks, and the rounding of the 22-bit sums)."""
+    bad = ~(np.abs(got - want) <= 2.0 ** -8 * np.abs(want) + 2.0 ** -19 * size)
+    assert not bad.any(), (what, int(bad.sum()), np.argwhere(bad)[:3], got[bad][:3], want[bad][:3])
+
+
+# rows at the edges of the tiles (16, 32, 64, 128), K of one unit, a part of one and many, N at the edges of units and of blocks
+SHAPES = [(1, 64, 16), (2, 512, 256), (16, 896, 1152), (16, 4864, 896), (17, 576, 250), (32, 1088, 272), (33, 512, 257), (64, 2048, 16), (65, 896, 304), (100, 4864, 896),
+          (128, 512, 40000), (129, 640, 512), (200, 3584, 4608), (300, 1024, 2056), (16, 3584, 40960), (5, 18944, 3584), (9, 32768, 64)]
+
+
+@pytest.mark.parametrize("m,k,n", SHAPES)
+@pytest.mark.parametrize("wide", [False, True])
+def test_staged_linear_against_64_bits(runtime, m, k, n, wide):
+    rt = runtime
+    w = _gen(f"staged.{k}.{n}", n, k, wide)
+    x, res = _rows(m, k, k + n + m, wide), O.f32_to_bf16(np.random.default_rng(m).normal(size=(m, n)).astype(np.float32))
+    wid = _weight(rt, w); rt.weight_finalize(wid)
+    xd, rd, yd = rt.to_device(x), rt.to_device(res), rt.alloc(m * n * 2)
+    staged, factor = _stage(rt, xd, m, k)
+    V, X = _values(w), O.bf16_to_f32(x).astype(np.float64)
+    want, size, r = X @ V.T, np.abs(X) @ np.abs(V).T, O.bf16_to_f32(res).astype(np.float64)
+    for resid, one in ((rd, 0), (rd, 1), (0, 0)):
+        N.check(rt.L.fk_memset(rt.h, yd, 0xff, m * n * 2), "memset")
+        for _ in range(2):                              # the tickets of a split product are ready again
+            rt.launch(T(N.TASK_STAGED_LINEAR, -1, {0: staged, 1: factor, 2: wid, 3: resid, 4: yd}, [k, n, m, one]))
+        got = O.bf16_to_f32(rt.download(yd, (m, n), np.uint16)).astype(np.float64)
+        add = (r[:1] if one else r) if resid else 0.0
+        _check(got, want + add, size + np.abs(add), (m, k, n, wide, bool(resid), one))
+    assert rt.state_get()[2] == 0
+    for p in (xd, rd, yd, staged, factor):
+        N.check(rt.L.fk_free(rt.h, p), "fk_free")
+
+
+def test_staged_linear_keeps_infinities_and_nan_in_their_rows(runtime):
+    rt = runtime
+    m, k, n = 20, 576, 300
+    w = _gen("staged.inf", n, k)
+    x = _rows(m, k, 3)
+    x[4, 100], x[7, 5], x[9, 0] = 0x7f80, 0x7fc0, 0xff80
+    wid = _weight(rt, w); rt.weight_finalize(wid)
+    staged, factor = _stage(rt, rt.to_device(x), m, k)
+    yd = rt.alloc(m * n * 2)
+    rt.launch(T(N.TASK_STAGED_LINEAR, -1, {0: staged, 1: factor, 2: wid, 4: yd}, [k, n, m, 0]))
+    got = O.bf16_to_f32(rt.download(yd, (m, n), np.uint16))
+    finite = np.isfinite(got).all(1)
+    assert not np.isfinite(got[[4, 7, 9]]).any() and finite[[i for i in range(m) if i not in (4, 7, 9)]].all()
+
+
+@pytest.mark.parametrize("act", [N.ACT_SWIGLU, N.ACT_GEGLU_TANH])
+@pytest.mark.parametrize("m,h,inter", [(1, 64, 8), (2, 896, 4864), (16, 256, 520), (33, 512, 137), (100, 896, 1000), (130, 1088, 512)])
+def test_staged_gateup_matches_the_one_row_kernel(runtime, m, h, inter, act):
+    """Norm, product and activation of every row against the one-row kernel on the same row: the same roundings around the sums, so
+    at most one bf16 step of the result where a sum falls on the other side of a rounding."""
+    rt = runtime
+    g, u = _gen(f"staged.g{h}.{inter}", inter, h), _gen(f"staged.u{h}.{inter}", inter, h)
+    pair = rt.weight_pair(_weight(rt, g), _weight(rt, u))
+    x, nw = _rows(m, h, m + h), O.f32_to_bf16(1 + 0.1 * np.random.default_rng(1).normal(size=h).astype(np.float32))
+    xd, nd, yd, one = rt.to_device(x), rt.to_device(nw), rt.alloc(m * inter * 2), rt.alloc(inter * 2)
+    staged, factor = _stage(rt, xd, m, h, nd)
+    rt.launch(T(N.TASK_STAGED_GATEUP, -1, {0: staged, 1: factor, 2: pair, 4: yd}, [h, inter, m, act]))
+    got = O.bf16_to_f32(rt.download(yd, (m, inter), np.uint16)).astype(np.float64)
+    for i in sorted({0, m // 2, m - 1}):
+        rt.launch(T(N.TASK_RMSNORM_GATEUP_ACT, -1, {0: xd + i * h * 2, 1: nd, 2: pair, 4: one}, [h, inter, act], [1e-6]))
+        want = O.bf16_to_f32(rt.download(one, (inter,), np.uint16)).astype(np.float64)
+        # gate and up are rounded to bf16 before the activation: a flip in each moves the result by up to 2^-8 of gate and of up,
+        # and the geglu chain carries up to four more roundings
+        rms = np.sqrt(np.mean(want ** 2))
+        assert np.abs(got[i] - want).max() <= 2.0 ** -5 * max(np.abs(want).max(), rms) and np.sqrt(np.mean((got[i] - want) ** 2)) <= 4e-3 * rms, (m, h, inter, act, i)
+
+
+@pytest.mark.parametrize("rows,count", [(16, 17), (16, 90), (4, 5), (4, 7), (5, 23), (16, 150)])
+def test_whole_prompts_match_the_steps(rows, count):
+    """A prompt through the kernels of whole prompts against the same engine stepping it (the mma.sync kernels asked for by name): caches
+    and the last step's logits within what two orders of summation differ by over the toy's layers, greedy tokens but for near-ties;
+    with portions of 32 positions too, so that a portion starts past position 0."""
+    from fusekit_b200.batch import PrefillEngine
+    from fusekit_b200.model_spec import CONFIGS, stream_id
+    spec, cap, base = CONFIGS["tiny-qwen"], 192, 3
+    prompt = [O.uniform_u32(stream_id(spec.seed, "prompt"), i, spec.vocab) for i in range(count + base)]
+    hd, got = spec.head_dim, {}
+    for name, qmm, portion in (("steps", 2, 1024), ("whole", 0, 1024), ("portions", 0, 32)):
+        eng = PrefillEngine(spec, cap, rows, qmm=qmm)
+        try:
+            eng.PORTION = portion
+            eng.load_synthetic()
+            eng.prefill(prompt[:base])
+            preds = eng.prefill(prompt[base:], base)
+            caches = np.stack([[eng.rt.download(p, (spec.n_kv, cap, hd), np.uint16)[:, :count + base] for p in kv] for kv in eng.cache])
+            logits = eng.rt.download(eng.logits, (rows, spec.vocab), np.uint16)[:(count - 1) % rows + 1]
+            got[name] = preds, O.bf16_to_f32(caches).astype(np.float64), O.bf16_to_f32(logits).astype(np.float64)
+            if name == "whole":
+                with pytest.raises(ValueError):
+                    eng.prefill(prompt * 2, cap - count)
+                with pytest.raises(N.FusekitError):
+                    eng.prefill(prompt[:-1] + [spec.vocab])
+                assert list(eng.prefill(prompt[base:], base)) == list(preds)
+        finally:
+            eng.close()
+    for name in ("whole", "portions"):
+        assert sum(a != b for a, b in zip(got[name][0], got["steps"][0])) <= max(2, count // 16), name
+        for a, b in zip(got[name][1:], got["steps"][1:]):
+            assert np.sqrt(np.mean((a - b) ** 2)) <= 8e-3 * np.sqrt(np.mean(b ** 2)), name
