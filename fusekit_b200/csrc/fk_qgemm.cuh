@@ -13,7 +13,7 @@
 // A block owns 256 weight rows (two M = 128 accumulators) x BN rows of X.  16 warps turn one unit each (16 weight rows) into fp16
 // and write it straight into tensor memory as the A operand (tcgen05.st .16x256b: the lane layout of the units is its lane layout; a ring
 // of four k-blocks); through shared memory the expanded operand costs two more crossings of it than the packed weights.  One warp
-// fetches X by TMA (128-byte swizzle), one thread issues the MMAs, 8 warps store finished tiles.  Weight rings are filled before
+// fetches X by TMA (128-byte swizzle), one warp per accumulator issues its MMAs, 8 warps store finished tiles.  Weight rings are filled before
 // griddepcontrol.wait.  Every wait is bounded; when one runs out the kernel sets an error bit, waits (bounded) for its copies, frees
 // its tensor memory and returns.
 //
@@ -27,7 +27,7 @@
 #define FKQ_SB 576                      // staged halves per super-block: 512 activations, 32 slots for the sums, 32 unused
 #define FKQ_DEQ 16                      // dequantising warps: one unit each
 #define FKQ_EPI 8                       // storing warps
-#define FKQ_THREADS ((FKQ_DEQ + FKQ_EPI + 2) * 32)
+#define FKQ_THREADS ((FKQ_DEQ + FKQ_EPI + 3) * 32)      // .. a warp for X, two for the MMAs
 #define FKQ_ROWS 256                    // weight rows of a block
 #define FKQ_AS 4                        // k-blocks of A operand in tensor memory (64 columns each)
 #define FKQ_SPIN (1u << 21)
@@ -36,12 +36,17 @@
 #define FKQ_COUNTERS 65536              // ticket words: 8 per tile that is split
 template <int BN> struct QgTile {
     static constexpr int XS = BN >= 128 ? 4 : BN == 64 ? 8 : 12, XBYTES = BN * 128, NBUF = BN <= 64 ? 2 : 1;
-    static constexpr size_t SMEM = 1024 + (size_t)XS * XBYTES + (size_t)FKQ_DEQ * FK_STAGES * FK_UNIT_BYTES;
+    static constexpr size_t SMEM = 1024 + (size_t)XS * XBYTES + (size_t)FKQ_DEQ * FK_STAGES * FK_UNIT_BYTES + (size_t)FKQ_EPI * BN * 4;
 };
 __host__ __device__ inline size_t fkq_part_floats(int bn) { return (size_t)bn * FKQ_ROWS; }
 
 struct QGemmArgs { TiledW W; const float *xscale; const uint16_t *residual; uint16_t *y; float *scratch; unsigned int *counters; int m, n, ldr, act, whole, mtiles, tiles; float wmul, wscale; };
 
+__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    return ok != 0;
+}
 __device__ __forceinline__ bool qg_wait(uint32_t bar, uint32_t parity) {
     for (uint32_t i = 0; i < FKQ_SPIN; ++i) {
         uint32_t ok;
@@ -53,6 +58,15 @@ __device__ __forceinline__ bool qg_wait(uint32_t bar, uint32_t parity) {
 __device__ __forceinline__ void qg_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
 __device__ __forceinline__ void qg_expect(uint32_t bar, uint32_t bytes) { asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory"); }
 __device__ __forceinline__ void qg_commit(uint32_t bar) { asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory"); }
+__device__ __forceinline__ bool qg_elect() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
+// D += A B^T: A (128 rows, 16 halves) in tensor memory, B (the descriptor's rows) in shared memory; more = 0 overwrites D
+__device__ __forceinline__ void qg_mma(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t more) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(more) : "memory");
+}
 __device__ __forceinline__ uint32_t h2_sub(uint32_t a, uint32_t b) { __half2 r = __hsub2(*reinterpret_cast<__half2 *>(&a), *reinterpret_cast<__half2 *>(&b)); return *reinterpret_cast<uint32_t *>(&r); }
 __device__ __forceinline__ uint32_t h2_mul(uint32_t a, uint32_t b) { __half2 r = __hmul2(*reinterpret_cast<__half2 *>(&a), *reinterpret_cast<__half2 *>(&b)); return *reinterpret_cast<uint32_t *>(&r); }
 __device__ __forceinline__ uint32_t h2_pack(float lo, float hi) { __half2 r = __floats2half2_rn(lo, hi); return *reinterpret_cast<uint32_t *>(&r); }
@@ -84,12 +98,14 @@ __host__ __device__ inline bool fkq_work(int whole, int tiles, int nsb, int b, i
 __host__ __device__ inline int fkq_owner(int tiles, int nsb, int G, int s) { return (int)((((long long)s + 1) * G - 1) / ((long long)tiles * nsb)); }
 __host__ __device__ inline int fkq_slot(int tiles, int nsb, int G, int b, int tile) { return 2 * b + ((int)((long long)b * tiles * nsb / G) / nsb == tile ? 0 : 1); }
 
-// Rows of X per tile, blocks and split of a product of m rows: the widest tile that the rows fill; up to 32 rows the steps are dealt in
-// equal runs (a part's sums are small, and the product is bound by the weights), from 33 on only while less than half of the blocks have a tile.
+// Rows of X per tile, blocks and split of a product of m rows: the widest tile that the rows fill, a narrower one while that gives more
+// blocks a tile of their own (a step costs a block the same up to 64 rows); up to 32 rows the steps are dealt in equal runs (a part's
+// sums are small, and the product is bound by the weights), from 33 on only while less than half of the blocks have a tile.
 struct QPlan { int bn, mtiles, tiles, grid, whole; };
 inline QPlan fkq_plan(int m, int ntiles, int nsb, int sm) {
     QPlan p;
     p.bn = m <= 16 ? 16 : m <= 32 ? 32 : m <= 64 ? 64 : 128;
+    while (p.bn > 16 && (ntiles + 15) / 16 * ((m + p.bn / 2 - 1) / (p.bn / 2)) <= sm) p.bn /= 2;
     p.mtiles = (m + p.bn - 1) / p.bn; p.tiles = (ntiles + 15) / 16 * p.mtiles; p.whole = 1; p.grid = p.tiles < sm ? p.tiles : sm;
     if (p.tiles > FKQ_COUNTERS / FKQ_EPI) return p;
     if (p.bn <= 32) {
@@ -108,7 +124,7 @@ __global__ void __launch_bounds__(FKQ_THREADS, 1) k_qgemm(FkState *st, const __g
     extern __shared__ unsigned char qg_smem[];
     __shared__ __align__(8) uint64_t bars[FKQ_DEQ * FK_STAGES + 2 * XS + 2 * FKQ_AS + 2 * NBUF];
     __shared__ uint32_t tmem_slot;
-    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, wid = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const uint32_t base = (smem_u32(qg_smem) + 1023u) & ~1023u, ring = base + XS * T::XBYTES;
     const uint32_t wfull = smem_u32(bars), xfull = wfull + 8 * FKQ_DEQ * FK_STAGES, xempty = xfull + 8 * XS, afull = xempty + 8 * XS, aempty = afull + 8 * FKQ_AS,
                    dfull = aempty + 8 * FKQ_AS, dempty = dfull + 8 * NBUF;
@@ -116,11 +132,11 @@ __global__ void __launch_bounds__(FKQ_THREADS, 1) k_qgemm(FkState *st, const __g
     if (tid == 0) {
         for (int i = 0; i < FKQ_DEQ * FK_STAGES; ++i) mbar_init(bars + i, 1);
         uint64_t *b = bars + FKQ_DEQ * FK_STAGES;
-        for (int i = 0; i < 2 * XS; ++i) mbar_init(b + i, 1);
+        for (int i = 0; i < XS; ++i) { mbar_init(b + i, 1); mbar_init(b + XS + i, 2); }
         b += 2 * XS;
-        for (int i = 0; i < FKQ_AS; ++i) { mbar_init(b + i, FKQ_DEQ); mbar_init(b + FKQ_AS + i, 1); }
+        for (int i = 0; i < FKQ_AS; ++i) { mbar_init(b + i, FKQ_DEQ); mbar_init(b + FKQ_AS + i, 2); }
         b += 2 * FKQ_AS;
-        for (int i = 0; i < NBUF; ++i) { mbar_init(b + i, 1); mbar_init(b + NBUF + i, FKQ_EPI); }
+        for (int i = 0; i < NBUF; ++i) { mbar_init(b + i, 2); mbar_init(b + NBUF + i, FKQ_EPI); }
         mbar_fence_init();
     }
     if (wid == FKQ_DEQ) {
@@ -240,59 +256,116 @@ __global__ void __launch_bounds__(FKQ_THREADS, 1) k_qgemm(FkState *st, const __g
             for (int j = it > XS ? it - XS : 0; j < it; ++j) if (!qg_wait((ok ? xempty : xfull) + 8 * (j % XS), (uint32_t)(j / XS) & 1u)) ok = false;
             if (!ok) atomicOr(&st->error, FKQ_ERR_WAIT);
         }
-    } else if (wid == FKQ_DEQ + FKQ_EPI + 1) {
-        // ---------------------------------------------------------------- MMA issue
+    } else if (wid > FKQ_DEQ + FKQ_EPI) {
+        // ---------------------------------------------------------------- MMA issue, a warp per accumulator: the warp stays together and one elected lane
+        // issues, so that addresses and descriptors live in uniform registers (a branch on the lane costs moves into them before every
+        // instruction: 84 cycles an MMA, 33 with the election); the next k-block's barriers are looked at while this one's MMAs go out,
+        // and one warp's waits pass under the other's issue
         pdl_wait();
-        if (lane == 0) {
-            const uint32_t idesc = (1u << 4) | ((uint32_t)(BN >> 3) << 17) | ((128u >> 4) << 24);          // fp16 x fp16 -> fp32
-            int it = 0;
-            for (int v = 0; ok && fkq_work(a.whole, a.tiles, nsb, me, G, v, w); ++v) {
-                const int d = v % NBUF, steps = (w.k1 - w.k0) * 9;
-                if (v >= NBUF && !qg_wait(dempty + 8 * d, (uint32_t)(v / NBUF - 1) & 1u)) { ok = false; break; }
-                int kk = 0;
-                for (int kb = 0; kb < steps; ++kb, ++it) {
-                    const int s = it % XS, as = it % FKQ_AS;
-                    if (!qg_wait(xfull + 8 * s, (uint32_t)(it / XS) & 1u) || !qg_wait(afull + 8 * as, (uint32_t)(it / FKQ_AS) & 1u)) { ok = false; break; }
+        const int sub = wid - (FKQ_DEQ + FKQ_EPI + 1);
+        const uint32_t idesc = (1u << 4) | ((uint32_t)(BN >> 3) << 17) | ((128u >> 4) << 24);          // fp16 x fp16 -> fp32
+        const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0), tma = tm + 256u + (uint32_t)(sub * 32);
+        const uint64_t db0 = (uint64_t)((base >> 4) & 0x3FFFu) | (1ull << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
+        int s = 0, as = 0;
+        uint32_t xph = 0, aph = 0;
+        bool xready = false, aready = false;
+        for (int v = 0; ok && fkq_work(a.whole, a.tiles, nsb, me, G, v, w); ++v) {
+            const int d = v % NBUF;
+            if (v >= NBUF && !qg_wait(dempty + 8 * d, (uint32_t)(v / NBUF - 1) & 1u)) { ok = false; break; }
+            const uint32_t dd = tm + (uint32_t)((d * 2 + sub) * BN);
+            uint32_t more = 0;                          // 0: the tile's first MMA overwrites
+            for (int sb = w.k0; sb < w.k1 && ok; ++sb)
+#pragma unroll 1
+                for (int kk = 0; kk < 9; ++kk) {
+                    if ((!xready && !qg_wait(xfull + 8 * s, xph)) || (!aready && !qg_wait(afull + 8 * as, aph))) { ok = false; break; }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint32_t xb = base + s * T::XBYTES;
-                    const uint64_t db = (uint64_t)((xb >> 4) & 0x3FFFu) | (1ull << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
-                    const int nk = kk == 8 ? 2 : 4;
-                    kk = kk == 8 ? 0 : kk + 1;
-#pragma unroll
-                    for (int sub = 0; sub < 2; ++sub)
-#pragma unroll
-                        for (int k = 0; k < 4; ++k)
-                            if (k < nk)
-                                asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-                                             ::"r"(tmem + (uint32_t)((d * 2 + sub) * BN)), "r"(tmem_a + (uint32_t)(as * 64 + sub * 32 + k * 8)), "l"(db + (uint64_t)(k * 2)),
-                                               "r"(idesc), "r"(kb | k) : "memory");
-                    qg_commit(aempty + 8 * as); qg_commit(xempty + 8 * s);
+                    const uint64_t db = db0 + (uint64_t)(s * (T::XBYTES >> 4));
+                    const uint32_t aa = tma + (uint32_t)(as * 64), as_bar = aempty + 8 * as, xs_bar = xempty + 8 * s;
+                    if (++s == XS) { s = 0; xph ^= 1u; }
+                    if (++as == FKQ_AS) { as = 0; aph ^= 1u; }
+                    xready = mbar_try(xfull + 8 * s, xph); aready = mbar_try(afull + 8 * as, aph);
+                    if (qg_elect()) {
+                        qg_mma(dd, aa, db, idesc, more);
+                        qg_mma(dd, aa + 8, db + 2, idesc, 1u);
+                        if (kk < 8) { qg_mma(dd, aa + 16, db + 4, idesc, 1u); qg_mma(dd, aa + 24, db + 6, idesc, 1u); }
+                        qg_commit(as_bar); qg_commit(xs_bar);
+                    }
+                    __syncwarp();
+                    more = 1;
                 }
-                if (ok) qg_commit(dfull + 8 * d);
-            }
-            if (!ok) atomicOr(&st->error, FKQ_ERR_WAIT);
+            if (ok && qg_elect()) qg_commit(dfull + 8 * d);
+            __syncwarp();
         }
+        if (!ok && lane == 0) atomicOr(&st->error, FKQ_ERR_WAIT);
     } else {
         // ---------------------------------------------------------------- finished tiles: lane = weight row, registers = rows of X
         pdl_wait();
         const int ew = wid - FKQ_DEQ, q = ew & 3, sub = ew >> 2;
+        float *factors = reinterpret_cast<float *>(qg_smem + (ring - smem_u32(qg_smem)) + (size_t)FKQ_DEQ * FK_STAGES * FK_UNIT_BYTES) + ew * BN;
         for (int v = 0; ok && fkq_work(a.whole, a.tiles, nsb, me, G, v, w); ++v) {
-            const int d = v % NBUF, rt = w.tile / a.mtiles, m0 = (w.tile - rt * a.mtiles) * BN, row0 = rt * FKQ_ROWS + sub * 128 + q * 32;
+            const int d = v % NBUF, rt = w.tile / a.mtiles, m0 = (w.tile - rt * a.mtiles) * BN, row0 = rt * FKQ_ROWS + sub * 128 + q * 32, n = row0 + lane;
+            const bool part = w.k0 != 0 || w.k1 != nsb, adds = !GATEUP && a.residual && n < a.n;
+            uint16_t res[2][16];                        // residuals of 32 rows of X on their way
+            auto fetch = [&](int c, uint16_t (&r)[16]) {
+#pragma unroll
+                for (int i = 0; i < 16; ++i) r[i] = adds && m0 + c + i < a.m ? __ldcg(a.residual + (size_t)(m0 + c + i) * a.ldr + n) : (uint16_t)0;
+            };
+            auto fetch_all = [&]() {
+                for (int i = lane; i < BN; i += 32) factors[i] = m0 + i < a.m ? __ldcg(a.xscale + m0 + i) * a.wscale : 0.0f;
+                if (!GATEUP) { fetch(0, res[0]); if (BN > 16) fetch(16, res[1]); }
+                __syncwarp();
+            };
+            if (!part) fetch_all();                     // under the tile's MMAs
             if (!qg_wait(dfull + 8 * d, (uint32_t)(v / NBUF) & 1u)) { ok = false; break; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t src = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)((d * 2 + sub) * BN);
-            const bool part = w.k0 != 0 || w.k1 != nsb;
-            bool finish = !part;
-            int first = 0, last = 0;
-            if (part) {
+            const int rows = min(BN, a.m - m0);         // of X that there are
+            auto store = [&](int c, float (&acc)[16], uint16_t (&r)[16]) {
+#pragma unroll
+                for (int i = 0; i < 16; i += 4) {
+                    const float4 f = *reinterpret_cast<const float4 *>(factors + c + i);
+                    acc[i] *= f.x; acc[i + 1] *= f.y; acc[i + 2] *= f.z; acc[i + 3] *= f.w;
+                }
+                if (GATEUP) {
+                    // lanes 0-7 / 16-23 hold gate rows, 8-15 / 24-31 the up rows of the same outputs: the lower half takes the even row of X of a
+                    // pair, the upper half the odd one
+                    const bool up = lane & 8;
+                    const int out = (row0 >> 4) * 8 + (lane >> 4) * 8 + (lane & 7);
+#pragma unroll
+                    for (int i = 0; i < 16; i += 2) {
+                        const float other = __shfl_xor_sync(0xffffffffu, up ? acc[i] : acc[i + 1], 8);
+                        const float gate = up ? other : acc[i], upv = up ? acc[i + 1] : other;
+                        const int m = c + i + (up ? 1 : 0);
+                        if (m < rows && out < a.n) a.y[(size_t)(m0 + m) * a.n + out] = a.act == 1 ? s_act_geglu(gate, upv) : s_act_swiglu(gate, upv);
+                    }
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) if (n < a.n && c + i < rows) a.y[(size_t)(m0 + c + i) * a.n + n] = f2bf(acc[i] + bf2f(r[i]));
+                    if (c + 32 < rows) fetch(c + 32, r);
+                }
+            };
+            if (!part) {
+#pragma unroll 1
+                for (int c = 0; c < rows; c += 32) {
+#pragma unroll
+                    for (int h = 0; h < (BN > 16 ? 2 : 1); ++h) {
+                        uint32_t r[16]; qg_ld16(r, src + (uint32_t)(c + 16 * h));
+                        float acc[16];
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) acc[i] = __uint_as_float(r[i]);
+                        store(c + 16 * h, acc, res[h]);
+                        __syncwarp();
+                    }
+                }
+            } else {
                 float *mine = a.scratch + (size_t)fkq_slot(a.tiles, nsb, G, me, w.tile) * fkq_part_floats(BN) + sub * 128 + q * 32 + lane;
 #pragma unroll 1
-                for (int c = 0; c < BN; c += 16) {
+                for (int c = 0; c < rows; c += 16) {
                     uint32_t r[16]; qg_ld16(r, src + (uint32_t)c);
 #pragma unroll
                     for (int i = 0; i < 16; ++i) __stcg(mine + (size_t)(c + i) * FKQ_ROWS, __uint_as_float(r[i]));
                 }
-                first = fkq_owner(a.tiles, nsb, G, w.tile * nsb); last = fkq_owner(a.tiles, nsb, G, (w.tile + 1) * nsb - 1);
+                const int first = fkq_owner(a.tiles, nsb, G, w.tile * nsb), last = fkq_owner(a.tiles, nsb, G, (w.tile + 1) * nsb - 1);
                 __threadfence();
                 __syncwarp();
                 unsigned int ticket = 0;
@@ -300,56 +373,33 @@ __global__ void __launch_bounds__(FKQ_THREADS, 1) k_qgemm(FkState *st, const __g
                     ticket = atomicAdd(a.counters + (size_t)w.tile * FKQ_EPI + ew, 1u);
                     if (ticket == (unsigned int)(last - first)) a.counters[(size_t)w.tile * FKQ_EPI + ew] = 0u;      // all parts are in: ready for the next launch
                 }
-                finish = __shfl_sync(0xffffffffu, ticket, 0) == (unsigned int)(last - first);
-                __threadfence();
-            }
-            if (finish) {
+                const bool finish = __shfl_sync(0xffffffffu, ticket, 0) == (unsigned int)(last - first);
+                if (finish) {
+                    __threadfence();
+                    fetch_all();
+                    const float *from = a.scratch + sub * 128 + q * 32 + lane;
 #pragma unroll 1
-                for (int c = 0; c < BN && m0 + c < a.m; c += 16) {
-                    float acc[16];
-                    if (!part) {
-                        uint32_t r[16]; qg_ld16(r, src + (uint32_t)c);
+                    for (int c = 0; c < rows; c += 32) {
 #pragma unroll
-                        for (int i = 0; i < 16; ++i) acc[i] = __uint_as_float(r[i]);
-                    } else {
+                        for (int h = 0; h < (BN > 16 ? 2 : 1); ++h) {
+                            float acc[16];
 #pragma unroll
-                        for (int i = 0; i < 16; ++i) acc[i] = 0.0f;
-                        for (int p = first; p <= last; ++p) {
-                            const float *from = a.scratch + (size_t)fkq_slot(a.tiles, nsb, G, p, w.tile) * fkq_part_floats(BN) + sub * 128 + q * 32 + lane;
+                            for (int i = 0; i < 16; ++i) acc[i] = 0.0f;
+                            for (int p = first; p <= last; p += 2) {          // in K order, two parts on their way
+                                const float *f0 = from + (size_t)fkq_slot(a.tiles, nsb, G, p, w.tile) * fkq_part_floats(BN), *f1 = f0;
+                                if (p < last) f1 = from + (size_t)fkq_slot(a.tiles, nsb, G, p + 1, w.tile) * fkq_part_floats(BN);
+                                float u0[16], u1[16];
 #pragma unroll
-                            for (int i = 0; i < 16; ++i) acc[i] += __ldcg(from + (size_t)(c + i) * FKQ_ROWS);
-                        }
-                    }
-                    const float xs = lane < 16 && m0 + c + lane < a.m ? __ldcg(a.xscale + m0 + c + lane) * a.wscale : 0.0f;
+                                for (int i = 0; i < 16; ++i) u0[i] = __ldcg(f0 + (size_t)(c + 16 * h + i) * FKQ_ROWS);
 #pragma unroll
-                    for (int i = 0; i < 16; ++i) acc[i] *= __shfl_sync(0xffffffffu, xs, i);
-                    if (GATEUP) {
-                        // lanes 0-7 / 16-23 hold gate rows, 8-15 / 24-31 the up rows of the same outputs: the lower half takes the even row of X of a
-                        // pair, the upper half the odd one
-                        const bool up = lane & 8;
-                        const int out = (row0 >> 4) * 8 + (lane >> 4) * 8 + (lane & 7);
+                                for (int i = 0; i < 16; ++i) u1[i] = __ldcg(f1 + (size_t)(c + 16 * h + i) * FKQ_ROWS);
 #pragma unroll
-                        for (int i = 0; i < 16; i += 2) {
-                            const float other = __shfl_xor_sync(0xffffffffu, up ? acc[i] : acc[i + 1], 8);
-                            const float gate = up ? other : acc[i], upv = up ? acc[i + 1] : other;
-                            const int m = m0 + c + i + (up ? 1 : 0);
-                            if (m < a.m && out < a.n) a.y[(size_t)m * a.n + out] = a.act == 1 ? s_act_geglu(gate, upv) : s_act_swiglu(gate, upv);
-                        }
-                    } else {
-                        const int n = row0 + lane;
-                        if (n < a.n) {
-                            if (a.residual) {
-                                uint16_t r[16];
-#pragma unroll
-                                for (int i = 0; i < 16; ++i) r[i] = m0 + c + i < a.m ? __ldcg(a.residual + (size_t)(m0 + c + i) * a.ldr + n) : (uint16_t)0;
-#pragma unroll
-                                for (int i = 0; i < 16; ++i) acc[i] += bf2f(r[i]);
+                                for (int i = 0; i < 16; ++i) { acc[i] += u0[i]; if (p < last) acc[i] += u1[i]; }
                             }
-#pragma unroll
-                            for (int i = 0; i < 16; ++i) if (m0 + c + i < a.m) a.y[(size_t)(m0 + c + i) * a.n + n] = f2bf(acc[i]);
+                            store(c + 16 * h, acc, res[h]);
+                            __syncwarp();
                         }
                     }
-                    __syncwarp();
                 }
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
