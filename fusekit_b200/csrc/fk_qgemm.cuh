@@ -2,8 +2,11 @@
 // or the gated activation of gate/up pairs, 4-bit weights in the streaming layout (units of 16 rows x 8 groups, fk_stream.cuh).
 //
 // Arithmetic: one pass of kind::f16 (fp16 operands, fp32 accumulation over all of K in tensor memory), with operands that are exact.
-//   * A weight is (q - 8) s + e, e = b + 8 s.  (q - 8) s has 3 + 8 significant bits, fp16's 11; scaled by one power of two per weight
-//     (k_weight_peak: the largest of 16 |s| and |e| lands in [2^14, 2^15)) it is exact for every s down to 2^-28 of that.
+//   * A weight is (q - 8) s + e, e = b + 8 s, after a power of two per weight row (k_row_factors: the larger of 1024 |s| and |e| lands in
+//     [2^14, 2^15)).  A nibble in the low bits of 0x6400 is 1024 + q, so one fused multiply-add gives (1024 + q) s + c; with c = -1032 s
+//     rounded towards zero to fp16, c = -1032 s + d, the result (q - 8) s + d is a multiple of s's last place below 2^11 of them, hence exact,
+//     and d (the same for all nibbles of a group: c + 960 s, the constant of nibbles 4 bits up, is exact too) is taken off e.
+//     Scales down to 2^-18 of the row's largest are exact, smaller ones carry an error of 2^-23 of the row's largest weight.
 //   * An activation is bf16: 8 bits, exact in fp16 after a power of two per row (k_stage_rows: the row's largest lands in [2^8, 2^9))
 //     for everything down to 2^-25 of the row's largest, rounded to 2^-33 of it below.
 //   * e enters as three extra k slots per group, (e_hi, e_hi, e_lo) . (X_hi, X_lo, X_hi), X the sum of the group's activations: 22 bits
@@ -12,7 +15,7 @@
 //
 // A block owns 256 weight rows (two M = 128 accumulators) x BN rows of X.  16 warps turn one unit each (16 weight rows) into fp16
 // and write it straight into tensor memory as the A operand (tcgen05.st .16x256b: the lane layout of the units is its lane layout; a ring
-// of four k-blocks); through shared memory the expanded operand costs two more crossings of it than the packed weights.  One warp
+// of four to seven k-blocks); through shared memory the expanded operand costs two more crossings of it than the packed weights.  One warp
 // fetches X by TMA (128-byte swizzle), one warp per accumulator issues its MMAs, 8 warps store finished tiles.  Weight rings are filled before
 // griddepcontrol.wait.  Every wait is bounded; when one runs out the kernel sets an error bit, waits (bounded) for its copies, frees
 // its tensor memory and returns.
@@ -29,18 +32,18 @@
 #define FKQ_EPI 8                       // storing warps
 #define FKQ_THREADS ((FKQ_DEQ + FKQ_EPI + 3) * 32)      // .. a warp for X, two for the MMAs
 #define FKQ_ROWS 256                    // weight rows of a block
-#define FKQ_AS 4                        // k-blocks of A operand in tensor memory (64 columns each)
 #define FKQ_SPIN (1u << 21)
 #define FKQ_MAX_K 32768                 // a row is staged from registers: 1024 threads x 4 vectors of 8
 #define FKQ_ERR_WAIT 0x400000u
 #define FKQ_COUNTERS 65536              // ticket words: 8 per tile that is split
 template <int BN> struct QgTile {
-    static constexpr int XS = BN >= 128 ? 4 : BN == 64 ? 8 : 12, XBYTES = BN * 128, NBUF = BN <= 64 ? 2 : 1;
-    static constexpr size_t SMEM = 1024 + (size_t)XS * XBYTES + (size_t)FKQ_DEQ * FK_STAGES * FK_UNIT_BYTES + (size_t)FKQ_EPI * BN * 4;
+    static constexpr int XG = BN >= 128 ? 1 : 3, XS = BN >= 128 ? 5 : BN == 64 ? 3 : 4, XBYTES = BN * 128;        // k-blocks per stage of X, stages, bytes of a k-block
+    static constexpr int NBUF = BN <= 64 ? 2 : 1, DCOLS = NBUF * 2 * BN, AS = (512 - DCOLS) / 64;                 // accumulators of a tile and the next, columns, k-blocks of A operand
+    static constexpr size_t SMEM = 1024 + (size_t)XS * XG * XBYTES + (size_t)FKQ_DEQ * FK_STAGES * FK_UNIT_BYTES;
 };
 __host__ __device__ inline size_t fkq_part_floats(int bn) { return (size_t)bn * FKQ_ROWS; }
 
-struct QGemmArgs { TiledW W; const float *xscale; const uint16_t *residual; uint16_t *y; float *scratch; unsigned int *counters; int m, n, ldr, act, whole, mtiles, tiles; float wmul, wscale; };
+struct QGemmArgs { TiledW W; const float *xscale; const uint16_t *residual; uint16_t *y; float *scratch; unsigned int *counters; const float *rowmul; int m, n, ldr, act, whole, mtiles, tiles; };
 
 __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
     uint32_t ok;
@@ -67,7 +70,13 @@ __device__ __forceinline__ bool qg_elect() {
 __device__ __forceinline__ void qg_mma(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t more) {
     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(more) : "memory");
 }
-__device__ __forceinline__ uint32_t h2_sub(uint32_t a, uint32_t b) { __half2 r = __hsub2(*reinterpret_cast<__half2 *>(&a), *reinterpret_cast<__half2 *>(&b)); return *reinterpret_cast<uint32_t *>(&r); }
+__device__ __forceinline__ uint32_t h2_fma(uint32_t a, uint32_t b, uint32_t c) {
+    __half2 r = __hfma2(*reinterpret_cast<__half2 *>(&a), *reinterpret_cast<__half2 *>(&b), *reinterpret_cast<__half2 *>(&c)); return *reinterpret_cast<uint32_t *>(&r);
+}
+// (w & MASK) | 0x64006400 in one instruction
+template <uint32_t MASK> __device__ __forceinline__ uint32_t qg_nibbles(uint32_t w) {
+    uint32_t r; asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(r) : "r"(w), "n"(MASK), "r"(0x64006400u)); return r;
+}
 __device__ __forceinline__ uint32_t h2_mul(uint32_t a, uint32_t b) { __half2 r = __hmul2(*reinterpret_cast<__half2 *>(&a), *reinterpret_cast<__half2 *>(&b)); return *reinterpret_cast<uint32_t *>(&r); }
 __device__ __forceinline__ uint32_t h2_pack(float lo, float hi) { __half2 r = __floats2half2_rn(lo, hi); return *reinterpret_cast<uint32_t *>(&r); }
 __device__ __forceinline__ void qg_st16(uint32_t addr, const uint32_t (&r)[16]) {
@@ -120,22 +129,22 @@ inline QPlan fkq_plan(int m, int ntiles, int nsb, int sm) {
 template <int BN, bool GATEUP>
 __global__ void __launch_bounds__(FKQ_THREADS, 1) k_qgemm(FkState *st, const __grid_constant__ CUtensorMap mx, QGemmArgs a) {
     using T = QgTile<BN>;
-    constexpr int XS = T::XS, NBUF = T::NBUF;
+    constexpr int XS = T::XS, XG = T::XG, NBUF = T::NBUF, AS = T::AS;
     extern __shared__ unsigned char qg_smem[];
-    __shared__ __align__(8) uint64_t bars[FKQ_DEQ * FK_STAGES + 2 * XS + 2 * FKQ_AS + 2 * NBUF];
+    __shared__ __align__(8) uint64_t bars[FKQ_DEQ * FK_STAGES + 2 * XS + 2 * AS + 2 * NBUF];
     __shared__ uint32_t tmem_slot;
     const int tid = threadIdx.x, lane = tid & 31, wid = __shfl_sync(0xffffffffu, tid >> 5, 0);
-    const uint32_t base = (smem_u32(qg_smem) + 1023u) & ~1023u, ring = base + XS * T::XBYTES;
-    const uint32_t wfull = smem_u32(bars), xfull = wfull + 8 * FKQ_DEQ * FK_STAGES, xempty = xfull + 8 * XS, afull = xempty + 8 * XS, aempty = afull + 8 * FKQ_AS,
-                   dfull = aempty + 8 * FKQ_AS, dempty = dfull + 8 * NBUF;
+    const uint32_t base = (smem_u32(qg_smem) + 1023u) & ~1023u, ring = base + XS * XG * T::XBYTES;
+    const uint32_t wfull = smem_u32(bars), xfull = wfull + 8 * FKQ_DEQ * FK_STAGES, xempty = xfull + 8 * XS, afull = xempty + 8 * XS, aempty = afull + 8 * AS,
+                   dfull = aempty + 8 * AS, dempty = dfull + 8 * NBUF;
     pdl_launch_dependents();
     if (tid == 0) {
         for (int i = 0; i < FKQ_DEQ * FK_STAGES; ++i) mbar_init(bars + i, 1);
         uint64_t *b = bars + FKQ_DEQ * FK_STAGES;
         for (int i = 0; i < XS; ++i) { mbar_init(b + i, 1); mbar_init(b + XS + i, 2); }
         b += 2 * XS;
-        for (int i = 0; i < FKQ_AS; ++i) { mbar_init(b + i, FKQ_DEQ); mbar_init(b + FKQ_AS + i, 2); }
-        b += 2 * FKQ_AS;
+        for (int i = 0; i < AS; ++i) { mbar_init(b + i, FKQ_DEQ); mbar_init(b + AS + i, 2); }
+        b += 2 * AS;
         for (int i = 0; i < NBUF; ++i) { mbar_init(b + i, 2); mbar_init(b + NBUF + i, FKQ_EPI); }
         mbar_fence_init();
     }
@@ -146,7 +155,7 @@ __global__ void __launch_bounds__(FKQ_THREADS, 1) k_qgemm(FkState *st, const __g
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem = tmem_slot, tmem_a = tmem + 256;
+    const uint32_t tmem = tmem_slot, tmem_a = tmem + T::DCOLS;      // accumulators, A operand
     const int nsb = a.W.nsb, G = gridDim.x, me = blockIdx.x;
     bool ok = true;
     QWork w;
@@ -155,7 +164,8 @@ __global__ void __launch_bounds__(FKQ_THREADS, 1) k_qgemm(FkState *st, const __g
         const int q = wid & 3, sub = wid >> 3, half = (wid >> 2) & 1, mine = sub * 8 + q * 2 + half;
         const uint32_t bar0 = wfull + 8 * FK_STAGES * wid, ring0 = ring + (uint32_t)(wid * FK_STAGES * FK_UNIT_BYTES);
         const uint32_t dst0 = tmem_a + ((uint32_t)(32 * q + 16 * half) << 16) + (uint32_t)(sub * 32);
-        int iv = 0, ikb = 0, issued = 0, used = 0, it = 0;
+        int iv = 0, ikb = 0, issued = 0, used = 0, as = 0, stages = 0;
+        uint32_t aph = 1u, pend = 0;                    // a ring that was never used counts as free; pend: the barrier of what is not announced yet
         QWork iw; bool more = fkq_work(a.whole, a.tiles, nsb, me, G, 0, iw);
         ikb = more ? iw.k0 : 0;
         // the next unit of this warp in the block's order of steps (tiles past the last row tile have none)
@@ -173,70 +183,88 @@ __global__ void __launch_bounds__(FKQ_THREADS, 1) k_qgemm(FkState *st, const __g
             if (++ikb == iw.k1) { more = fkq_work(a.whole, a.tiles, nsb, me, G, ++iv, iw); ikb = more ? iw.k0 : 0; }
         };
         for (int s = 0; s < FK_STAGES; ++s) issue();
-        auto slot = [&]() {                             // the next A stage is free
-            if (it >= FKQ_AS && !qg_wait(aempty + 8 * (it % FKQ_AS), (uint32_t)(it / FKQ_AS - 1) & 1u)) { ok = false; return false; }
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            return true;
-        };
-        auto publish = [&]() {
+        // A k-block is announced when the next one's values are worked out, and its slot is looked at before: both latencies pass under the
+        // arithmetic
+        auto announce = [&]() {
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
-            if (lane == 0) qg_arrive(afull + 8 * (it % FKQ_AS));
-            ++it;
+            if (lane == 0 && pend) qg_arrive(pend);
         };
+        auto claim = [&](bool free) {                   // the slot `as` may be written; a wait that runs out gives the kernel up
+            announce();
+            if (!free && !qg_wait(aempty + 8 * as, aph)) ok = false;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        };
+        auto taken = [&]() { pend = afull + 8 * as; if (++as == AS) { as = 0; aph ^= 1u; } };
         for (int v = 0; ok && fkq_work(a.whole, a.tiles, nsb, me, G, v, w); ++v) {
-            const bool have = (w.tile / a.mtiles) * 16 + mine < a.W.ntiles;
+            const int tile = (w.tile / a.mtiles) * 16 + mine;
+            const bool have = tile < a.W.ntiles;
+            const float mul = have ? __ldg(a.rowmul + tile * 16 + (lane >> 2)) : 1.0f, mul8 = have ? __ldg(a.rowmul + tile * 16 + 8 + (lane >> 2)) : 1.0f;
             for (int kb = w.k0; kb < w.k1 && ok; ++kb) {
                 const int s = used & (FK_STAGES - 1);
                 if (have && !qg_wait(bar0 + 8 * s, (uint32_t)(used / FK_STAGES) & 1u)) { ok = false; break; }
-                const uint32_t u = ring0 + (uint32_t)(s * FK_UNIT_BYTES);
-                // scales and biases of rows g and g + 8, groups 2t and 2t + 1
-                uint4 sb = make_uint4(0, 0, 0, 0);
-                if (have) sb = lds128(u + 4096 + (uint32_t)lane * 16u);
-                const float s0 = bf_lo(sb.x) * a.wmul, s1 = bf_hi(sb.x) * a.wmul, s8 = bf_lo(sb.y) * a.wmul, s9 = bf_hi(sb.y) * a.wmul;
-                const uint32_t pg = h2_pack(s0, s1), pg8 = h2_pack(s8, s9);
-#pragma unroll 2
-                for (int j = 0; j < 8; ++j) {
-                    uint4 p = make_uint4(0, 0, 0, 0);
-                    if (have) p = lds128(u + (uint32_t)(j * 512 + lane * 16));
-                    const int src = (lane & ~3) | (j >> 1);
-                    const uint32_t c = __shfl_sync(0xffffffffu, pg, src), c8 = __shfl_sync(0xffffffffu, pg8, src);
-                    const uint32_t sel = (j & 1) ? 0x3232u : 0x1010u, sg = __byte_perm(c, c, sel), sg8 = __byte_perm(c8, c8, sel);
-                    const uint32_t hg = h2_mul(sg, 0x2C002C00u), hg8 = h2_mul(sg8, 0x2C002C00u);      // scale / 16: odd nibbles stay at their place
-                    uint32_t r[16];
-                    auto expand = [&](uint32_t word, uint32_t sc, uint32_t sc16, int i) {            // pairs (0,4) (1,5) | (2,6) (3,7)
-                        const uint32_t hi = word >> 8;
-                        r[i] = h2_mul(h2_sub((word & 0x000F000Fu) | 0x64006400u, 0x64086408u), sc);
-                        r[i + 1] = h2_mul(h2_sub((word & 0x00F000F0u) | 0x64006400u, 0x64806480u), sc16);
-                        r[i + 4] = h2_mul(h2_sub((hi & 0x000F000Fu) | 0x64006400u, 0x64086408u), sc);
-                        r[i + 5] = h2_mul(h2_sub((hi & 0x00F000F0u) | 0x64006400u, 0x64806480u), sc16);
-                    };
-                    expand(p.x, sg, hg, 0); expand(p.z, sg8, hg8, 2); expand(p.y, sg, hg, 8); expand(p.w, sg8, hg8, 10);
-                    if (!slot()) break;
-                    qg_st16(dst0 + (uint32_t)((it % FKQ_AS) * 64), r);
-                    publish();
+                const uint32_t u = ring0 + (uint32_t)(s * FK_UNIT_BYTES + lane * 16);
+                // scales and biases of rows g and g + 8, groups 2t and 2t + 1: s and c for the shuffles below, e for the sums' slots
+                // (a warp without a unit works on what the ring holds: rows that nobody stores)
+                const uint4 sb = lds128(u + 4096u);
+                uint4 p = lds128(u);
+                uint32_t sc[4], cc[4]; float e[4];      // (row g, group 2t) (g, 2t + 1) (g + 8, 2t) (g + 8, 2t + 1), both halves alike
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const uint32_t sw = i < 2 ? sb.x : sb.y, bw = i < 2 ? sb.z : sb.w;
+                    const float f = i < 2 ? mul : mul8, sv = ((i & 1) ? bf_hi(sw) : bf_lo(sw)) * f, bv = ((i & 1) ? bf_hi(bw) : bf_lo(bw)) * f;
+                    const __half sh = __float2half_rn(sv), ch = __float2half_rz(-1032.0f * __half2float(sh));
+                    e[i] = fmaf(8.0f, sv, bv) - fmaf(1032.0f, __half2float(sh), __half2float(ch));
+                    sc[i] = (uint32_t)__half_as_ushort(sh) * 0x10001u; cc[i] = (uint32_t)__half_as_ushort(ch) * 0x10001u;
+                }
+#pragma unroll 1
+                for (int j = 0; j < 4; ++j) {           // groups 2j and 2j + 1
+                    const int src = (lane & ~3) | j;
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const uint4 nx = lds128(u + (uint32_t)((2 * j + h + 1) * 512));      // after the last group: the scales, not used
+                        const bool free = mbar_try(aempty + 8 * as, aph);
+                        const uint32_t sg = __shfl_sync(0xffffffffu, sc[h], src), cg = __shfl_sync(0xffffffffu, cc[h], src);
+                        const uint32_t sg8 = __shfl_sync(0xffffffffu, sc[2 + h], src), cg8 = __shfl_sync(0xffffffffu, cc[2 + h], src);
+                        // nibbles 4 bits up: (1024 + 16 q) s / 16 + c + 960 s
+                        const uint32_t hg = h2_mul(sg, 0x2C002C00u), hg8 = h2_mul(sg8, 0x2C002C00u), dg = h2_fma(sg, 0x63806380u, cg), dg8 = h2_fma(sg8, 0x63806380u, cg8);
+                        uint32_t r[16];
+                        auto expand = [&](uint32_t word, uint32_t s1, uint32_t c1, uint32_t s16, uint32_t c16, int i) {            // pairs (0,4) (1,5) | (2,6) (3,7)
+                            const uint32_t hi = word >> 8;
+                            r[i] = h2_fma(qg_nibbles<0x000F000Fu>(word), s1, c1); r[i + 1] = h2_fma(qg_nibbles<0x00F000F0u>(word), s16, c16);
+                            r[i + 4] = h2_fma(qg_nibbles<0x000F000Fu>(hi), s1, c1); r[i + 5] = h2_fma(qg_nibbles<0x00F000F0u>(hi), s16, c16);
+                        };
+                        expand(p.x, sg, cg, hg, dg, 0); expand(p.z, sg8, cg8, hg8, dg8, 2); expand(p.y, sg, cg, hg, dg, 8); expand(p.w, sg8, cg8, hg8, dg8, 10);
+                        claim(free);
+                        qg_st16(dst0 + (uint32_t)(as * 64), r);
+                        taken();
+                        p = nx;
+                    }
+                    if (!ok) break;
                 }
                 if (!ok) break;
+                stages += 9;
                 {                                       // the sums' slots: columns 8b + 2t (e_hi, e_hi) and 8b + 2t + 1 (e_lo, 0) of group 2t + b
+                    const bool free = mbar_try(aempty + 8 * as, aph);
                     uint32_t r[8];
-                    auto edge = [&](float e, uint32_t &hi, uint32_t &lo) {
-                        const float h = __half2float(__float2half_rn(e));
-                        hi = h2_pack(h, h); lo = h2_pack(e - h, 0.0f);
-                    };
-                    edge(fmaf(bf_lo(sb.z), a.wmul, 8.0f * s0), r[0], r[1]); edge(fmaf(bf_lo(sb.w), a.wmul, 8.0f * s8), r[2], r[3]);
-                    edge(fmaf(bf_hi(sb.z), a.wmul, 8.0f * s1), r[4], r[5]); edge(fmaf(bf_hi(sb.w), a.wmul, 8.0f * s9), r[6], r[7]);
-                    if (!slot()) break;
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {       // e[i] is row g + 8 (i / 2), group 2t + (i & 1)
+                        const float h = __half2float(__float2half_rn(e[i]));
+                        r[(i & 1) * 4 + (i >> 1) * 2] = h2_pack(h, h); r[(i & 1) * 4 + (i >> 1) * 2 + 1] = h2_pack(e[i] - h, 0.0f);
+                    }
+                    if (have) { ++used; __syncwarp(); issue(); }        // the unit is in registers: its ring slot is refilled
+                    claim(free);
                     asm volatile("tcgen05.st.sync.aligned.16x256b.x2.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
-                                 ::"r"(dst0 + (uint32_t)((it % FKQ_AS) * 64)), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
-                    publish();
+                                 ::"r"(dst0 + (uint32_t)(as * 64)), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
+                    taken();
                 }
-                if (have) { ++used; __syncwarp(); issue(); }
             }
+            announce(); pend = 0;                       // the tile's last
         }
         // what is still in flight lands, and the MMAs that read the last stages have been counted, before the block may leave
         for (; used < issued; ++used) if (!qg_wait(bar0 + 8 * (used & (FK_STAGES - 1)), (uint32_t)(used / FK_STAGES) & 1u)) ok = false;
-        if (ok) for (int j = it > FKQ_AS ? it - FKQ_AS : 0; j < it; ++j) if (!qg_wait(aempty + 8 * (j % FKQ_AS), (uint32_t)(j / FKQ_AS) & 1u)) ok = false;
+        if (ok) for (int j = stages > AS ? stages - AS : 0; j < stages; ++j) if (!qg_wait(aempty + 8 * (j % AS), (uint32_t)(j / AS) & 1u)) ok = false;
         if (!ok && lane == 0) atomicOr(&st->error, FKQ_ERR_WAIT);
     } else if (wid == FKQ_DEQ + FKQ_EPI) {
         // ---------------------------------------------------------------- X
@@ -245,12 +273,14 @@ __global__ void __launch_bounds__(FKQ_THREADS, 1) k_qgemm(FkState *st, const __g
             int it = 0;
             for (int v = 0; ok && fkq_work(a.whole, a.tiles, nsb, me, G, v, w); ++v) {
                 const int m0 = (w.tile % a.mtiles) * BN;
-                for (int kb = w.k0 * 9; kb < w.k1 * 9; ++kb, ++it) {
+                for (int kb = w.k0 * 9; kb < w.k1 * 9; kb += XG, ++it) {
                     const int s = it % XS;
                     if (it >= XS && !qg_wait(xempty + 8 * s, (uint32_t)(it / XS - 1) & 1u)) { ok = false; break; }
-                    qg_expect(xfull + 8 * s, (uint32_t)T::XBYTES);
-                    asm volatile("cp.async.bulk.tensor.2d.shared::cta.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-                                 ::"r"(base + s * T::XBYTES), "l"(&mx), "r"(kb * 64), "r"(m0), "r"(xfull + 8 * s) : "memory");
+                    qg_expect(xfull + 8 * s, (uint32_t)(XG * T::XBYTES));
+#pragma unroll
+                    for (int g = 0; g < XG; ++g)
+                        asm volatile("cp.async.bulk.tensor.2d.shared::cta.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+                                     ::"r"(base + (s * XG + g) * T::XBYTES), "l"(&mx), "r"((kb + g) * 64), "r"(m0), "r"(xfull + 8 * s) : "memory");
                 }
             }
             for (int j = it > XS ? it - XS : 0; j < it; ++j) if (!qg_wait((ok ? xempty : xfull) + 8 * (j % XS), (uint32_t)(j / XS) & 1u)) ok = false;
@@ -264,7 +294,7 @@ __global__ void __launch_bounds__(FKQ_THREADS, 1) k_qgemm(FkState *st, const __g
         pdl_wait();
         const int sub = wid - (FKQ_DEQ + FKQ_EPI + 1);
         const uint32_t idesc = (1u << 4) | ((uint32_t)(BN >> 3) << 17) | ((128u >> 4) << 24);          // fp16 x fp16 -> fp32
-        const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0), tma = tm + 256u + (uint32_t)(sub * 32);
+        const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0), tma = tm + (uint32_t)(T::DCOLS + sub * 32);
         const uint64_t db0 = (uint64_t)((base >> 4) & 0x3FFFu) | (1ull << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
         int s = 0, as = 0;
         uint32_t xph = 0, aph = 0;
@@ -273,25 +303,27 @@ __global__ void __launch_bounds__(FKQ_THREADS, 1) k_qgemm(FkState *st, const __g
             const int d = v % NBUF;
             if (v >= NBUF && !qg_wait(dempty + 8 * d, (uint32_t)(v / NBUF - 1) & 1u)) { ok = false; break; }
             const uint32_t dd = tm + (uint32_t)((d * 2 + sub) * BN);
-            uint32_t more = 0;                          // 0: the tile's first MMA overwrites
+            uint32_t again = 0;                         // 0: the tile's first MMA overwrites
             for (int sb = w.k0; sb < w.k1 && ok; ++sb)
 #pragma unroll 1
-                for (int kk = 0; kk < 9; ++kk) {
-                    if ((!xready && !qg_wait(xfull + 8 * s, xph)) || (!aready && !qg_wait(afull + 8 * as, aph))) { ok = false; break; }
+                for (int kk = 0, g = 0; kk < 9; ++kk) {
+                    if ((g == 0 && !xready && !qg_wait(xfull + 8 * s, xph)) || (!aready && !qg_wait(afull + 8 * as, aph))) { ok = false; break; }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint64_t db = db0 + (uint64_t)(s * (T::XBYTES >> 4));
-                    const uint32_t aa = tma + (uint32_t)(as * 64), as_bar = aempty + 8 * as, xs_bar = xempty + 8 * s;
-                    if (++s == XS) { s = 0; xph ^= 1u; }
-                    if (++as == FKQ_AS) { as = 0; aph ^= 1u; }
-                    xready = mbar_try(xfull + 8 * s, xph); aready = mbar_try(afull + 8 * as, aph);
+                    const uint64_t db = db0 + (uint64_t)((s * XG + g) * (T::XBYTES >> 4));
+                    const uint32_t aa = tma + (uint32_t)(as * 64), xs_bar = xempty + 8 * s, as_bar = aempty + 8 * as;
+                    const bool last = ++g == XG;
+                    if (last) { g = 0; if (++s == XS) { s = 0; xph ^= 1u; } xready = mbar_try(xfull + 8 * s, xph); }
+                    if (++as == AS) { as = 0; aph ^= 1u; }
+                    aready = mbar_try(afull + 8 * as, aph);
                     if (qg_elect()) {
-                        qg_mma(dd, aa, db, idesc, more);
+                        qg_mma(dd, aa, db, idesc, again);
                         qg_mma(dd, aa + 8, db + 2, idesc, 1u);
                         if (kk < 8) { qg_mma(dd, aa + 16, db + 4, idesc, 1u); qg_mma(dd, aa + 24, db + 6, idesc, 1u); }
-                        qg_commit(as_bar); qg_commit(xs_bar);
+                        qg_commit(as_bar);
+                        if (last) qg_commit(xs_bar);
                     }
                     __syncwarp();
-                    more = 1;
+                    again = 1;
                 }
             if (ok && qg_elect()) qg_commit(dfull + 8 * d);
             __syncwarp();
@@ -300,61 +332,86 @@ __global__ void __launch_bounds__(FKQ_THREADS, 1) k_qgemm(FkState *st, const __g
     } else {
         // ---------------------------------------------------------------- finished tiles: lane = weight row, registers = rows of X
         pdl_wait();
-        const int ew = wid - FKQ_DEQ, q = ew & 3, sub = ew >> 2;
-        float *factors = reinterpret_cast<float *>(qg_smem + (ring - smem_u32(qg_smem)) + (size_t)FKQ_DEQ * FK_STAGES * FK_UNIT_BYTES) + ew * BN;
+        const int ew = wid - FKQ_DEQ, q = ew & 3, sub = ew >> 2, odd = lane & 1;
+        // plain rows in pairs: neighbouring lanes trade so that each holds two weight rows of one row of X (even lanes the even one), and
+        // loads and stores are 4 bytes wide
+        const bool pairs = !GATEUP && !(a.n & 1) && !(a.ldr & 1) && !(((uintptr_t)a.y | (uintptr_t)a.residual) & 3);
         for (int v = 0; ok && fkq_work(a.whole, a.tiles, nsb, me, G, v, w); ++v) {
             const int d = v % NBUF, rt = w.tile / a.mtiles, m0 = (w.tile - rt * a.mtiles) * BN, row0 = rt * FKQ_ROWS + sub * 128 + q * 32, n = row0 + lane;
-            const bool part = w.k0 != 0 || w.k1 != nsb, adds = !GATEUP && a.residual && n < a.n;
-            uint16_t res[2][16];                        // residuals of 32 rows of X on their way
-            auto fetch = [&](int c, uint16_t (&r)[16]) {
+            const bool part = w.k0 != 0 || w.k1 != nsb;
+            const int rows = min(BN, a.m - m0);         // of X that there are
+            uint32_t res[16];                           // residual pairs of 32 rows of X on their way
+            auto fetch = [&](int c, auto &r) {
+                constexpr int N2 = sizeof(r) / 4;
 #pragma unroll
-                for (int i = 0; i < 16; ++i) r[i] = adds && m0 + c + i < a.m ? __ldcg(a.residual + (size_t)(m0 + c + i) * a.ldr + n) : (uint16_t)0;
+                for (int i = 0; i < N2; ++i)
+                    r[i] = pairs && a.residual && n - odd < a.n && c + 2 * i + odd < rows ? __ldcg(reinterpret_cast<const uint32_t *>(a.residual + (size_t)(m0 + c + 2 * i + odd) * a.ldr + n - odd)) : 0u;
             };
-            auto fetch_all = [&]() {
-                for (int i = lane; i < BN; i += 32) factors[i] = m0 + i < a.m ? __ldcg(a.xscale + m0 + i) * a.wscale : 0.0f;
-                if (!GATEUP) { fetch(0, res[0]); if (BN > 16) fetch(16, res[1]); }
-                __syncwarp();
+            float fac[(BN + 31) / 32];                  // lane -> factor of row lane, + 32 ..
+#pragma unroll
+            for (int i = 0; i < (BN + 31) / 32; ++i) fac[i] = 32 * i + lane < rows ? __ldcg(a.xscale + m0 + 32 * i + lane) : 0.0f;
+            auto factors = [&](int c) {                 // of the 32 rows around row c
+                float f = fac[0];
+#pragma unroll
+                for (int i = 1; i < (BN + 31) / 32; ++i) if (c >= 32 * i) f = fac[i];
+                return f;
             };
-            if (!part) fetch_all();                     // under the tile's MMAs
+            const float rmul = row0 + lane < a.W.ntiles * 16 ? __uint_as_float(0x7F000000u - __float_as_uint(__ldg(a.rowmul + row0 + lane))) : 0.0f;       // 2^-k of 2^k
+            if (!GATEUP && !part) fetch(0, res);        // under the tile's MMAs
             if (!qg_wait(dfull + 8 * d, (uint32_t)(v / NBUF) & 1u)) { ok = false; break; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t src = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)((d * 2 + sub) * BN);
-            const int rows = min(BN, a.m - m0);         // of X that there are
-            auto store = [&](int c, float (&acc)[16], uint16_t (&r)[16]) {
+            // rows c .. of X, whose factors lanes f0 .. hold; r: their residual pairs
+            auto store = [&](int c, int f0, float factor, auto &acc, const uint32_t *r) {
+                constexpr int NM = sizeof(acc) / 4;
 #pragma unroll
-                for (int i = 0; i < 16; i += 4) {
-                    const float4 f = *reinterpret_cast<const float4 *>(factors + c + i);
-                    acc[i] *= f.x; acc[i + 1] *= f.y; acc[i + 2] *= f.z; acc[i + 3] *= f.w;
-                }
+                for (int i = 0; i < NM; ++i) acc[i] = acc[i] * __shfl_sync(0xffffffffu, factor, f0 + i) * rmul;
                 if (GATEUP) {
                     // lanes 0-7 / 16-23 hold gate rows, 8-15 / 24-31 the up rows of the same outputs: the lower half takes the even row of X of a
                     // pair, the upper half the odd one
                     const bool up = lane & 8;
                     const int out = (row0 >> 4) * 8 + (lane >> 4) * 8 + (lane & 7);
 #pragma unroll
-                    for (int i = 0; i < 16; i += 2) {
+                    for (int i = 0; i < NM; i += 2) {
                         const float other = __shfl_xor_sync(0xffffffffu, up ? acc[i] : acc[i + 1], 8);
                         const float gate = up ? other : acc[i], upv = up ? acc[i + 1] : other;
                         const int m = c + i + (up ? 1 : 0);
                         if (m < rows && out < a.n) a.y[(size_t)(m0 + m) * a.n + out] = a.act == 1 ? s_act_geglu(gate, upv) : s_act_swiglu(gate, upv);
                     }
-                } else {
+                } else if (pairs) {
 #pragma unroll
-                    for (int i = 0; i < 16; ++i) if (n < a.n && c + i < rows) a.y[(size_t)(m0 + c + i) * a.n + n] = f2bf(acc[i] + bf2f(r[i]));
-                    if (c + 32 < rows) fetch(c + 32, r);
+                    for (int i = 0; i < NM; i += 2) {
+                        const float other = __shfl_xor_sync(0xffffffffu, odd ? acc[i] : acc[i + 1], 1);
+                        const float lo = (odd ? other : acc[i]) + bf_lo(r[i >> 1]), hi = (odd ? acc[i + 1] : other) + bf_hi(r[i >> 1]);
+                        const int m = c + i + odd;
+                        if (m < rows && n - odd < a.n) *reinterpret_cast<uint32_t *>(a.y + (size_t)(m0 + m) * a.n + n - odd) = (uint32_t)f2bf(lo) | ((uint32_t)f2bf(hi) << 16);
+                    }
+                } else if (n < a.n) {
+#pragma unroll
+                    for (int i = 0; i < NM; ++i) if (c + i < rows) {
+                        const float add = a.residual ? bf2f(__ldcg(a.residual + (size_t)(m0 + c + i) * a.ldr + n)) : 0.0f;
+                        a.y[(size_t)(m0 + c + i) * a.n + n] = f2bf(acc[i] + add);
+                    }
                 }
+                __syncwarp();
             };
             if (!part) {
 #pragma unroll 1
-                for (int c = 0; c < rows; c += 32) {
+                for (int cc = 0; cc < rows; cc += 32) {
+                    const float f = factors(cc);
 #pragma unroll
                     for (int h = 0; h < (BN > 16 ? 2 : 1); ++h) {
-                        uint32_t r[16]; qg_ld16(r, src + (uint32_t)(c + 16 * h));
+                        const int c = cc + 16 * h;
+                        uint32_t r[16]; qg_ld16(r, src + (uint32_t)c);
                         float acc[16];
 #pragma unroll
                         for (int i = 0; i < 16; ++i) acc[i] = __uint_as_float(r[i]);
-                        store(c + 16 * h, acc, res[h]);
-                        __syncwarp();
+                        store(c, 16 * h, f, acc, res + 8 * h);
+                        if (!GATEUP) {
+                            uint32_t nx[8]; fetch(c + 32, nx);
+#pragma unroll
+                            for (int i = 0; i < 8; ++i) res[8 * h + i] = nx[i];
+                        }
                     }
                 }
             } else {
@@ -376,29 +433,29 @@ __global__ void __launch_bounds__(FKQ_THREADS, 1) k_qgemm(FkState *st, const __g
                 const bool finish = __shfl_sync(0xffffffffu, ticket, 0) == (unsigned int)(last - first);
                 if (finish) {
                     __threadfence();
-                    fetch_all();
                     const float *from = a.scratch + sub * 128 + q * 32 + lane;
 #pragma unroll 1
-                    for (int c = 0; c < rows; c += 32) {
+                    for (int c = 0; c < rows; c += 8) {
+                        uint32_t r8[4];
+                        if (!GATEUP) fetch(c, r8);
+                        float acc[8];
 #pragma unroll
-                        for (int h = 0; h < (BN > 16 ? 2 : 1); ++h) {
-                            float acc[16];
+                        for (int i = 0; i < 8; ++i) acc[i] = 0.0f;
+#pragma unroll 1
+                        for (int p = first; p <= last; p += 3) {          // in K order, three parts on their way
+                            float u[3][8];
 #pragma unroll
-                            for (int i = 0; i < 16; ++i) acc[i] = 0.0f;
-                            for (int p = first; p <= last; p += 2) {          // in K order, two parts on their way
-                                const float *f0 = from + (size_t)fkq_slot(a.tiles, nsb, G, p, w.tile) * fkq_part_floats(BN), *f1 = f0;
-                                if (p < last) f1 = from + (size_t)fkq_slot(a.tiles, nsb, G, p + 1, w.tile) * fkq_part_floats(BN);
-                                float u0[16], u1[16];
+                            for (int h = 0; h < 3; ++h) {
+                                const float *f = from + (size_t)fkq_slot(a.tiles, nsb, G, min(p + h, last), w.tile) * fkq_part_floats(BN) + (size_t)c * FKQ_ROWS;
 #pragma unroll
-                                for (int i = 0; i < 16; ++i) u0[i] = __ldcg(f0 + (size_t)(c + 16 * h + i) * FKQ_ROWS);
-#pragma unroll
-                                for (int i = 0; i < 16; ++i) u1[i] = __ldcg(f1 + (size_t)(c + 16 * h + i) * FKQ_ROWS);
-#pragma unroll
-                                for (int i = 0; i < 16; ++i) { acc[i] += u0[i]; if (p < last) acc[i] += u1[i]; }
+                                for (int i = 0; i < 8; ++i) u[h][i] = __ldcg(f + (size_t)i * FKQ_ROWS);
                             }
-                            store(c + 16 * h, acc, res[h]);
-                            __syncwarp();
+#pragma unroll
+                            for (int h = 0; h < 3; ++h)
+#pragma unroll
+                                for (int i = 0; i < 8; ++i) if (p + h <= last) acc[i] += u[h][i];
                         }
+                        store(c, c & 31, factors(c), acc, r8);
                     }
                 }
             }
@@ -414,22 +471,29 @@ __global__ void __launch_bounds__(FKQ_THREADS, 1) k_qgemm(FkState *st, const __g
     if (wid == FKQ_DEQ) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
 }
 
-// The largest of 16 |s| and |b + 8 s| of a weight (non-finite ones left out), as the bits of a non-negative float: what its common
-// power of two is chosen from.  Once per weight, when it is laid out.
-__global__ void k_weight_peak(const uint4 *units, long long nunits, unsigned int *peak) {
-    float top = 0.0f;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nunits * 32; i += (long long)gridDim.x * blockDim.x) {
-        const uint4 v = units[(i >> 5) * FK_UNIT_VEC + 256 + (i & 31)];
+// The power of two of every weight row (in the order of the units): what brings the larger of 1024 |s| and |b + 8 s| over the row into
+// [2^14, 2^15); values that are not finite do not count.  Once per weight, when it is laid out; a warp per unit row of 16.
+__global__ void __launch_bounds__(256) k_row_factors(const uint4 *units, float *mul, int ntiles, int nsb) {
+    const int tile = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (tile >= ntiles) return;
+    float top[2] = {0.0f, 0.0f};
+    for (int i = 0; i < nsb; ++i) {
+        const uint4 v = units[((size_t)tile * nsb + i) * FK_UNIT_VEC + 256 + lane];
         const uint32_t s[2] = {v.x, v.y}, b[2] = {v.z, v.w};
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-            const float c[4] = {16.0f * fabsf(bf_lo(s[h])), 16.0f * fabsf(bf_hi(s[h])), fabsf(fmaf(8.0f, bf_lo(s[h]), bf_lo(b[h]))), fabsf(fmaf(8.0f, bf_hi(s[h]), bf_hi(b[h])))};
+            const float c[4] = {1024.0f * fabsf(bf_lo(s[h])), 1024.0f * fabsf(bf_hi(s[h])), fabsf(fmaf(8.0f, bf_lo(s[h]), bf_lo(b[h]))), fabsf(fmaf(8.0f, bf_hi(s[h]), bf_hi(b[h])))};
 #pragma unroll
-            for (int j = 0; j < 4; ++j) if (c[j] <= 3.0e38f) top = fmaxf(top, c[j]);
+            for (int j = 0; j < 4; ++j) if (c[j] <= 3.0e38f) top[h] = fmaxf(top[h], c[j]);
         }
     }
-    top = warp_max(top);
-    if ((threadIdx.x & 31) == 0) atomicMax(peak, __float_as_uint(top));
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        top[h] = fmaxf(top[h], __shfl_xor_sync(0xffffffffu, top[h], 1)); top[h] = fmaxf(top[h], __shfl_xor_sync(0xffffffffu, top[h], 2));
+        int e = top[h] > 0.0f ? (int)(__float_as_uint(top[h]) >> 23) - 127 : 14;
+        e = e < -110 ? -110 : e;                        // factor and inverse stay normal numbers
+        if ((lane & 3) == 0) mul[tile * 16 + h * 8 + (lane >> 2)] = __uint_as_float((uint32_t)(127 + 14 - e) << 23);
+    }
 }
 
 // Rows of X as the product reads them: fp16 scaled by a power of two per row, in the k order in which the nibble pairs come out of

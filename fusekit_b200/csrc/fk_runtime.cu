@@ -73,7 +73,7 @@ struct Weight {
     // tiled layout (fk_stream.cuh): set by fk_weight_finalize / fk_weight_pair for 4- and 8-bit weights
     bool tiled = false; uint4 *units = nullptr; int ntiles = 0, nsb = 0; size_t unit_bytes = 0;
     int rows_kind = FK_ROWS_PLAIN, hd = 0, n_rot = 0;
-    float peak = 0.0f;                          // 4-bit streaming layout: what the fp16 operand's power of two is chosen from (k_weight_peak)
+    float *rowmul = nullptr;                    // 4-bit streaming layout: the power of two of every row's fp16 operand (k_row_factors)
     WView view() const { WView v; v.w = w; v.s = s; v.b = b; v.n = n; v.k = k; v.bits = bits; return v; }
     TiledW tview() const { TiledW t; t.units = units; t.ntiles = ntiles; t.nsb = nsb; t.n = (int)n; t.k = (int)k; t.bits = bits;
                            t.rows_kind = rows_kind; t.hd = hd; t.n_rot = n_rot; return t; }
@@ -90,7 +90,7 @@ struct Ctx {
     uint32_t *pinned = nullptr;                 // host staging for state / history
     std::vector<Weight> weights; std::vector<Graph> graphs; std::vector<void *> allocs;
     bool pending = false; bool pdl = true; int sm_count = 148;
-    float *qg_scratch = nullptr; unsigned int *qg_counters = nullptr; unsigned int *qg_peak = nullptr;      // of the staged products
+    float *qg_scratch = nullptr; unsigned int *qg_counters = nullptr;      // of the staged products
     float *qmm_scratch = nullptr; unsigned int *qmm_counters = nullptr;   // K-split partial sums and tickets of the several-row projection
     bool use_tiled = true; int stages = FK_STAGES; int force_warps = 0; int force_split = -1; bool qmm_tc = false; int wide_upto = 3; bool sdpa_cluster = true; bool sdpa_mma = true; int sdpa_cl = 0;
     ncclComm_t comm = nullptr; int rank = 0, world = 1;
@@ -140,8 +140,7 @@ extern "C" fk_status fk_open(int device, fk_handle *out) {
     CU(cudaMalloc(&c->qmm_scratch, sizeof(float) * 2 * c->sm_count * FK_QMM_PART_FLOATS));
     CU(cudaMalloc(&c->qmm_counters, sizeof(unsigned int) * 2 * c->sm_count)); CU(cudaMemset(c->qmm_counters, 0, sizeof(unsigned int) * 2 * c->sm_count));
     CU(cudaMalloc(&c->qg_scratch, sizeof(float) * 2 * c->sm_count * fkq_part_floats(128)));
-    CU(cudaMalloc(&c->qg_counters, sizeof(unsigned int) * (FKQ_COUNTERS + 1))); CU(cudaMemset(c->qg_counters, 0, sizeof(unsigned int) * (FKQ_COUNTERS + 1)));
-    c->qg_peak = c->qg_counters + FKQ_COUNTERS;
+    CU(cudaMalloc(&c->qg_counters, sizeof(unsigned int) * FKQ_COUNTERS)); CU(cudaMemset(c->qg_counters, 0, sizeof(unsigned int) * FKQ_COUNTERS));
     CU(cudaMalloc(&c->history, sizeof(uint32_t) * c->hist_cap)); CU(cudaMemset(c->history, 0, sizeof(uint32_t) * c->hist_cap));
     CU(cudaMallocHost(&c->pinned, sizeof(uint32_t) * (c->hist_cap + 64)));
     const char *e = getenv("FK_PDL"); if (e && e[0] == '0') c->pdl = false;
@@ -184,7 +183,7 @@ extern "C" fk_status fk_close(fk_handle h) {
     CTX(h);
     cudaStreamSynchronize(c->stream);
     for (auto &g : c->graphs) { if (g.exec) cudaGraphExecDestroy(g.exec); if (g.graph) cudaGraphDestroy(g.graph); }
-    for (auto &w : c->weights) { cudaFree(w.w); cudaFree(w.s); cudaFree(w.b); cudaFree(w.units); }
+    for (auto &w : c->weights) { cudaFree(w.w); cudaFree(w.s); cudaFree(w.b); cudaFree(w.units); cudaFree(w.rowmul); }
     for (void *p : c->allocs) cudaFree(p);
     if (c->comm && g_nccl.CommDestroy) g_nccl.CommDestroy(c->comm);
     for (void *p : c->ipc_open) cudaIpcCloseMemHandle(p);
@@ -329,13 +328,9 @@ static fk_status repack(Ctx *c, Weight *dstw, const Weight *a, const Weight *b2)
                                                                         dstw->rows_kind, dstw->hd, dstw->n_rot);
     CU(cudaGetLastError());
     if (a->bits == 4) {
-        unsigned int peak = 0;
-        CU(cudaMemsetAsync(c->qg_peak, 0, sizeof peak, c->stream));
-        k_weight_peak<<<2 * c->sm_count, 256, 0, c->stream>>>(dstw->units, (long long)dstw->ntiles * dstw->nsb, c->qg_peak);
+        CU(cudaMalloc(&dstw->rowmul, (size_t)dstw->ntiles * 16 * sizeof(float)));
+        k_row_factors<<<(dstw->ntiles + 7) / 8, 256, 0, c->stream>>>(dstw->units, dstw->rowmul, dstw->ntiles, dstw->nsb);
         CU(cudaGetLastError());
-        CU(cudaMemcpyAsync(&peak, c->qg_peak, sizeof peak, cudaMemcpyDeviceToHost, c->stream));
-        CU(cudaStreamSynchronize(c->stream));
-        memcpy(&dstw->peak, &peak, sizeof peak);
     }
     CU(cudaStreamSynchronize(c->stream));
     dstw->tiled = true;
@@ -469,9 +464,7 @@ static fk_status run_staged(Ctx *c, const Weight *w, bool gateup, const void *xs
     if (w->k != k || w->n != (gateup ? 2LL : 1LL) * n || m <= 0 || !xs || !xscale || !y || ((uintptr_t)xs & 15)) return fail(FK_ERR_VALUE, "staged product: shape mismatch");
     if (k > FKQ_MAX_K) return fail(FK_ERR_VALUE, "staged product: at most %d columns", FKQ_MAX_K);
     const QPlan p = fkq_plan(m, w->ntiles, w->nsb, c->sm_count);
-    int ex = 0;
-    if (w->peak > 0.0f) { frexpf(w->peak, &ex); ex = ex < -100 ? -100 : ex > 110 ? 110 : ex; } else ex = 15;      // peak in [2^(ex-1), 2^ex)
-    QGemmArgs a{w->tview(), xscale, residual, y, c->qg_scratch, c->qg_counters, m, n, ldr, act, p.whole, p.mtiles, p.tiles, ldexpf(1.0f, 15 - ex), ldexpf(1.0f, ex - 15)};
+    QGemmArgs a{w->tview(), xscale, residual, y, c->qg_scratch, c->qg_counters, w->rowmul, m, n, ldr, act, p.whole, p.mtiles, p.tiles};
     CUtensorMap mx;
     if (!fkl_tensor_map(&mx, xs, m, (long long)w->nsb * FKQ_SB, (long long)w->nsb * FKQ_SB, p.bn, true)) return fail(FK_ERR_VALUE, "staged product: tensor map refused");
     *e = p.bn == 16 ? launch_qgemm<16>(c, p, gateup, mx, a) : p.bn == 32 ? launch_qgemm<32>(c, p, gateup, mx, a) : p.bn == 64 ? launch_qgemm<64>(c, p, gateup, mx, a) : launch_qgemm<128>(c, p, gateup, mx, a);
