@@ -647,6 +647,55 @@ __global__ void __launch_bounds__(FK_SDPA_THREADS) k_sdpa_decode_q(const FkState
 __host__ __device__ inline size_t sdpa_cl_smem_bytes(int G, int hd) {
     return sizeof(float) * (size_t)(G * (hd + 16) + FK_SDPA_CW * G * (hd + 2) + G * (hd + 2) + FK_SDPA_CW * G + G + 16);
 }
+// Fold of an attention cluster whose warps left (m, l, o[HD]) per head in wpart: the warps of this CTA into cpart (weights
+// e^(m_w - M) once per (warp, head), then every thread sums its outputs), then this CTA's slice of the outputs over all CTAs.
+template <int HD, int CLMAX>
+__device__ __forceinline__ void cluster_fold(cg::cluster_group &cluster, int G, int kvh, int k_begin, int k_end, const float *wpart, float *cpart, float *wexp,
+                                             uint16_t *out, unsigned long long *tl) {
+    constexpr int NT = FK_SDPA_CW * 32;
+    const int tid = threadIdx.x, rank = (int)cluster.block_rank(), CL = (int)cluster.num_blocks(), stride = HD + 2;
+    const int nwp = min(FK_SDPA_CW, (k_end - k_begin + FK_SDPA_KPW - 1) / FK_SDPA_KPW);      // warps that saw keys
+    if (tid < G) {
+        float M = -INFINITY;
+        for (int w = 0; w < nwp; ++w) M = fmaxf(M, wpart[(w * G + tid) * stride]);
+        float L = 0.0f;
+        for (int w = 0; w < nwp; ++w) {
+            const float *pw = wpart + (w * G + tid) * stride;
+            const float e = pw[0] == -INFINITY ? 0.0f : expf(pw[0] - M);
+            wexp[w * G + tid] = e; L = fmaf(pw[1], e, L);
+        }
+        cpart[tid * stride] = M; cpart[tid * stride + 1] = L;
+    }
+    __syncthreads();
+    for (int i = tid; i < G * HD; i += NT) {
+        const int g = i / HD, d = i - g * HD;
+        float O = 0.0f;
+        for (int w = 0; w < nwp; ++w) O = fmaf(wpart[(w * G + g) * stride + 2 + d], wexp[w * G + g], O);
+        cpart[g * stride + 2 + d] = O;
+    }
+    sd_stamp(tl, 3);
+    cluster.sync();
+    sd_stamp(tl, 4);
+    const int total = G * HD, per = (total + CL - 1) / CL;
+    for (int i = rank * per + tid; i < min(total, (rank + 1) * per); i += NT) {      // fold the CTAs: this CTA's slice of outputs
+        const int g = i / HD, d = i - g * HD;
+        float mm[CLMAX], ll[CLMAX], oo[CLMAX];
+#pragma unroll
+        for (int r = 0; r < CLMAX; ++r) {
+            if (r < CL) { const float *rp = cluster.map_shared_rank(cpart, r) + g * stride; mm[r] = rp[0]; ll[r] = rp[1]; oo[r] = rp[2 + d]; }
+            else { mm[r] = -INFINITY; ll[r] = 0.0f; oo[r] = 0.0f; }
+        }
+        float M = -INFINITY;
+#pragma unroll
+        for (int r = 0; r < CLMAX; ++r) M = fmaxf(M, mm[r]);
+        float L = 0.0f, O = 0.0f;
+#pragma unroll
+        for (int r = 0; r < CLMAX; ++r) { const float e = mm[r] == -INFINITY ? 0.0f : expf(mm[r] - M); L = fmaf(ll[r], e, L); O = fmaf(oo[r], e, O); }
+        out[(kvh * G + g) * HD + d] = f2bf(O * __fdiv_rn(1.0f, L));
+    }
+    cluster.sync();                                      // peers may still be reading this CTA's partial
+    sd_stamp(tl, 6);
+}
 // Split-K GQA decode attention on a thread-block cluster: the CTAs of a cluster share one kv head and take
 // contiguous key ranges; inside a CTA every warp runs an online softmax over 8-key blocks, four lanes per key for
 // the scores (s = dot(q,k)*scale in fp32) and head_dim/32 output dims per lane for p*V, with running (m, l, o)
@@ -772,48 +821,129 @@ __global__ void __launch_bounds__(FK_SDPA_CW * 32) k_sdpa_cluster(const FkState 
         for (int j = 0; j < DPL; ++j) w[2 + lane * DPL + j] = o[g][j];
     }
     __syncthreads();
-    // fold the warps of this CTA: weights e^(m_w - M) once per (warp, head), then every thread sums its outputs
-    const int nwp = min(FK_SDPA_CW, (k_end - k_begin + FK_SDPA_KPW - 1) / FK_SDPA_KPW);      // warps that saw keys
-    if (tid < G) {
-        float M = -INFINITY;
-        for (int w = 0; w < nwp; ++w) M = fmaxf(M, wpart[(w * G + tid) * stride]);
-        float L = 0.0f;
-        for (int w = 0; w < nwp; ++w) {
-            const float *pw = wpart + (w * G + tid) * stride;
-            const float e = pw[0] == -INFINITY ? 0.0f : expf(pw[0] - M);
-            wexp[w * G + tid] = e; L = fmaf(pw[1], e, L);
+    cluster_fold<HD, FK_SDPA_CL>(cluster, G, kvh, k_begin, k_end, wpart, cpart, wexp, a.out, a.tl);
+}
+
+// The same over a quantised cache (layout and dequantisation of k_sdpa_decode_q: every element is float(code) * s + b, rounded to fp32
+// twice).  Four lanes share a key's scores, a lane owns HD / 32 value columns; packed words and scales of the next keys are requested as
+// soon as the registers of the current ones are read (keys before the softmax, values after the sums).  Bound by the latency of the
+// few rounds a warp makes and by the multiply-adds (2 G per element on the CUDA cores, in fp32).  Everything goes through L2: a
+// line of scales holds many keys, the newest among them, so none of it may be kept from before the dependency wait in L1.
+template <int BITS, int HD, int MAXG>
+__global__ void __launch_bounds__(FK_SDPA_CW * 32) k_sdpa_cluster_q(const FkState *st, SdpaQArgs a) {
+    extern __shared__ float sm[];
+    cg::cluster_group cluster = cg::this_cluster();
+    constexpr int DPL = HD / 32, NT = FK_SDPA_CW * 32, PER = 32 / BITS, NW = HD / PER, NG = HD / 64;      // columns a lane, codes a word, words and groups a row
+    constexpr int KW = NW / 4, VB = DPL * BITS / 8;                       // words of a key a lane reads, bytes of a value row a lane reads
+    constexpr uint32_t MASK = (1u << BITS) - 1u;
+    const int G = a.n_q / a.n_kv, kvh = blockIdx.y, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const int rank = (int)cluster.block_rank(), CL = (int)cluster.num_blocks(), stride = HD + 2;
+    constexpr int QS = HD + 16, QP = HD / 4 + 4;
+    float *qs = sm, *wpart = qs + G * QS, *cpart = wpart + FK_SDPA_CW * G * stride, *wexp = cpart + G * stride;
+    pdl_launch_dependents();
+    const uint32_t pos = st->offset;
+    const int kv_len = (int)min(pos + 1u, (uint32_t)a.capacity), newest = (int)(pos % (uint32_t)a.capacity);
+    const int kpc = ((kv_len + CL * FK_SDPA_KPW - 1) / (CL * FK_SDPA_KPW)) * FK_SDPA_KPW;
+    const int k_begin = rank * kpc, k_end = min(kv_len, k_begin + kpc);
+    const size_t row0 = (size_t)kvh * a.capacity;
+    const int part = lane & 3, kl = lane >> 2, kg = part * (HD / 4) / 64, vg = lane * DPL / 64;      // group of the lane's key and value columns
+    uint32_t kw[KW], ksb, vw[FK_SDPA_KPW], vw8[FK_SDPA_KPW], vsb[FK_SDPA_KPW];            // scale in the low half, bias in the high half
+    auto load_k = [&](int kb) {                         // keys past the end repeat the last one: masked below
+        const size_t r = row0 + min(kb + kl, k_end - 1);
+        const uint32_t *src = a.kp + r * NW + part * KW;
+        if (KW % 4 == 0) {
+#pragma unroll
+            for (int c = 0; c < KW / 4; ++c) { const uint4 v = __ldcg(reinterpret_cast<const uint4 *>(src) + c); kw[4 * c % KW] = v.x; kw[(4 * c + 1) % KW] = v.y; kw[(4 * c + 2) % KW] = v.z; kw[(4 * c + 3) % KW] = v.w; }
+        } else {
+#pragma unroll
+            for (int c = 0; c < KW; ++c) kw[c] = __ldcg(src + c);
         }
-        cpart[tid * stride] = M; cpart[tid * stride + 1] = L;
+        ksb = (uint32_t)__ldcg(a.ks + r * NG + kg) | ((uint32_t)__ldcg(a.kb + r * NG + kg) << 16);
+    };
+    auto load_v = [&](int kb) {
+#pragma unroll
+        for (int kk = 0; kk < FK_SDPA_KPW; ++kk) {
+            const size_t r = row0 + min(kb + kk, k_end - 1);
+            const unsigned char *src = reinterpret_cast<const unsigned char *>(a.vp + r * NW) + lane * VB;
+            if (VB == 8) { const uint2 v = __ldcg(reinterpret_cast<const uint2 *>(src)); vw[kk] = v.x; vw8[kk] = v.y; }
+            else vw[kk] = VB == 4 ? __ldcg(reinterpret_cast<const uint32_t *>(src)) : VB == 2 ? (uint32_t)__ldcg(reinterpret_cast<const uint16_t *>(src)) : (uint32_t)__ldcg(src);
+            vsb[kk] = (uint32_t)__ldcg(a.vs + r * NG + vg) | ((uint32_t)__ldcg(a.vb + r * NG + vg) << 16);
+        }
+    };
+    int kb = k_begin + wid * FK_SDPA_KPW;
+    const bool early = kb < k_end && !(newest >= kb && newest < kb + FK_SDPA_KPW);      // every row but the newest predates the kernels in flight
+    if (early) { load_k(kb); load_v(kb); }
+    pdl_wait();
+    for (int i = tid; i < G * HD; i += NT) { const int g = i / HD, d = i - g * HD; qs[g * QS + (d / (HD / 4)) * QP + d % (HD / 4)] = bf2f(a.q[kvh * G * HD + i]); }
+    if (kb < k_end && !early) { load_k(kb); load_v(kb); }
+    float m[MAXG], l[MAXG], o[MAXG][DPL];
+#pragma unroll
+    for (int g = 0; g < MAXG; ++g) { m[g] = -INFINITY; l[g] = 0.0f;
+#pragma unroll
+        for (int j = 0; j < DPL; ++j) o[g][j] = 0.0f; }
+    __syncthreads();
+    for (; kb < k_end; kb += FK_SDPA_CW * FK_SDPA_KPW) {
+        const bool valid = kb + kl < k_end, again = kb + FK_SDPA_CW * FK_SDPA_KPW < k_end;
+        float dot[MAXG];
+#pragma unroll
+        for (int g = 0; g < MAXG; ++g) dot[g] = 0.0f;
+        const float s = bf_lo(ksb), b = bf_hi(ksb);
+#pragma unroll
+        for (int c = 0; c < HD / 16; ++c) {             // four columns at a time
+            float kf[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) { const int e = 4 * c + j; kf[j] = __fadd_rn(__fmul_rn((float)((kw[e / PER] >> ((e % PER) * BITS)) & MASK), s), b); }
+            const float *qp = qs + part * QP + c * 4;
+#pragma unroll
+            for (int g = 0; g < MAXG; ++g) if (g < G) {
+                const float4 q = *reinterpret_cast<const float4 *>(qp + g * QS);
+                dot[g] = fmaf(q.x, kf[0], dot[g]); dot[g] = fmaf(q.y, kf[1], dot[g]); dot[g] = fmaf(q.z, kf[2], dot[g]); dot[g] = fmaf(q.w, kf[3], dot[g]);
+            }
+        }
+        if (again) load_k(kb + FK_SDPA_CW * FK_SDPA_KPW);
+        float p[MAXG];
+#pragma unroll
+        for (int g = 0; g < MAXG; ++g) if (g < G) {
+            float d = dot[g];
+            d += __shfl_xor_sync(0xffffffffu, d, 1); d += __shfl_xor_sync(0xffffffffu, d, 2);
+            const float sv = valid ? d * a.scale : -INFINITY;
+            float mb = sv;
+            mb = fmaxf(mb, __shfl_xor_sync(0xffffffffu, mb, 4)); mb = fmaxf(mb, __shfl_xor_sync(0xffffffffu, mb, 8));
+            mb = fmaxf(mb, __shfl_xor_sync(0xffffffffu, mb, 16));
+            const float mn = fmaxf(m[g], mb), alpha = expf(m[g] - mn);      // finite: the keys hold a valid one
+            p[g] = valid ? expf(sv - mn) : 0.0f;
+            float ls = p[g];
+            ls += __shfl_xor_sync(0xffffffffu, ls, 4); ls += __shfl_xor_sync(0xffffffffu, ls, 8); ls += __shfl_xor_sync(0xffffffffu, ls, 16);
+            l[g] = fmaf(l[g], alpha, ls); m[g] = mn;
+#pragma unroll
+            for (int j = 0; j < DPL; ++j) o[g][j] *= alpha;
+        }
+#pragma unroll
+        for (int kk = 0; kk < FK_SDPA_KPW; ++kk) {
+            float vf[DPL];
+#pragma unroll
+            for (int j = 0; j < DPL; ++j) {
+                const uint32_t word = j * BITS < 32 ? vw[kk] : vw8[kk];
+                vf[j] = __fadd_rn(__fmul_rn((float)((word >> (j * BITS % 32)) & MASK), bf_lo(vsb[kk])), bf_hi(vsb[kk]));
+            }
+#pragma unroll
+            for (int g = 0; g < MAXG; ++g) if (g < G) {
+                const float pk = __shfl_sync(0xffffffffu, p[g], kk * 4);
+#pragma unroll
+                for (int j = 0; j < DPL; ++j) o[g][j] = fmaf(pk, vf[j], o[g][j]);
+            }
+        }
+        if (again) load_v(kb + FK_SDPA_CW * FK_SDPA_KPW);
+    }
+#pragma unroll
+    for (int g = 0; g < MAXG; ++g) if (g < G) {
+        float *w = wpart + (wid * G + g) * stride;
+        if (lane == 0) { w[0] = m[g]; w[1] = l[g]; }
+#pragma unroll
+        for (int j = 0; j < DPL; ++j) w[2 + lane * DPL + j] = o[g][j];
     }
     __syncthreads();
-    for (int i = tid; i < G * HD; i += NT) {
-        const int g = i / HD, d = i - g * HD;
-        float O = 0.0f;
-        for (int w = 0; w < nwp; ++w) O = fmaf(wpart[(w * G + g) * stride + 2 + d], wexp[w * G + g], O);
-        cpart[g * stride + 2 + d] = O;
-    }
-    sd_stamp(a.tl, 3);
-    cluster.sync();
-    sd_stamp(a.tl, 4);
-    const int total = G * HD, per = (total + CL - 1) / CL;
-    for (int i = rank * per + tid; i < min(total, (rank + 1) * per); i += NT) {      // fold the CTAs: this CTA's slice of outputs
-        const int g = i / HD, d = i - g * HD;
-        float mm[FK_SDPA_CL], ll[FK_SDPA_CL], oo[FK_SDPA_CL];
-#pragma unroll
-        for (int r = 0; r < FK_SDPA_CL; ++r) {
-            if (r < CL) { const float *rp = cluster.map_shared_rank(cpart, r) + g * stride; mm[r] = rp[0]; ll[r] = rp[1]; oo[r] = rp[2 + d]; }
-            else { mm[r] = -INFINITY; ll[r] = 0.0f; oo[r] = 0.0f; }
-        }
-        float M = -INFINITY;
-#pragma unroll
-        for (int r = 0; r < FK_SDPA_CL; ++r) M = fmaxf(M, mm[r]);
-        float L = 0.0f, O = 0.0f;
-#pragma unroll
-        for (int r = 0; r < FK_SDPA_CL; ++r) { const float e = mm[r] == -INFINITY ? 0.0f : expf(mm[r] - M); L = fmaf(ll[r], e, L); O = fmaf(oo[r], e, O); }
-        a.out[(kvh * G + g) * HD + d] = f2bf(O * __fdiv_rn(1.0f, L));
-    }
-    cluster.sync();                                      // peers may still be reading this CTA's partial
-    sd_stamp(a.tl, 6);
+    cluster_fold<HD, FK_SDPA_CLMAX>(cluster, G, kvh, k_begin, k_end, wpart, cpart, wexp, a.out, nullptr);
 }
 
 // ---------------------------------------------------------------- tensor-core cluster SDPA

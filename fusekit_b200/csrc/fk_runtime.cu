@@ -163,6 +163,9 @@ extern "C" fk_status fk_open(int device, fk_handle *out) {
     CU(cudaFuncSetAttribute(k_sdpa_mma<64>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     CU(cudaFuncSetAttribute(k_sdpa_mma<128>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     CU(cudaFuncSetAttribute(k_sdpa_mma<256>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+#define SQ(B, HD, MG) CU(big_smem(k_sdpa_cluster_q<B, HD, MG>)); CU(cudaFuncSetAttribute(k_sdpa_cluster_q<B, HD, MG>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1))
+    SQ(4, 64, 8); SQ(4, 128, 8); SQ(4, 256, 2); SQ(8, 64, 8); SQ(8, 128, 8); SQ(8, 256, 2);
+#undef SQ
     CU(big_smem(k_qmm4<false>)); CU(big_smem(k_qmm4<true>)); CU(big_smem(k_qmm_tc<32>)); CU(big_smem(k_qmm_tc2));
     CU(big_smem(k_sdpa_decode)); CU(big_smem(k_sdpa_decode_q<4>)); CU(big_smem(k_sdpa_decode_q<8>)); CU(big_smem(k_sdpa_cluster<64, 8>)); CU(big_smem(k_sdpa_cluster<128, 8>)); CU(big_smem(k_sdpa_cluster<256, 2>));
     CU(big_smem(k_rmsnorm_qkv<4>)); CU(big_smem(k_rmsnorm_qkv<8>)); CU(big_smem(k_rmsnorm_qkv<16>));
@@ -919,6 +922,19 @@ static fk_status run_task(Ctx *c, const fk_task &t, const Weight *nextw = nullpt
                     (const uint16_t *)b[8], (const uint16_t *)b[9], (uint16_t *)b[3], (float *)b[4], (uint32_t *)b[5], nq, nkv, hd, cap, chunks, f[0]};
         const size_t smem = sdpa_smem_bytes(G, hd, chunks);
         if (smem > 200 * 1024) return fail(FK_ERR_VALUE, "sdpa_decode_quant: capacity too large for the merge table");
+        // a cluster per kv head, keys split over its CTAs: 16 for caches of 1024 rows and more while all are resident at once, 8 for shorter
+        // ones; more than two heads of 256 dimensions a kv head do not fit its registers (nor more than 8 heads): global partials
+        if (c->sdpa_cluster && G <= 8 && (hd < 256 || G <= 2) && !((b[1] | b[2]) & 15)) {
+            const int cl = cap >= 1024 && nkv * FK_SDPA_CLMAX <= c->sm_count ? FK_SDPA_CLMAX : FK_SDPA_CL;
+            const dim3 cgrid(cl, nkv), cblock(FK_SDPA_CW * 32);
+            const size_t csmem = sdpa_cl_smem_bytes(G, hd);
+#define SQ(B) (hd == 64 ? launch_cluster(c, k_sdpa_cluster_q<B, 64, 8>, cgrid, cblock, csmem, cl, (const FkState *)c->state, a) \
+               : hd == 128 ? launch_cluster(c, k_sdpa_cluster_q<B, 128, 8>, cgrid, cblock, csmem, cl, (const FkState *)c->state, a) \
+                           : launch_cluster(c, k_sdpa_cluster_q<B, 256, 2>, cgrid, cblock, csmem, cl, (const FkState *)c->state, a))
+            e = bits == 4 ? SQ(4) : SQ(8);
+#undef SQ
+            break;
+        }
         if (bits == 4) e = launch(c, k_sdpa_decode_q<4>, dim3(chunks, nkv), dim3(FK_SDPA_THREADS), smem, (const FkState *)c->state, a);
         else e = launch(c, k_sdpa_decode_q<8>, dim3(chunks, nkv), dim3(FK_SDPA_THREADS), smem, (const FkState *)c->state, a);
         break;
