@@ -32,6 +32,16 @@ __device__ __forceinline__ bool tcg_wait(uint32_t bar, uint32_t parity) {
     }
     return false;
 }
+__device__ __forceinline__ bool tcg_try(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    return ok != 0;
+}
+__device__ __forceinline__ bool tcg_elect() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
 __device__ __forceinline__ void tcg_load(uint32_t dst, const CUtensorMap *map, int k, int row, uint32_t bar) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cta.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
                  ::"r"(dst), "l"(map), "r"(k), "r"(row), "r"(bar) : "memory");
@@ -49,7 +59,7 @@ __global__ void __launch_bounds__(FKL_TC_THREADS, 1) k_gemm_tc(FkState *st, cons
     __shared__ uint32_t tmem_slot;
     __shared__ int first[FKL_MAX_EXPERTS + 1];          // grouped: first 128-row tile of every expert
     __shared__ int wsum[8];
-    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, wid = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const uint32_t base = (tcg_smem(smem_raw) + 1023u) & ~1023u;
     const uint32_t full = tcg_smem(bars), empty = full + 8 * S, afull = empty + 8 * S, aempty = afull + 16;
     pdl_launch_dependents();
@@ -116,28 +126,39 @@ __global__ void __launch_bounds__(FKL_TC_THREADS, 1) k_gemm_tc(FkState *st, cons
             if (!ok) atomicOr(&st->error, FKL_ERR_TC_WAIT);
         }
     } else if (wid == 1) {
-        if (lane == 0) {
-            const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((128u >> 4) << 24);
-            int it = 0, j = 0;
-            for (int t = blockIdx.x; t < total && ok; t += gridDim.x, ++j) {
-                const int b = j & 1;
-                if (j >= 2 && !tcg_wait(aempty + 8 * b, (uint32_t)(j / 2 - 1) & 1u)) { ok = false; break; }
-                for (int kb = 0; kb < a.kblocks; ++kb, ++it) {
-                    const int s = it % S;
-                    if (!tcg_wait(full + 8 * s, (uint32_t)(it / S) & 1u)) { ok = false; break; }
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint64_t da = tcg_desc(base + s * T::STAGE), db = tcg_desc(base + s * T::STAGE + T::A_BYTES);
+        // The warp stays together and one elected lane issues: addresses and descriptors live in uniform registers (behind a branch on the
+        // lane every instruction waits for moves into them, 84 cycles an MMA where 33 do), and the next slice's barrier is looked at
+        // while this one's MMAs go out.
+        const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((128u >> 4) << 24);
+        const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
+        const uint64_t da0 = tcg_desc(base), db0 = tcg_desc(base + T::A_BYTES);
+        int s = 0, j = 0;
+        uint32_t ph = 0;
+        bool ready = false;
+        for (int t = blockIdx.x; t < total && ok; t += gridDim.x, ++j) {
+            const int b = j & 1;
+            if (j >= 2 && !tcg_wait(aempty + 8 * b, (uint32_t)(j / 2 - 1) & 1u)) { ok = false; break; }
+            const uint32_t d = tm + (uint32_t)(b * BN);
+            for (int kb = 0; kb < a.kblocks; ++kb) {
+                if (!ready && !tcg_wait(full + 8 * s, ph)) { ok = false; break; }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint64_t off = (uint64_t)(s * (T::STAGE >> 4)), da = da0 + off, db = db0 + off;
+                const uint32_t bar = empty + 8 * s;
+                if (++s == S) { s = 0; ph ^= 1u; }
+                ready = tcg_try(full + 8 * s, ph);
+                if (tcg_elect()) {
 #pragma unroll
                     for (int k = 0; k < FKL_TC_BK / 16; ++k)
                         asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-                                     ::"r"(tmem + (uint32_t)(b * BN)), "l"(da + (uint64_t)(k * 2)), "l"(db + (uint64_t)(k * 2)), "r"(idesc), "r"(kb | k) : "memory");
-                    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(empty + 8 * s) : "memory");
+                                     ::"r"(d), "l"(da + (uint64_t)(k * 2)), "l"(db + (uint64_t)(k * 2)), "r"(idesc), "r"(kb | k) : "memory");
+                    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+                    if (kb + 1 == a.kblocks) asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(afull + 8 * b) : "memory");
                 }
-                if (ok) asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(afull + 8 * b) : "memory");
+                __syncwarp();
             }
-            // the last commits have arrived before tensor memory is freed: the epilogue waits for every accumulator
-            if (!ok) atomicOr(&st->error, FKL_ERR_TC_WAIT);
         }
+        // the last commits have arrived before tensor memory is freed: the epilogue waits for every accumulator
+        if (!ok && lane == 0) atomicOr(&st->error, FKL_ERR_TC_WAIT);
     } else if (wid >= 4) {
         const int q = wid - 4;
         int j = 0;
