@@ -254,10 +254,9 @@ class PrefillEngine(BatchDecodeEngine):
     def _prompt(self, toks, base_offset: int):
         """A prompt of more than one step in portions of up to PORTION positions (whole steps but for the last)."""
         rt, M, n, out = self.rt, self.rows, len(toks), []
-        ids = np.array(toks, np.int64)
-        if ids.min() < 0 or ids.max() >= self.spec.vocab:
-            raise N.FusekitError(f"fk_decode_chunk_rows: token id {int(ids[(ids < 0) | (ids >= self.spec.vocab)][0])} is outside the embedding table ({self.spec.vocab} rows)")
-        ids = ids.astype(np.uint32)
+        ids = np.array(toks, np.uint32)
+        if ids.max() >= self.spec.vocab:
+            raise N.FusekitError(f"token id {int(ids[ids >= self.spec.vocab][0])} is outside the embedding table ({self.spec.vocab} rows)")
         most = min(self.PORTION, self.capacity) // M * M
         for c0 in range(0, n, most):
             part = ids[c0:c0 + most]
@@ -275,7 +274,10 @@ class PrefillEngine(BatchDecodeEngine):
             err = rt.state_get()[2]
             if err:
                 raise N.FusekitError(f"device error word {err:#x}")
-        return np.concatenate(out)
+        out = np.concatenate(out)
+        first = (n - 1) // M * M                    # the decode state as the last step leaves it
+        rt.state_set(int(out[first]), base_offset + first + M)
+        return out
 
     def prefill(self, tokens, base_offset: int = 0):
         """Run `tokens` through the model from position `base_offset` on; returns the greedy prediction after every position,
@@ -284,7 +286,7 @@ class PrefillEngine(BatchDecodeEngine):
         read the weights once per portion instead of once per step, or (see `_staged`) step by step."""
         toks = [int(t) for t in tokens]
         M, preds = self.rows, []
-        if len(toks) > M and self._staged:
+        if len(toks) > M and base_offset >= 0 and self._staged:
             if base_offset + (len(toks) + M - 1) // M * M > self.capacity:
                 raise ValueError("prefill chunk reaches beyond the cache capacity")
             if not self.graph:

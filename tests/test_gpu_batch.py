@@ -92,3 +92,24 @@ def test_chunked_prefill_matches_the_oracle_stepping_the_prompt(rows, qmm):
         assert not mism and len(ties) <= 2, (mism, ties)
     finally:
         dec.close()
+
+
+@pytest.mark.parametrize("vocab", [5, 8, 1000, 1003, 151936])
+def test_greedy_tokens_of_rows(runtime, vocab):
+    """Eight logits per load, and the scalar tail of a vocabulary that is no multiple of eight: the lowest index of the largest logit."""
+    from fusekit_b200 import _native as N
+    rt, rows = runtime, 6
+    x = O.f32_to_bf16(np.random.default_rng(vocab).normal(size=(rows, vocab)).astype(np.float32))
+    x[0, vocab - 1] = x[1, 0] = 0x4300                      # 128, at either end
+    x[2, vocab // 2:] = 0x4300                              # ties: the first of them
+    x[3, :] = 0xff7f                                        # the lowest finite number everywhere
+    f = O.bf16_to_f32(x)
+    logits, counter, preds = rt.to_device(x), rt.to_device(np.zeros(1, np.uint32)), rt.alloc(rows * 4)
+    rt.state_set(0, 7)
+    rt.launch(N.Task.make(N.TASK_ARGMAX_ROWS, -1, {0: logits, 5: counter}, [vocab, rows, 1]))
+    assert rt.state_get()[:2] == (int(f[0].argmax()), 8)
+    if vocab % 8 == 0:
+        rt.launch(N.Task.make(N.TASK_ARGMAX_PROMPT, -1, {0: logits, 1: preds}, [vocab, rows]))
+        assert list(rt.download(preds, (rows,), np.uint32)) == list(f.argmax(1))
+    for p in (logits, counter, preds):
+        N.check(rt.L.fk_free(rt.h, p), "fk_free")

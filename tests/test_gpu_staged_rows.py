@@ -145,8 +145,10 @@ def test_whole_prompts_match_the_steps(rows, count):
             eng.load_synthetic()
             eng.prefill(prompt[:base])
             preds = eng.prefill(prompt[base:], base)
+            state = eng.rt.state_get()[:2]
             caches = np.stack([[eng.rt.download(p, (spec.n_kv, cap, hd), np.uint16)[:, :count + base] for p in kv] for kv in eng.cache])
             logits = eng.rt.download(eng.logits, (rows, spec.vocab), np.uint16)[:(count - 1) % rows + 1]
+            assert state == (int(preds[(count - 1) // rows * rows]), base + -(-count // rows) * rows)
             got[name] = preds, O.bf16_to_f32(caches).astype(np.float64), O.bf16_to_f32(logits).astype(np.float64)
             if name == "whole":
                 with pytest.raises(ValueError):
