@@ -186,7 +186,7 @@ extern "C" fk_status fk_close(fk_handle h) {
     CTX(h);
     cudaStreamSynchronize(c->stream);
     for (auto &g : c->graphs) { if (g.exec) cudaGraphExecDestroy(g.exec); if (g.graph) cudaGraphDestroy(g.graph); }
-    for (auto &w : c->weights) { cudaFree(w.w); cudaFree(w.s); cudaFree(w.b); cudaFree(w.units); cudaFree(w.rowmul); }
+    for (auto &w : c->weights) { cudaFree(w.w); cudaFree(w.s); cudaFree(w.b); cudaFree(w.units); }
     for (void *p : c->allocs) cudaFree(p);
     if (c->comm && g_nccl.CommDestroy) g_nccl.CommDestroy(c->comm);
     for (void *p : c->ipc_open) cudaIpcCloseMemHandle(p);
@@ -315,7 +315,8 @@ static fk_status repack(Ctx *c, Weight *dstw, const Weight *a, const Weight *b2)
     const int kpu = unit_k(a->bits);                             // activations per unit
     dstw->ntiles = (int)((dstw->n + 15) / 16); dstw->nsb = (int)((a->k + kpu - 1) / kpu);
     dstw->unit_bytes = (size_t)dstw->ntiles * dstw->nsb * unit_vec(a->bits) * 16;
-    CU(cudaMalloc(&dstw->units, dstw->unit_bytes));
+    // 4 bits: the rows' powers of two lie behind the units, in the same allocation
+    CU(cudaMalloc(&dstw->units, dstw->unit_bytes + (a->bits == 4 ? (size_t)dstw->ntiles * 16 * sizeof(float) : 0)));
     if (a->bits == 16) {
         const long long tot16 = (long long)dstw->ntiles * dstw->nsb * 256;
         k_repack_tiled16<<<(unsigned)((tot16 + 255) / 256), 256, 0, c->stream>>>((const uint16_t *)a->w, (const uint16_t *)(b2 ? b2->w : a->w), dstw->units, a->n,
@@ -331,7 +332,7 @@ static fk_status repack(Ctx *c, Weight *dstw, const Weight *a, const Weight *b2)
                                                                         dstw->rows_kind, dstw->hd, dstw->n_rot);
     CU(cudaGetLastError());
     if (a->bits == 4) {
-        CU(cudaMalloc(&dstw->rowmul, (size_t)dstw->ntiles * 16 * sizeof(float)));
+        dstw->rowmul = reinterpret_cast<float *>(reinterpret_cast<unsigned char *>(dstw->units) + dstw->unit_bytes);
         k_row_factors<<<(dstw->ntiles + 7) / 8, 256, 0, c->stream>>>(dstw->units, dstw->rowmul, dstw->ntiles, dstw->nsb);
         CU(cudaGetLastError());
     }
