@@ -829,6 +829,8 @@ __global__ void __launch_bounds__(FK_SDPA_CW * 32) k_sdpa_cluster(const FkState 
 // soon as the registers of the current ones are read (keys before the softmax, values after the sums).  Bound by the latency of the
 // few rounds a warp makes and by the multiply-adds (2 G per element on the CUDA cores, in fp32).  Everything goes through L2: a
 // line of scales holds many keys, the newest among them, so none of it may be kept from before the dependency wait in L1.
+// A layer of the 7B shape at context 4000 with an 8-bit cache takes 49 us less than with the global partials of k_sdpa_decode_q, whose last
+// block walks 125 of them per output.
 template <int BITS, int HD, int MAXG>
 __global__ void __launch_bounds__(FK_SDPA_CW * 32) k_sdpa_cluster_q(const FkState *st, SdpaQArgs a) {
     extern __shared__ float sm[];
