@@ -5,71 +5,41 @@
 // TMA (128-byte swizzle) into a ring of shared-memory stages, one thread of warp 1 issues tcgen05.mma (cta_group::1, M = 128,
 // N = BN, K = 16) into one of two accumulators in tensor memory, warps 4 .. 7 read finished accumulators back and store them
 // while the next tile is being multiplied.  Rows past the end of a tile's range are multiplied and not stored (past the end of
-// the tensor TMA delivers zeros).  Every wait is bounded: when one runs out the kernel sets an error bit, waits (bounded) for
-// its copies in flight, frees its tensor memory and returns.
+// the tensor TMA delivers zeros).  Every wait is bounded (fk_tc.cuh).
 #pragma once
 #include "fk_layers.cuh"
-#include <cuda.h>
+#include "fk_tc.cuh"
 
 #define FKL_TC_BK 64
 #define FKL_TC_THREADS 256
-#define FKL_TC_SPIN (1u << 21)
 template <int BN> struct TcTile {
     static constexpr int STAGES = BN == 256 ? 4 : BN == 128 ? 6 : 8;
     static constexpr int A_BYTES = 128 * FKL_TC_BK * 2, B_BYTES = BN * FKL_TC_BK * 2, STAGE = A_BYTES + B_BYTES, COLS = 2 * BN;
     static constexpr size_t SMEM = (size_t)STAGES * STAGE + 1024;
 };
-struct TcGemmArgs { void *y; const int *offsets; int m, n, kblocks, row0, ldy, act, out_f32, experts; float scale; BlockCols b; };       // b: BLOCK form
+struct TcGemmArgs { void *y; const int *offsets; int m, n, kblocks, row0, ldy, act, out_f32, experts; float scale; BlockCols b; uint32_t limit; };       // b: BLOCK form
 
-__device__ __forceinline__ uint32_t tcg_smem(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void tcg_init(uint32_t bar, uint32_t count) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory"); }
-__device__ __forceinline__ void tcg_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
-__device__ __forceinline__ bool tcg_wait(uint32_t bar, uint32_t parity) {
-    for (uint32_t i = 0; i < FKL_TC_SPIN; ++i) {
-        uint32_t ok;
-        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-        if (ok) return true;
-    }
-    return false;
-}
-__device__ __forceinline__ bool tcg_try(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-    return ok != 0;
-}
-__device__ __forceinline__ bool tcg_elect() {
-    uint32_t p;
-    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
-    return p != 0;
-}
-__device__ __forceinline__ void tcg_load(uint32_t dst, const CUtensorMap *map, int k, int row, uint32_t bar) {
-    asm volatile("cp.async.bulk.tensor.2d.shared::cta.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-                 ::"r"(dst), "l"(map), "r"(k), "r"(row), "r"(bar) : "memory");
-}
-// K-major operand with 128-byte swizzle: rows of 128 bytes, groups of 8 rows 1024 bytes apart
-__device__ __forceinline__ uint64_t tcg_desc(uint32_t addr) {
-    return (uint64_t)((addr >> 4) & 0x3FFFu) | (1ull << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
-}
 template <int BN, bool BLOCK>
 __global__ void __launch_bounds__(FKL_TC_THREADS, 1) k_gemm_tc(FkState *st, const __grid_constant__ CUtensorMap mx, const __grid_constant__ CUtensorMap mw, TcGemmArgs a) {
     using T = TcTile<BN>;
     constexpr int S = T::STAGES;
     extern __shared__ unsigned char smem_raw[];
-    __shared__ __align__(8) uint64_t bars[2 * S + 4];
+    __shared__ __align__(8) uint64_t bars[2 * S + 5];
     __shared__ uint32_t tmem_slot;
     __shared__ int first[FKL_MAX_EXPERTS + 1];          // grouped: first 128-row tile of every expert
     __shared__ int wsum[8];
     const int tid = threadIdx.x, lane = tid & 31, wid = __shfl_sync(0xffffffffu, tid >> 5, 0);
-    const uint32_t base = (tcg_smem(smem_raw) + 1023u) & ~1023u;
-    const uint32_t full = tcg_smem(bars), empty = full + 8 * S, afull = empty + 8 * S, aempty = afull + 16;
+    const uint32_t base = (tc_smem(smem_raw) + 1023u) & ~1023u;
+    const uint32_t full = tc_smem(bars), empty = full + 8 * S, afull = empty + 8 * S, aempty = afull + 16, drained = aempty + 16;
     pdl_launch_dependents();
     if (tid == 0) {
-        for (int s = 0; s < S; ++s) { tcg_init(full + 8 * s, 1); tcg_init(empty + 8 * s, 1); }
-        for (int s = 0; s < 2; ++s) { tcg_init(afull + 8 * s, 1); tcg_init(aempty + 8 * s, 4); }
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        for (int s = 0; s < S; ++s) { tc_init(full + 8 * s, 1); tc_init(empty + 8 * s, 1); }
+        for (int s = 0; s < 2; ++s) { tc_init(afull + 8 * s, 1); tc_init(aempty + 8 * s, 4); }
+        tc_init(drained, 1);
+        tc_init_fence();
     }
     if (wid == 2) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tcg_smem(&tmem_slot)), "r"((uint32_t)T::COLS) : "memory");
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc_smem(&tmem_slot)), "r"((uint32_t)T::COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     pdl_wait();
@@ -115,14 +85,17 @@ __global__ void __launch_bounds__(FKL_TC_THREADS, 1) k_gemm_tc(FkState *st, cons
                 int m0, mend, wrow, n0; place(t, m0, mend, wrow, n0);
                 for (int kb = 0; kb < a.kblocks; ++kb, ++it) {
                     const int s = it % S;
-                    if (it >= S && !tcg_wait(empty + 8 * s, (uint32_t)(it / S - 1) & 1u)) { ok = false; break; }
-                    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(full + 8 * s), "r"((uint32_t)T::STAGE) : "memory");
-                    tcg_load(base + s * T::STAGE, &mx, kb * FKL_TC_BK, m0, full + 8 * s);
-                    tcg_load(base + s * T::STAGE + T::A_BYTES, &mw, kb * FKL_TC_BK, wrow, full + 8 * s);
+                    if (it >= S && !tc_wait(empty + 8 * s, (uint32_t)(it / S - 1) & 1u, a.limit)) { ok = false; break; }
+                    tc_expect(full + 8 * s, (uint32_t)T::STAGE);
+                    tc_load(base + s * T::STAGE, &mx, kb * FKL_TC_BK, m0, full + 8 * s);
+                    tc_load(base + s * T::STAGE + T::A_BYTES, &mw, kb * FKL_TC_BK, wrow, full + 8 * s);
                 }
             }
-            // the last stages are multiplied (or at least have landed) before the block may leave
-            for (int j = it > S ? it - S : 0; j < it; ++j) if (!tcg_wait((ok ? empty : full) + 8 * (j % S), (uint32_t)(j / S) & 1u)) ok = false;
+            // the last stages have landed and, unless a wait ran out, are multiplied before the block may leave
+            for (int j = it > S ? it - S : 0; j < it; ++j) {
+                if (!tc_wait(full + 8 * (j % S), (uint32_t)(j / S) & 1u, TC_DRAIN)) ok = false;
+                if (ok && !tc_wait(empty + 8 * (j % S), (uint32_t)(j / S) & 1u, a.limit)) ok = false;
+            }
             if (!ok) atomicOr(&st->error, FKL_ERR_TC_WAIT);
         }
     } else if (wid == 1) {
@@ -131,33 +104,33 @@ __global__ void __launch_bounds__(FKL_TC_THREADS, 1) k_gemm_tc(FkState *st, cons
         // while this one's MMAs go out.
         const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((128u >> 4) << 24);
         const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
-        const uint64_t da0 = tcg_desc(base), db0 = tcg_desc(base + T::A_BYTES);
+        const uint64_t da0 = tc_desc(base), db0 = tc_desc(base + T::A_BYTES);
         int s = 0, j = 0;
         uint32_t ph = 0;
         bool ready = false;
         for (int t = blockIdx.x; t < total && ok; t += gridDim.x, ++j) {
             const int b = j & 1;
-            if (j >= 2 && !tcg_wait(aempty + 8 * b, (uint32_t)(j / 2 - 1) & 1u)) { ok = false; break; }
+            if (j >= 2 && !tc_wait_warp(aempty + 8 * b, (uint32_t)(j / 2 - 1) & 1u, a.limit)) { ok = false; break; }
             const uint32_t d = tm + (uint32_t)(b * BN);
             for (int kb = 0; kb < a.kblocks; ++kb) {
-                if (!ready && !tcg_wait(full + 8 * s, ph)) { ok = false; break; }
+                if (!ready && !tc_wait_warp(full + 8 * s, ph, a.limit)) { ok = false; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint64_t off = (uint64_t)(s * (T::STAGE >> 4)), da = da0 + off, db = db0 + off;
                 const uint32_t bar = empty + 8 * s;
                 if (++s == S) { s = 0; ph ^= 1u; }
-                ready = tcg_try(full + 8 * s, ph);
-                if (tcg_elect()) {
+                ready = tc_try_warp(full + 8 * s, ph);
+                if (tc_elect()) {
 #pragma unroll
                     for (int k = 0; k < FKL_TC_BK / 16; ++k)
                         asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
                                      ::"r"(d), "l"(da + (uint64_t)(k * 2)), "l"(db + (uint64_t)(k * 2)), "r"(idesc), "r"(kb | k) : "memory");
-                    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-                    if (kb + 1 == a.kblocks) asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(afull + 8 * b) : "memory");
+                    tc_commit(bar);
+                    if (kb + 1 == a.kblocks) tc_commit(afull + 8 * b);
                 }
                 __syncwarp();
             }
         }
-        // the last commits have arrived before tensor memory is freed: the epilogue waits for every accumulator
+        if (!tc_drain_mmas(drained)) ok = false;        // before tensor memory is freed, also where the storing warps gave up
         if (!ok && lane == 0) atomicOr(&st->error, FKL_ERR_TC_WAIT);
     } else if (wid >= 4) {
         const int q = wid - 4;
@@ -165,7 +138,7 @@ __global__ void __launch_bounds__(FKL_TC_THREADS, 1) k_gemm_tc(FkState *st, cons
         for (int t = blockIdx.x; t < total && ok; t += gridDim.x, ++j) {
             int m0, mend, wrow, n0; place(t, m0, mend, wrow, n0);
             const int b = j & 1, row = m0 + q * 32 + lane;
-            if (!tcg_wait(afull + 8 * b, (uint32_t)(j / 2) & 1u)) { ok = false; break; }
+            if (!tc_wait_warp(afull + 8 * b, (uint32_t)(j / 2) & 1u, a.limit)) { ok = false; break; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll 1
             for (int c = 0; c < BN; c += 32) {
@@ -234,7 +207,7 @@ __global__ void __launch_bounds__(FKL_TC_THREADS, 1) k_gemm_tc(FkState *st, cons
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
-            if (lane == 0) tcg_arrive(aempty + 8 * b);
+            if (lane == 0) tc_arrive(aempty + 8 * b);
         }
         if (!ok && lane == 0) atomicOr(&st->error, FKL_ERR_TC_WAIT);
     }

@@ -155,7 +155,7 @@ fk_status fkl_run(FklEnv &c, const fk_task &t, char *err, size_t ecap) {
         const float scale = block || f[0] == 0.0f ? 1.0f : f[0];
         if (!f32) {           // tensor cores
             if (ldx % 64 || (b[0] & 15) || (block && ((b[2] & 15) || ldy % 8))) return bad(err, ecap, "linear_rows: bf16 rows need a stride in multiples of 64 and 16-byte alignment");
-            TcGemmArgs a{(void *)b[2], groups, M, N, (int)(w.k / FKL_TC_BK), row0, ldy, act, outf, E, scale, cols};
+            TcGemmArgs a{(void *)b[2], groups, M, N, (int)(w.k / FKL_TC_BK), row0, ldy, act, outf, E, scale, cols, c.wait_limit};
             const long long mt = groups ? (M < E ? M : E) + M / 128 : (M + 127) / 128;
             const int bn = tc_tile(c.sm_count, mt, N);
             const long long tiles = mt * ((N + bn - 1) / bn);

@@ -12,6 +12,7 @@ struct FklEnv {
     cudaStream_t stream; bool pdl; int sm_count;
     FkState *state; uint32_t *history; long long *launches;
     void *owner; bool (*weight)(void *owner, uint64_t id, FklWeight *out);      // false: no such weight, or not frozen as rows
+    uint32_t wait_limit;                                           // polls before a wait of the tcgen05 kernels gives up
 };
 bool fkl_owns(int kind);                                           // whether a task kind is handled here
 fk_status fkl_run(FklEnv &env, const fk_task &t, char *err, size_t cap);

@@ -17,8 +17,7 @@
 // and write it straight into tensor memory as the A operand (tcgen05.st .16x256b: the lane layout of the units is its lane layout; a ring
 // of four to seven k-blocks); through shared memory the expanded operand costs two more crossings of it than the packed weights.  One warp
 // fetches X by TMA (128-byte swizzle), one warp per accumulator issues its MMAs, 8 warps store finished tiles.  Weight rings are filled before
-// griddepcontrol.wait.  Every wait is bounded; when one runs out the kernel sets an error bit, waits (bounded) for its copies, frees
-// its tensor memory and returns.
+// griddepcontrol.wait.  Every wait is bounded (fk_tc.cuh).
 //
 // Bound by the issue of the dequantising warps (538 instructions a k-block and scheduler, 72 % of its slots): 1000 rows, 3584 -> 2 x 18944, 292 us =
 // 931 TFLOP/s; 16 rows, 5120 -> 2 x 27648, 65 us = 2.45 TB/s of weights (k_qmm4 98 us; 20 -> 22 us at 5120 -> 5120, where start-up counts).
@@ -28,6 +27,7 @@
 #pragma once
 #include "fk_stream.cuh"
 #include "fk_layers.h"
+#include "fk_tc.cuh"
 #include <cuda_fp16.h>
 
 #define FKQ_SB 576                      // staged halves per super-block: 512 activations, 32 slots for the sums, 32 unused
@@ -35,7 +35,6 @@
 #define FKQ_EPI 8                       // storing warps
 #define FKQ_THREADS ((FKQ_DEQ + FKQ_EPI + 3) * 32)      // .. a warp for X, two for the MMAs
 #define FKQ_ROWS 256                    // weight rows of a block
-#define FKQ_SPIN (1u << 21)
 #define FKQ_MAX_K 32768                 // a row is staged from registers: 1024 threads x 4 vectors of 8
 #define FKQ_ERR_WAIT 0x400000u
 #define FKQ_COUNTERS 65536              // ticket words: 8 per tile that is split
@@ -46,29 +45,8 @@ template <int BN> struct QgTile {
 };
 __host__ __device__ inline size_t fkq_part_floats(int bn) { return (size_t)bn * FKQ_ROWS; }
 
-struct QGemmArgs { TiledW W; const float *xscale; const uint16_t *residual; uint16_t *y; float *scratch; unsigned int *counters; const float *rowmul; int m, n, ldr, act, whole, mtiles, tiles; };
+struct QGemmArgs { TiledW W; const float *xscale; const uint16_t *residual; uint16_t *y; float *scratch; unsigned int *counters; const float *rowmul; int m, n, ldr, act, whole, mtiles, tiles; uint32_t limit; };
 
-__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-    return ok != 0;
-}
-__device__ __forceinline__ bool qg_wait(uint32_t bar, uint32_t parity) {
-    for (uint32_t i = 0; i < FKQ_SPIN; ++i) {
-        uint32_t ok;
-        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-        if (ok) return true;
-    }
-    return false;
-}
-__device__ __forceinline__ void qg_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
-__device__ __forceinline__ void qg_expect(uint32_t bar, uint32_t bytes) { asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory"); }
-__device__ __forceinline__ void qg_commit(uint32_t bar) { asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory"); }
-__device__ __forceinline__ bool qg_elect() {
-    uint32_t p;
-    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
-    return p != 0;
-}
 // D += A B^T: A (128 rows, 16 halves) in tensor memory, B (the descriptor's rows) in shared memory; more = 0 overwrites D
 __device__ __forceinline__ void qg_mma(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t more) {
     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(more) : "memory");
@@ -136,12 +114,12 @@ __global__ void __launch_bounds__(FKQ_THREADS, 1) k_qgemm(FkState *st, const __g
     using T = QgTile<BN>;
     constexpr int XS = T::XS, XG = T::XG, NBUF = T::NBUF, AS = T::AS;
     extern __shared__ unsigned char qg_smem[];
-    __shared__ __align__(8) uint64_t bars[FKQ_DEQ * FK_STAGES + 2 * XS + 2 * AS + 2 * NBUF];
+    __shared__ __align__(8) uint64_t bars[FKQ_DEQ * FK_STAGES + 2 * XS + 2 * AS + 2 * NBUF + 2];
     __shared__ uint32_t tmem_slot;
     const int tid = threadIdx.x, lane = tid & 31, wid = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const uint32_t base = (smem_u32(qg_smem) + 1023u) & ~1023u, ring = base + XS * XG * T::XBYTES;
     const uint32_t wfull = smem_u32(bars), xfull = wfull + 8 * FKQ_DEQ * FK_STAGES, xempty = xfull + 8 * XS, afull = xempty + 8 * XS, aempty = afull + 8 * AS,
-                   dfull = aempty + 8 * AS, dempty = dfull + 8 * NBUF;
+                   dfull = aempty + 8 * AS, dempty = dfull + 8 * NBUF, drained = dempty + 8 * NBUF;
     pdl_launch_dependents();
     if (tid == 0) {
         for (int i = 0; i < FKQ_DEQ * FK_STAGES; ++i) mbar_init(bars + i, 1);
@@ -151,6 +129,7 @@ __global__ void __launch_bounds__(FKQ_THREADS, 1) k_qgemm(FkState *st, const __g
         for (int i = 0; i < AS; ++i) { mbar_init(b + i, FKQ_DEQ); mbar_init(b + AS + i, 2); }
         b += 2 * AS;
         for (int i = 0; i < NBUF; ++i) { mbar_init(b + i, 2); mbar_init(b + NBUF + i, FKQ_EPI); }
+        mbar_init(b + 2 * NBUF, 1); mbar_init(b + 2 * NBUF + 1, 1);
         mbar_fence_init();
     }
     if (wid == FKQ_DEQ) {
@@ -179,7 +158,7 @@ __global__ void __launch_bounds__(FKQ_THREADS, 1) k_qgemm(FkState *st, const __g
             if (!more) return;
             if (lane == 0) {
                 const int s = issued & (FK_STAGES - 1);
-                qg_expect(bar0 + 8 * s, FK_UNIT_BYTES);
+                tc_expect(bar0 + 8 * s, FK_UNIT_BYTES);
                 asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                              ::"r"(ring0 + (uint32_t)(s * FK_UNIT_BYTES)), "l"(a.W.units + ((size_t)((iw.tile / a.mtiles) * 16 + mine) * nsb + ikb) * FK_UNIT_VEC),
                                "r"((uint32_t)FK_UNIT_BYTES), "r"(bar0 + 8 * s) : "memory");
@@ -194,11 +173,11 @@ __global__ void __launch_bounds__(FKQ_THREADS, 1) k_qgemm(FkState *st, const __g
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
-            if (lane == 0 && pend) qg_arrive(pend);
+            if (lane == 0 && pend) tc_arrive(pend);
         };
         auto claim = [&](bool free) {                   // the slot `as` may be written; a wait that runs out gives the kernel up
             announce();
-            if (!free && !qg_wait(aempty + 8 * as, aph)) ok = false;
+            if (!free && !tc_wait_warp(aempty + 8 * as, aph, a.limit)) ok = false;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         };
         auto taken = [&]() { pend = afull + 8 * as; if (++as == AS) { as = 0; aph ^= 1u; } };
@@ -208,7 +187,7 @@ __global__ void __launch_bounds__(FKQ_THREADS, 1) k_qgemm(FkState *st, const __g
             const float mul = have ? __ldg(a.rowmul + tile * 16 + (lane >> 2)) : 1.0f, mul8 = have ? __ldg(a.rowmul + tile * 16 + 8 + (lane >> 2)) : 1.0f;
             for (int kb = w.k0; kb < w.k1 && ok; ++kb) {
                 const int s = used & (FK_STAGES - 1);
-                if (have && !qg_wait(bar0 + 8 * s, (uint32_t)(used / FK_STAGES) & 1u)) { ok = false; break; }
+                if (have && !tc_wait_warp(bar0 + 8 * s, (uint32_t)(used / FK_STAGES) & 1u, a.limit)) { ok = false; break; }
                 const uint32_t u = ring0 + (uint32_t)(s * FK_UNIT_BYTES + lane * 16);
                 // scales and biases of rows g and g + 8, groups 2t and 2t + 1: s and c for the shuffles below, e for the sums' slots
                 // (a warp without a unit works on what the ring holds: rows that nobody stores)
@@ -229,7 +208,7 @@ __global__ void __launch_bounds__(FKQ_THREADS, 1) k_qgemm(FkState *st, const __g
 #pragma unroll
                     for (int h = 0; h < 2; ++h) {
                         const uint4 nx = lds128(u + (uint32_t)((2 * j + h + 1) * 512));      // after the last group: the scales, not used
-                        const bool free = mbar_try(aempty + 8 * as, aph);
+                        const bool free = tc_try_warp(aempty + 8 * as, aph);
                         const uint32_t sg = __shfl_sync(0xffffffffu, sc[h], src), cg = __shfl_sync(0xffffffffu, cc[h], src);
                         const uint32_t sg8 = __shfl_sync(0xffffffffu, sc[2 + h], src), cg8 = __shfl_sync(0xffffffffu, cc[2 + h], src);
                         // nibbles 4 bits up: (1024 + 16 q) s / 16 + c + 960 s
@@ -251,7 +230,7 @@ __global__ void __launch_bounds__(FKQ_THREADS, 1) k_qgemm(FkState *st, const __g
                 if (!ok) break;
                 stages += 9;
                 {                                       // the sums' slots: columns 8b + 2t (e_hi, e_hi) and 8b + 2t + 1 (e_lo, 0) of group 2t + b
-                    const bool free = mbar_try(aempty + 8 * as, aph);
+                    const bool free = tc_try_warp(aempty + 8 * as, aph);
                     uint32_t r[8];
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {       // e[i] is row g + 8 (i / 2), group 2t + (i & 1)
@@ -268,8 +247,8 @@ __global__ void __launch_bounds__(FKQ_THREADS, 1) k_qgemm(FkState *st, const __g
             announce(); pend = 0;                       // the tile's last
         }
         // what is still in flight lands, and the MMAs that read the last stages have been counted, before the block may leave
-        for (; used < issued; ++used) if (!qg_wait(bar0 + 8 * (used & (FK_STAGES - 1)), (uint32_t)(used / FK_STAGES) & 1u)) ok = false;
-        if (ok) for (int j = stages > AS ? stages - AS : 0; j < stages; ++j) if (!qg_wait(aempty + 8 * (j % AS), (uint32_t)(j / AS) & 1u)) ok = false;
+        for (; used < issued; ++used) if (!tc_wait_warp(bar0 + 8 * (used & (FK_STAGES - 1)), (uint32_t)(used / FK_STAGES) & 1u, TC_DRAIN)) ok = false;
+        if (ok) for (int j = stages > AS ? stages - AS : 0; j < stages; ++j) if (!tc_wait_warp(aempty + 8 * (j % AS), (uint32_t)(j / AS) & 1u, a.limit)) ok = false;
         if (!ok && lane == 0) atomicOr(&st->error, FKQ_ERR_WAIT);
     } else if (wid == FKQ_DEQ + FKQ_EPI) {
         // ---------------------------------------------------------------- X
@@ -280,15 +259,17 @@ __global__ void __launch_bounds__(FKQ_THREADS, 1) k_qgemm(FkState *st, const __g
                 const int m0 = (w.tile % a.mtiles) * BN;
                 for (int kb = w.k0 * 9; kb < w.k1 * 9; kb += XG, ++it) {
                     const int s = it % XS;
-                    if (it >= XS && !qg_wait(xempty + 8 * s, (uint32_t)(it / XS - 1) & 1u)) { ok = false; break; }
-                    qg_expect(xfull + 8 * s, (uint32_t)(XG * T::XBYTES));
+                    if (it >= XS && !tc_wait(xempty + 8 * s, (uint32_t)(it / XS - 1) & 1u, a.limit)) { ok = false; break; }
+                    tc_expect(xfull + 8 * s, (uint32_t)(XG * T::XBYTES));
 #pragma unroll
                     for (int g = 0; g < XG; ++g)
-                        asm volatile("cp.async.bulk.tensor.2d.shared::cta.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-                                     ::"r"(base + (s * XG + g) * T::XBYTES), "l"(&mx), "r"((kb + g) * 64), "r"(m0), "r"(xfull + 8 * s) : "memory");
+                        tc_load(base + (s * XG + g) * T::XBYTES, &mx, (kb + g) * 64, m0, xfull + 8 * s);
                 }
             }
-            for (int j = it > XS ? it - XS : 0; j < it; ++j) if (!qg_wait((ok ? xempty : xfull) + 8 * (j % XS), (uint32_t)(j / XS) & 1u)) ok = false;
+            for (int j = it > XS ? it - XS : 0; j < it; ++j) {      // landed and, unless a wait ran out, multiplied
+                if (!tc_wait(xfull + 8 * (j % XS), (uint32_t)(j / XS) & 1u, TC_DRAIN)) ok = false;
+                if (ok && !tc_wait(xempty + 8 * (j % XS), (uint32_t)(j / XS) & 1u, a.limit)) ok = false;
+            }
             if (!ok) atomicOr(&st->error, FKQ_ERR_WAIT);
         }
     } else if (wid > FKQ_DEQ + FKQ_EPI) {
@@ -300,39 +281,40 @@ __global__ void __launch_bounds__(FKQ_THREADS, 1) k_qgemm(FkState *st, const __g
         const int sub = wid - (FKQ_DEQ + FKQ_EPI + 1);
         const uint32_t idesc = (1u << 4) | ((uint32_t)(BN >> 3) << 17) | ((128u >> 4) << 24);          // fp16 x fp16 -> fp32
         const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0), tma = tm + (uint32_t)(T::DCOLS + sub * 32);
-        const uint64_t db0 = (uint64_t)((base >> 4) & 0x3FFFu) | (1ull << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
+        const uint64_t db0 = tc_desc(base);
         int s = 0, as = 0;
         uint32_t xph = 0, aph = 0;
         bool xready = false, aready = false;
         for (int v = 0; ok && fkq_work(a.whole, a.tiles, nsb, me, G, v, w); ++v) {
             const int d = v % NBUF;
-            if (v >= NBUF && !qg_wait(dempty + 8 * d, (uint32_t)(v / NBUF - 1) & 1u)) { ok = false; break; }
+            if (v >= NBUF && !tc_wait_warp(dempty + 8 * d, (uint32_t)(v / NBUF - 1) & 1u, a.limit)) { ok = false; break; }
             const uint32_t dd = tm + (uint32_t)((d * 2 + sub) * BN);
             uint32_t again = 0;                         // 0: the tile's first MMA overwrites
             for (int sb = w.k0; sb < w.k1 && ok; ++sb)
 #pragma unroll 1
                 for (int kk = 0, g = 0; kk < 9; ++kk) {
-                    if ((g == 0 && !xready && !qg_wait(xfull + 8 * s, xph)) || (!aready && !qg_wait(afull + 8 * as, aph))) { ok = false; break; }
+                    if ((g == 0 && !xready && !tc_wait_warp(xfull + 8 * s, xph, a.limit)) || (!aready && !tc_wait_warp(afull + 8 * as, aph, a.limit))) { ok = false; break; }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint64_t db = db0 + (uint64_t)((s * XG + g) * (T::XBYTES >> 4));
                     const uint32_t aa = tma + (uint32_t)(as * 64), xs_bar = xempty + 8 * s, as_bar = aempty + 8 * as;
                     const bool last = ++g == XG;
-                    if (last) { g = 0; if (++s == XS) { s = 0; xph ^= 1u; } xready = mbar_try(xfull + 8 * s, xph); }
+                    if (last) { g = 0; if (++s == XS) { s = 0; xph ^= 1u; } xready = tc_try_warp(xfull + 8 * s, xph); }
                     if (++as == AS) { as = 0; aph ^= 1u; }
-                    aready = mbar_try(afull + 8 * as, aph);
-                    if (qg_elect()) {
+                    aready = tc_try_warp(afull + 8 * as, aph);
+                    if (tc_elect()) {
                         qg_mma(dd, aa, db, idesc, again);
                         qg_mma(dd, aa + 8, db + 2, idesc, 1u);
                         if (kk < 8) { qg_mma(dd, aa + 16, db + 4, idesc, 1u); qg_mma(dd, aa + 24, db + 6, idesc, 1u); }
-                        qg_commit(as_bar);
-                        if (last) qg_commit(xs_bar);
+                        tc_commit(as_bar);
+                        if (last) tc_commit(xs_bar);
                     }
                     __syncwarp();
                     again = 1;
                 }
-            if (ok && qg_elect()) qg_commit(dfull + 8 * d);
+            if (ok && tc_elect()) tc_commit(dfull + 8 * d);
             __syncwarp();
         }
+        if (!tc_drain_mmas(drained + 8 * sub)) ok = false;      // before tensor memory is freed, also where the storing warps gave up
         if (!ok && lane == 0) atomicOr(&st->error, FKQ_ERR_WAIT);
     } else {
         // ---------------------------------------------------------------- finished tiles: lane = weight row, registers = rows of X
@@ -363,7 +345,7 @@ __global__ void __launch_bounds__(FKQ_THREADS, 1) k_qgemm(FkState *st, const __g
             };
             const float rmul = row0 + lane < a.W.ntiles * 16 ? __uint_as_float(0x7F000000u - __float_as_uint(__ldg(a.rowmul + row0 + lane))) : 0.0f;       // 2^-k of 2^k
             if (!GATEUP && !part) fetch(0, res);        // under the tile's MMAs
-            if (!qg_wait(dfull + 8 * d, (uint32_t)(v / NBUF) & 1u)) { ok = false; break; }
+            if (!tc_wait_warp(dfull + 8 * d, (uint32_t)(v / NBUF) & 1u, a.limit)) { ok = false; break; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t src = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)((d * 2 + sub) * BN);
             // rows c .. of X, whose factors lanes f0 .. hold; r: their residual pairs
@@ -466,7 +448,7 @@ __global__ void __launch_bounds__(FKQ_THREADS, 1) k_qgemm(FkState *st, const __g
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
-            if (lane == 0) qg_arrive(dempty + 8 * d);
+            if (lane == 0) tc_arrive(dempty + 8 * d);
         }
         if (!ok && lane == 0) atomicOr(&st->error, FKQ_ERR_WAIT);
     }

@@ -94,7 +94,7 @@ struct Ctx {
     float *qmm_scratch = nullptr; unsigned int *qmm_counters = nullptr;   // K-split partial sums and tickets of the several-row projection
     bool use_tiled = true; int stages = FK_STAGES; int force_warps = 0; int force_split = -1; bool qmm_tc = false; int wide_upto = 3; bool sdpa_cluster = true; bool sdpa_mma = true; int sdpa_cl = 0;
     ncclComm_t comm = nullptr; int rank = 0, world = 1;
-    bool comm_lost = false; long comm_timeout_ms = 0;
+    bool comm_lost = false; long comm_timeout_ms = 0; uint32_t wait_limit = TC_WAIT_LIMIT;
     unsigned long long *timeline = nullptr; int timeline_task = 0;      // tuning aid: per-task slices of 512 x 8 stamps
     long long launches = 0;
     uint32_t vocab = 0;                         // rows of the embedding table of the last embed task seen (0 = unknown)
@@ -145,6 +145,7 @@ extern "C" fk_status fk_open(int device, fk_handle *out) {
     CU(cudaMallocHost(&c->pinned, sizeof(uint32_t) * (c->hist_cap + 64)));
     const char *e = getenv("FK_PDL"); if (e && e[0] == '0') c->pdl = false;
     e = getenv("FK_COMM_TIMEOUT_MS"); if (e) c->comm_timeout_ms = atol(e);
+    e = getenv("FK_TC_WAIT_LIMIT"); if (e) c->wait_limit = (uint32_t)strtoul(e, nullptr, 10);
     e = getenv("FK_LAYOUT"); if (e && !strcmp(e, "mlx")) c->use_tiled = false;
     e = getenv("FK_SDPA"); if (e && !strcmp(e, "ticket")) c->sdpa_cluster = false;
     if (e && !strcmp(e, "mma")) c->sdpa_mma = true;
@@ -468,7 +469,7 @@ static fk_status run_staged(Ctx *c, const Weight *w, bool gateup, const void *xs
     if (w->k != k || w->n != (gateup ? 2LL : 1LL) * n || m <= 0 || !xs || !xscale || !y || ((uintptr_t)xs & 15)) return fail(FK_ERR_VALUE, "staged product: shape mismatch");
     if (k > FKQ_MAX_K) return fail(FK_ERR_VALUE, "staged product: at most %d columns", FKQ_MAX_K);
     const QPlan p = fkq_plan(m, w->ntiles, w->nsb, c->sm_count);
-    QGemmArgs a{w->tview(), xscale, residual, y, c->qg_scratch, c->qg_counters, w->rowmul, m, n, ldr, act, p.whole, p.mtiles, p.tiles};
+    QGemmArgs a{w->tview(), xscale, residual, y, c->qg_scratch, c->qg_counters, w->rowmul, m, n, ldr, act, p.whole, p.mtiles, p.tiles, c->wait_limit};
     CUtensorMap mx;
     if (!fkl_tensor_map(&mx, xs, m, (long long)w->nsb * FKQ_SB, (long long)w->nsb * FKQ_SB, p.bn, true)) return fail(FK_ERR_VALUE, "staged product: tensor map refused");
     *e = p.bn == 16 ? launch_qgemm<16>(c, p, gateup, mx, a) : p.bn == 32 ? launch_qgemm<32>(c, p, gateup, mx, a) : p.bn == 64 ? launch_qgemm<64>(c, p, gateup, mx, a) : launch_qgemm<128>(c, p, gateup, mx, a);
@@ -594,7 +595,7 @@ static bool rows_weight(void *owner, uint64_t id, FklWeight *out) {
 }
 static fk_status run_task(Ctx *c, const fk_task &t, const Weight *nextw = nullptr) {
     if (fkl_owns(t.kind)) {
-        FklEnv env{c->stream, c->pdl, c->sm_count, c->state, c->history, &c->launches, c, rows_weight};
+        FklEnv env{c->stream, c->pdl, c->sm_count, c->state, c->history, &c->launches, c, rows_weight, c->wait_limit};
         char err[256] = "";
         fk_status s = fkl_run(env, t, err, sizeof err);
         return s ? fail(s, "%s", err) : FK_OK;

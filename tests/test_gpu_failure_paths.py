@@ -55,6 +55,56 @@ def test_seed_token_outside_the_embedding_table_is_refused_on_the_host():
         eng.close()
 
 
+def _tensor_core_products(rt, seed):
+    """Every tcgen05 product once with its tiles whole and once split over K or spread over many blocks: (error word, results)."""
+    T, rng, out = N.Task.make, np.random.default_rng(seed), []
+    bf = lambda a: (np.ascontiguousarray(a, np.float32).view(np.uint32) >> 16).astype(np.uint16)                   # noqa: E731
+    rt.state_set(0, 0)
+    for m, k, n in ((40, 1024, 512), (16, 4096, 304), (300, 512, 2560)):
+        wid, x = rt.weight_alloc(n, k, 4), rt.to_device(bf(rng.normal(size=(m, k))))
+        rt.weight_synth_rows(wid, 0, n, 77, 0.02, k, 0, 0); rt.weight_finalize(wid)
+        y, staged, factor = rt.alloc(m * n * 2), rt.alloc(m * -(-k // 512) * 1152), rt.alloc(m * 4)
+        N.check(rt.L.fk_memset(rt.h, y, 0, m * n * 2), "fk_memset")
+        rt.launch(T(N.TASK_STAGE_ROWS, -1, {0: x, 2: staged, 3: factor}, [k, m], [1e-6]))
+        rt.launch(T(N.TASK_STAGED_LINEAR, -1, {0: staged, 1: factor, 2: wid, 4: y}, [k, n, m, 0]))
+        out.append(rt.download(y, (m, n), np.uint16))
+    staged_error = rt.state_get()[2]
+    rt.state_set(0, 0)
+    for m, k, n in ((40, 1024, 64), (700, 1024, 2048)):
+        wid, w = rt.weight_alloc(n, k, 16), bf(rng.normal(size=(n, k)))
+        rt.weight_upload_rows(wid, 0, w); rt.weight_keep_rows(wid)
+        x, y = rt.to_device(bf(rng.normal(size=(m, k)))), rt.alloc(m * n * 4)
+        N.check(rt.L.fk_memset(rt.h, y, 0, m * n * 4), "fk_memset")
+        rt.launch(T(N.TASK_LINEAR_ROWS, -1, {0: x, 1: wid, 2: y}, [m, 0, n, k, n, 0, 256, 0]))
+        out.append(rt.download(y, (m, n), np.float32))
+    return staged_error, rt.state_get()[2], out
+
+
+def test_tensor_core_products_whose_waits_run_out_report_it_and_end(monkeypatch):
+    """With no polls at all the first wait of every warp runs out: the kernels set their error bits, wait for the copies they had begun
+    and return; the handle runs other kernels afterwards, and another handle's products on the same GPU are right."""
+    want = None
+    for limit in (None, "0", None):
+        if limit is None:
+            monkeypatch.delenv("FK_TC_WAIT_LIMIT", raising=False)
+        else:
+            monkeypatch.setenv("FK_TC_WAIT_LIMIT", limit)
+        rt = Runtime(0)
+        try:
+            for _ in range(2):
+                staged, rows, got = _tensor_core_products(rt, 5)
+                if limit is None:
+                    assert staged == 0 and rows == 0
+                    want = want or got
+                    assert all(np.array_equal(a, b) and a.any() for a, b in zip(got, want))
+                else:
+                    assert staged & 0x400000 and rows & 0x200000
+                    a = np.arange(256, dtype=np.uint16)
+                    assert np.array_equal(rt.smoke(a, a).shape, a.shape)
+        finally:
+            rt.close()
+
+
 def test_close_releases_device_memory():
     """Opening and closing handles (with weights, graphs and loopback arenas) does not accumulate device memory."""
     import torch
