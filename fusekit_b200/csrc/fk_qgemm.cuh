@@ -27,23 +27,20 @@
 #pragma once
 #include "fk_stream.cuh"
 #include "fk_layers.h"
+#include "fk_qplan.h"
 #include "fk_tc.cuh"
 #include <cuda_fp16.h>
 
 #define FKQ_SB 576                      // staged halves per super-block: 512 activations, 32 slots for the sums, 32 unused
 #define FKQ_DEQ 16                      // dequantising warps: one unit each
-#define FKQ_EPI 8                       // storing warps
 #define FKQ_THREADS ((FKQ_DEQ + FKQ_EPI + 3) * 32)      // .. a warp for X, two for the MMAs
-#define FKQ_ROWS 256                    // weight rows of a block
 #define FKQ_MAX_K 32768                 // a row is staged from registers: 1024 threads x 4 vectors of 8
 #define FKQ_ERR_WAIT 0x400000u
-#define FKQ_COUNTERS 65536              // ticket words: 8 per tile that is split
 template <int BN> struct QgTile {
     static constexpr int XG = BN >= 128 ? 1 : 3, XS = BN >= 128 ? 5 : BN == 64 ? 3 : 4, XBYTES = BN * 128;        // k-blocks per stage of X, stages, bytes of a k-block
     static constexpr int NBUF = BN <= 64 ? 2 : 1, DCOLS = NBUF * 2 * BN, AS = (512 - DCOLS) / 64;                 // accumulators of a tile and the next, columns, k-blocks of A operand
     static constexpr size_t SMEM = 1024 + (size_t)XS * XG * XBYTES + (size_t)FKQ_DEQ * FK_STAGES * FK_UNIT_BYTES;
 };
-__host__ __device__ inline size_t fkq_part_floats(int bn) { return (size_t)bn * FKQ_ROWS; }
 
 struct QGemmArgs { TiledW W; const float *xscale; const uint16_t *residual; uint16_t *y; float *scratch; unsigned int *counters; const float *rowmul; int m, n, ldr, act, whole, mtiles, tiles; uint32_t limit; };
 
@@ -70,43 +67,6 @@ __device__ __forceinline__ void qg_ld16(uint32_t (&d)[16], uint32_t addr) {
                  : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]), "=r"(d[4]), "=r"(d[5]), "=r"(d[6]), "=r"(d[7]),
                    "=r"(d[8]), "=r"(d[9]), "=r"(d[10]), "=r"(d[11]), "=r"(d[12]), "=r"(d[13]), "=r"(d[14]), "=r"(d[15]) : "r"(addr) : "memory");
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-
-// The v-th piece of work of block `b` of `G`: super-blocks [k0, k1) of a tile.
-struct QWork { int tile, k0, k1; };
-__host__ __device__ inline bool fkq_work(int whole, int tiles, int nsb, int b, int G, int v, QWork &w) {
-    if (whole) { w.tile = b + v * G; w.k0 = 0; w.k1 = nsb; return w.tile < tiles; }
-    const long long T = (long long)tiles * nsb;
-    const int s0 = (int)(b * T / G), s1 = (int)((b + 1) * T / G);
-    w.tile = s0 / nsb + v;
-    const int t0 = w.tile * nsb, a = s0 > t0 ? s0 : t0, e = s1 < t0 + nsb ? s1 : t0 + nsb;
-    if (w.tile >= tiles || a >= e) return false;
-    w.k0 = a - t0; w.k1 = e - t0;
-    return true;
-}
-// the block whose run holds step s, and the scratch slot of block b's part of `tile` (two slots a block: the tile its run begins in, the one it ends in)
-__host__ __device__ inline int fkq_owner(int tiles, int nsb, int G, int s) { return (int)((((long long)s + 1) * G - 1) / ((long long)tiles * nsb)); }
-__host__ __device__ inline int fkq_slot(int tiles, int nsb, int G, int b, int tile) { return 2 * b + ((int)((long long)b * tiles * nsb / G) / nsb == tile ? 0 : 1); }
-
-// Rows of X per tile, blocks and split of a product of m rows: the widest tile that the rows fill, a narrower one while that gives more
-// blocks a tile of their own (a step costs a block the same up to 64 rows); up to 32 rows the steps are dealt in equal runs (a part's
-// sums are small, and the product is bound by the weights), from 33 on only while less than half of the blocks have a tile.
-// Measured: 100 rows, 896 -> 1152: 11 us with tiles of 16 rows, 31 with one tile of 128 split over K (its fold passes 128 rows through memory);
-// 4864 -> 896: 19 against 63.
-struct QPlan { int bn, mtiles, tiles, grid, whole; };
-inline QPlan fkq_plan(int m, int ntiles, int nsb, int sm) {
-    QPlan p;
-    p.bn = m <= 16 ? 16 : m <= 32 ? 32 : m <= 64 ? 64 : 128;
-    while (p.bn > 16 && (ntiles + 15) / 16 * ((m + p.bn / 2 - 1) / (p.bn / 2)) <= sm) p.bn /= 2;
-    p.mtiles = (m + p.bn - 1) / p.bn; p.tiles = (ntiles + 15) / 16 * p.mtiles; p.whole = 1; p.grid = p.tiles < sm ? p.tiles : sm;
-    if (p.tiles > FKQ_COUNTERS / FKQ_EPI) return p;
-    if (p.bn <= 32) {
-        if (p.tiles % sm) { const long long steps = (long long)p.tiles * nsb; p.whole = 0; p.grid = steps < sm ? (int)steps : sm; }
-    } else if (2 * p.tiles <= sm && nsb > 1) {
-        const int parts = sm / p.tiles < nsb ? sm / p.tiles : nsb;
-        p.whole = 0; p.grid = p.tiles * parts;
-    }
-    return p;
 }
 
 template <int BN, bool GATEUP>
@@ -323,9 +283,20 @@ __global__ void __launch_bounds__(FKQ_THREADS, 1) k_qgemm(FkState *st, const __g
         // plain rows in pairs: neighbouring lanes trade so that each holds two weight rows of one row of X (even lanes the even one), and
         // loads and stores are 4 bytes wide
         const bool pairs = !GATEUP && !(a.n & 1) && !(a.ldr & 1) && !(((uintptr_t)a.y | (uintptr_t)a.residual) & 3);
-        for (int v = 0; ok && fkq_work(a.whole, a.tiles, nsb, me, G, v, w); ++v) {
+        // counts a part of a tile; true for the last one
+        auto count = [&](int tile) {
+            const unsigned int most = (unsigned int)fkq_parts(a.tiles, nsb, G, tile) - 1u;
+            unsigned int ticket = 0;
+            if (lane == 0) {
+                unsigned int *word = a.counters + (size_t)tile * FKQ_EPI + ew;
+                ticket = atomicAdd(word, 1u);
+                if (ticket == most) *word = 0u;         // all parts are in: ready for the next launch
+            }
+            return __shfl_sync(0xffffffffu, ticket, 0) == most;
+        };
+        ok = fkq_pieces(a.whole, a.tiles, nsb, me, G, [&](int v, const QWork &w) {
             const int d = v % NBUF, rt = w.tile / a.mtiles, m0 = (w.tile - rt * a.mtiles) * BN, row0 = rt * FKQ_ROWS + sub * 128 + q * 32, n = row0 + lane;
-            const bool part = w.k0 != 0 || w.k1 != nsb;
+            const bool part = fkq_part(w, nsb);
             const int rows = min(BN, a.m - m0);         // of X that there are
             uint32_t res[16];                           // residual pairs of 32 rows of X on their way
             auto fetch = [&](int c, auto &r) {
@@ -345,7 +316,7 @@ __global__ void __launch_bounds__(FKQ_THREADS, 1) k_qgemm(FkState *st, const __g
             };
             const float rmul = row0 + lane < a.W.ntiles * 16 ? __uint_as_float(0x7F000000u - __float_as_uint(__ldg(a.rowmul + row0 + lane))) : 0.0f;       // 2^-k of 2^k
             if (!GATEUP && !part) fetch(0, res);        // under the tile's MMAs
-            if (!tc_wait_warp(dfull + 8 * d, (uint32_t)(v / NBUF) & 1u, a.limit)) { ok = false; break; }
+            if (!tc_wait_warp(dfull + 8 * d, (uint32_t)(v / NBUF) & 1u, a.limit)) return false;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t src = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)((d * 2 + sub) * BN);
             // rows c .. of X, whose factors lanes f0 .. hold; r: their residual pairs
@@ -409,16 +380,10 @@ __global__ void __launch_bounds__(FKQ_THREADS, 1) k_qgemm(FkState *st, const __g
 #pragma unroll
                     for (int i = 0; i < 16; ++i) __stcg(mine + (size_t)(c + i) * FKQ_ROWS, __uint_as_float(r[i]));
                 }
-                const int first = fkq_owner(a.tiles, nsb, G, w.tile * nsb), last = fkq_owner(a.tiles, nsb, G, (w.tile + 1) * nsb - 1);
+                const int first = fkq_owner(a.tiles, nsb, G, w.tile * nsb), last = first + fkq_parts(a.tiles, nsb, G, w.tile) - 1;
                 __threadfence();
                 __syncwarp();
-                unsigned int ticket = 0;
-                if (lane == 0) {
-                    ticket = atomicAdd(a.counters + (size_t)w.tile * FKQ_EPI + ew, 1u);
-                    if (ticket == (unsigned int)(last - first)) a.counters[(size_t)w.tile * FKQ_EPI + ew] = 0u;      // all parts are in: ready for the next launch
-                }
-                const bool finish = __shfl_sync(0xffffffffu, ticket, 0) == (unsigned int)(last - first);
-                if (finish) {
+                if (count(w.tile)) {
                     __threadfence();
                     const float *from = a.scratch + sub * 128 + q * 32 + lane;
 #pragma unroll 1
@@ -449,7 +414,8 @@ __global__ void __launch_bounds__(FKQ_THREADS, 1) k_qgemm(FkState *st, const __g
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) tc_arrive(dempty + 8 * d);
-        }
+            return true;
+        }, [&](const QWork &w) { count(w.tile); });
         if (!ok && lane == 0) atomicOr(&st->error, FKQ_ERR_WAIT);
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");

@@ -1,0 +1,70 @@
+// How a product of staged rows (fk_qgemm.cuh) is dealt to blocks.  Plain C++, so that the host plans with it and tests run it without a GPU.
+#pragma once
+#include <stddef.h>
+
+#if defined(__CUDACC__)
+#define FKQ_HD __host__ __device__
+#else
+#define FKQ_HD
+#endif
+#define FKQ_EPI 8                       // storing warps of a block
+#define FKQ_ROWS 256                    // weight rows of a block
+#define FKQ_COUNTERS 65536              // ticket words: 8 per tile that is split
+FKQ_HD inline size_t fkq_part_floats(int bn) { return (size_t)bn * FKQ_ROWS; }
+
+// The v-th piece of work of block `b` of `G`: super-blocks [k0, k1) of a tile.
+struct QWork { int tile, k0, k1; };
+FKQ_HD inline bool fkq_work(int whole, int tiles, int nsb, int b, int G, int v, QWork &w) {
+    if (whole) { w.tile = b + v * G; w.k0 = 0; w.k1 = nsb; return w.tile < tiles; }
+    const long long T = (long long)tiles * nsb;
+    const int s0 = (int)(b * T / G), s1 = (int)((b + 1) * T / G);
+    w.tile = s0 / nsb + v;
+    const int t0 = w.tile * nsb, a = s0 > t0 ? s0 : t0, e = s1 < t0 + nsb ? s1 : t0 + nsb;
+    if (w.tile >= tiles || a >= e) return false;
+    w.k0 = a - t0; w.k1 = e - t0;
+    return true;
+}
+// the block whose run holds step s, and the scratch slot of block b's part of `tile` (two slots a block: the tile its run begins in, the one it ends in)
+FKQ_HD inline int fkq_owner(int tiles, int nsb, int G, int s) { return (int)((((long long)s + 1) * G - 1) / ((long long)tiles * nsb)); }
+FKQ_HD inline int fkq_slot(int tiles, int nsb, int G, int b, int tile) { return 2 * b + ((int)((long long)b * tiles * nsb / G) / nsb == tile ? 0 : 1); }
+
+// A piece that covers part of a tile: its sums go to the scratch area and a ticket of the tile is counted; of the warps that store the same
+// rows the one that counts the last of the tile's parts adds them up and sets the ticket word to zero.
+FKQ_HD inline bool fkq_part(const QWork &w, int nsb) { return w.k0 != 0 || w.k1 != nsb; }
+FKQ_HD inline int fkq_parts(int tiles, int nsb, int G, int tile) { return fkq_owner(tiles, nsb, G, (tile + 1) * nsb - 1) - fkq_owner(tiles, nsb, G, tile * nsb) + 1; }
+// The pieces of block b in the hands of one storing warp.  take(v, w) waits for the piece and stores it (counting its ticket if it is a part); it
+// returns false, with nothing counted, when the wait runs out.  From then on nothing is taken, but skip(w) still counts the
+// ticket of every part: the ticket words are zero again after every launch, also after one that gave up.
+#if defined(__CUDACC__)
+#pragma nv_exec_check_disable
+#endif
+template <typename Take, typename Skip> FKQ_HD inline bool fkq_pieces(int whole, int tiles, int nsb, int b, int G, Take take, Skip skip) {
+    bool ok = true;
+    QWork w;
+    for (int v = 0; fkq_work(whole, tiles, nsb, b, G, v, w); ++v) {
+        ok = ok && take(v, w);
+        if (!ok && fkq_part(w, nsb)) skip(w);
+    }
+    return ok;
+}
+
+// Rows of X per tile, blocks and split of a product of m rows: the widest tile that the rows fill, a narrower one while that gives more
+// blocks a tile of their own (a step costs a block the same up to 64 rows); up to 32 rows the steps are dealt in equal runs (a part's
+// sums are small, and the product is bound by the weights), from 33 on only while less than half of the blocks have a tile.
+// Measured: 100 rows, 896 -> 1152: 11 us with tiles of 16 rows, 31 with one tile of 128 split over K (its fold passes 128 rows through memory);
+// 4864 -> 896: 19 against 63.
+struct QPlan { int bn, mtiles, tiles, grid, whole; };
+inline QPlan fkq_plan(int m, int ntiles, int nsb, int sm) {
+    QPlan p;
+    p.bn = m <= 16 ? 16 : m <= 32 ? 32 : m <= 64 ? 64 : 128;
+    while (p.bn > 16 && (ntiles + 15) / 16 * ((m + p.bn / 2 - 1) / (p.bn / 2)) <= sm) p.bn /= 2;
+    p.mtiles = (m + p.bn - 1) / p.bn; p.tiles = (ntiles + 15) / 16 * p.mtiles; p.whole = 1; p.grid = p.tiles < sm ? p.tiles : sm;
+    if (p.tiles > FKQ_COUNTERS / FKQ_EPI) return p;
+    if (p.bn <= 32) {
+        if (p.tiles % sm) { const long long steps = (long long)p.tiles * nsb; p.whole = 0; p.grid = steps < sm ? (int)steps : sm; }
+    } else if (2 * p.tiles <= sm && nsb > 1) {
+        const int parts = sm / p.tiles < nsb ? sm / p.tiles : nsb;
+        p.whole = 0; p.grid = p.tiles * parts;
+    }
+    return p;
+}
