@@ -39,7 +39,7 @@ __global__ void __launch_bounds__(256, VD <= 128 && KD <= 64 ? 2 : 1) k_flash_ro
     pdl_launch_dependents(); pdl_wait();
     const int off = (int)st->offset;
     const int last = off + min(row0 + 63, a.rows - 1);  // newest position of the block
-    if (off + a.rows > a.cap) return;                   // reported by the cache store that came before
+    if (a.rows > a.cap || st->offset > (uint32_t)(a.cap - a.rows)) return;      // reported by the cache store that came before
     const int wtile = WIN ? max(0, off + row0 - a.window + 1) / 64 : 0, kept = WIN ? min((a.keep + 63) / 64, wtile) : 0, ntiles = kept + last / 64 - wtile + 1;
     auto place = [&](int i) { return i < kept ? i : wtile + i - kept; };
     const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(fl_smem), stage = (uint32_t)flash_stage_bytes<KD, VD>(a.maps);

@@ -6,7 +6,6 @@
 #define FKL_MAX_EXPERTS 1024
 #define FKL_MAX_TOP 64
 #define FKL_GV_MAX_GROUPS 1024        // groups of a mixer's output norm
-#define FKL_ERR_CAPACITY 0x100000u
 #define FKL_ERR_TC_WAIT 0x200000u
 
 enum { FKL_ACT_NONE = 0, FKL_ACT_RELU2 = 2, FKL_ACT_SILU = 3 };

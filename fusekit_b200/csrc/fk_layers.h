@@ -6,6 +6,7 @@
 #include <cuda.h>
 
 #define FKL_ERR_TOKEN 0x20000u
+#define FKL_ERR_CAPACITY 0x100000u
 
 struct FklWeight { const uint16_t *rows; long long n, k; };       // bf16 rows [n, k] as uploaded (fk_weight_keep_rows)
 struct FklEnv {

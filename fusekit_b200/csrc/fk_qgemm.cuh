@@ -564,13 +564,18 @@ __global__ void __launch_bounds__(512) k_argmax_prompt(const FkState *st, const 
     }
 }
 // RoPE and the cache store of consecutive positions: a block takes a position, works out its angles once for all heads (rope_pair's
-// arithmetic) and moves 4 bytes a thread.  (A block per head and position, each with its own sine and cosine, took 39 us for 1000 positions
+// arithmetic) and moves 4 bytes a thread.  Positions past the capacity are an error, and
+// nothing is stored.  (A block per head and position, each with its own sine and cosine, took 39 us for 1000 positions
 // of the 7B shape: 36000 blocks of 64 threads.)
-__global__ void __launch_bounds__(256) k_rope_store_prompt(const FkState *st, RopeRowsArgs a) {
+__global__ void __launch_bounds__(256) k_rope_store_prompt(FkState *st, RopeRowsArgs a) {
     __shared__ float2 turn[256];
     const int m = blockIdx.x, half = a.hd >> 1, quads = half >> 1;       // pairs of dimensions a thread turns together
     pdl_wait(); pdl_launch_dependents();
-    const uint32_t pos = st->offset + (uint32_t)m; const int wrow = (int)(pos % (uint32_t)a.capacity);
+    const uint32_t pos = st->offset + (uint32_t)m;
+    if (a.rows > a.capacity || st->offset > (uint32_t)(a.capacity - a.rows)) {      // two blocks might store one row, and k_flash_rows does not wrap
+        if (m == 0 && threadIdx.x == 0) atomicOr(&st->error, FKL_ERR_CAPACITY);
+        return;
+    }
     for (int d = threadIdx.x; d < half; d += blockDim.x) {
         const float e = __fmul_rn(-__fdiv_rn((float)d, (float)half), a.log2theta), ang = __fmul_rn((float)pos, exp2f(e));
         float s, c; sincosf(ang, &s, &c);
@@ -588,7 +593,7 @@ __global__ void __launch_bounds__(256) k_rope_store_prompt(const FkState *st, Ro
             lo = o0; hi = o1;
         }
         uint16_t *dst = head < a.n_q ? a.q_out + ((size_t)m * a.n_q + head) * a.hd
-                      : head < a.n_q + a.n_kv ? a.cache_k + ((size_t)(head - a.n_q) * a.capacity + wrow) * a.hd : a.cache_v + ((size_t)(head - a.n_q - a.n_kv) * a.capacity + wrow) * a.hd;
+                      : head < a.n_q + a.n_kv ? a.cache_k + ((size_t)(head - a.n_q) * a.capacity + pos) * a.hd : a.cache_v + ((size_t)(head - a.n_q - a.n_kv) * a.capacity + pos) * a.hd;
         *reinterpret_cast<uint32_t *>(dst + d) = lo; *reinterpret_cast<uint32_t *>(dst + d + half) = hi;
     }
 }

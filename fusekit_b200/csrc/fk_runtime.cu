@@ -898,7 +898,7 @@ static fk_status run_task(Ctx *c, const fk_task &t, const Weight *nextw = nullpt
         const int nq = i[0], nkv = i[1], hd = i[2], cap = i[3], rows = i[4];
         if (!b[0] || !b[1] || !b[5] || !b[6] || nq <= 0 || nkv <= 0 || hd <= 0 || hd % 8 || hd > 512 || cap <= 0 || rows <= 0 || ((b[0] | b[1] | b[5] | b[6]) & 3)) return fail(FK_ERR_VALUE, "rope_store_prompt: bad arguments (head sizes in multiples of 8 up to 512)");
         RopeRowsArgs a{(const uint16_t *)b[0], (uint16_t *)b[1], (uint16_t *)b[5], (uint16_t *)b[6], nq, nkv, hd, cap, rows, (float)log2((double)f[1]), 1};
-        e = launch(c, k_rope_store_prompt, dim3(rows), dim3(256), 0, (const FkState *)c->state, a);
+        e = launch(c, k_rope_store_prompt, dim3(rows), dim3(256), 0, c->state, a);
         break;
     }
     case FK_TASK_ARGMAX_PROMPT: {

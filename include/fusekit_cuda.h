@@ -237,7 +237,8 @@ enum { FK_ACT_NONE = 0, FK_ACT_RELU_SQUARED = 2, FK_ACT_SILU = 3 };
  *                      i0 K  i1 N  i2 M (any number)  i3 = 1: one residual row T[N] for all.  Row m is LINEAR_RESIDUAL's for x[m]
  * STAGED_GATEUP        buf0 staged rows  buf1 row factors  buf2 weight (fk_weight_pair)  buf4 act_out T[M, I]   i0 H  i1 I  i2 M  i3 act
  * EMBED_PROMPT         buf0 table T[V, H]  buf1 x T[M, H]  buf2 token ids u32[M] (a device buffer)   i0 H  i1 M  i2 V
- * ROPE_STORE_PROMPT    ROPE_STORE_ROWS for any number of consecutive positions (head_dim a multiple of 8, at most 512)
+ * ROPE_STORE_PROMPT    ROPE_STORE_ROWS for any number of consecutive positions (head_dim a multiple of 8, at most 512), without its wrap: past the
+ *                      capacity nothing is stored and the error word gets 0x100000
  * ARGMAX_PROMPT        buf0 logits T[M, V]  buf1 greedy ids u32[M]   i0 V (a multiple of 8)  i1 M; the decode state is left alone
  *
  * Batch decode (M = 2..16 independent sequences at one position): EMBED with i1 = M, LINEAR_RESIDUAL / RMSNORM_GATEUP_ACT

@@ -162,3 +162,28 @@ def test_whole_prompts_match_the_steps(rows, count):
         assert sum(a != b for a, b in zip(got[name][0], got["steps"][0])) <= max(2, count // 16), name
         for a, b in zip(got[name][1:], got["steps"][1:]):
             assert np.sqrt(np.mean((a - b) ** 2)) <= 8e-3 * np.sqrt(np.mean(b ** 2)), name
+
+
+@pytest.mark.parametrize("offset,rows", [(41, 60), (0, 101), (100, 1), (2 ** 31 - 20, 40), (2 ** 32 - 1, 2)])
+def test_prompt_positions_past_the_capacity_are_reported(runtime, offset, rows):
+    """The store sets its error bit and leaves queries and caches alone, and attention over them writes nothing; at the capacity's very end both work."""
+    rt, nq, nkv, hd, cap = runtime, 4, 2, 64, 100
+    qkv = rt.to_device(_rows(rows, (nq + 2 * nkv) * hd, 3))
+    sizes = {"q": rows * nq * hd, "k": nkv * cap * hd, "v": nkv * cap * hd, "out": rows * nq * hd}
+    buf = {n: rt.alloc(s * 2) for n, s in sizes.items()}
+
+    def run(at, m):
+        for n, s in sizes.items():
+            N.check(rt.L.fk_memset(rt.h, buf[n], 0x3f, s * 2), "fk_memset")
+        rt.state_set(0, at)
+        rt.launch(T(N.TASK_ROPE_STORE_PROMPT, 0, {0: qkv, 1: buf["q"], 5: buf["k"], 6: buf["v"]}, [nq, nkv, hd, cap, m], [0.0, 1e4]))
+        rt.launch(T(N.TASK_ATTENTION_ROWS, 0, {0: buf["q"], 1: buf["k"], 2: buf["v"], 3: buf["out"]}, [nq, nkv, hd, hd, cap, m, 1 << 8], [0.125]))
+        return rt.state_get()[2], {n: rt.download(buf[n], (s,), np.uint16) for n, s in sizes.items()}
+
+    err, got = run(offset, rows)
+    assert err == 0x100000 and all((a == 0x3f3f).all() for a in got.values())
+    m = min(rows, cap)
+    err, got = run(cap - m, m)
+    assert err == 0 and (got["k"].reshape(nkv, cap, hd)[:, cap - m:] != 0x3f3f).any(2).all()
+    for p in [qkv, *buf.values()]:
+        N.check(rt.L.fk_free(rt.h, p), "fk_free")
