@@ -63,6 +63,7 @@ class BatchDecodeEngine:
         self.staged, self.factor = rt.alloc(M * -(-H // 512) * 1152), rt.alloc(M * 4)      # rows as the staged products read them
         self.graph = 0
         self.scratch: dict[str, int] = {}       # of whole prompts (PrefillEngine)
+        self.most = (0, 0)                      # positions of a portion and rows of logits that it holds
         self.portions: dict[tuple, object] = {}     # task lists by (rows, last portion)
 
     def x_ptr(self, l): return self.X + l * self.rows * self.spec.hidden * 2
@@ -216,11 +217,11 @@ class PrefillEngine(BatchDecodeEngine):
 
     def capture(self) -> int:
         if self._staged and not self.scratch and self.capacity > self.rows:
-            s, P, rt = self.spec, min(self.PORTION, self.capacity), self.rt
-            H, A = s.hidden, s.n_q * s.head_dim
+            s, P, rt = self.spec, max(self.rows, min(self.PORTION, self.capacity)), self.rt
+            H, A, self.most = s.hidden, s.n_q * s.head_dim, (P, min(P, self.HEAD_ROWS))
             self.scratch = {k: rt.alloc(n) for k, n in {
                 "tokens": P * 4, "greedy": P * 4, "x": P * H * 2, "hb": P * H * 2, "qkv": P * self.nqkv * 2, "q": P * A * 2, "att": P * A * 2, "act": P * s.inter * 2,
-                "staged": P * max(-(-k // 512) for k in (H, A, s.inter)) * 1152, "factor": P * 4, "logits": min(P, self.HEAD_ROWS) * s.vocab * 2}.items()}
+                "staged": P * max(-(-k // 512) for k in (H, A, s.inter)) * 1152, "factor": P * 4, "logits": self.most[1] * s.vocab * 2}.items()}
         return super().capture()
 
     def prompt_dispatches(self, rows: int, last: bool) -> list:
@@ -243,9 +244,9 @@ class PrefillEngine(BatchDecodeEngine):
             tasks += [T(N.TASK_STAGE_ROWS, l, {0: S["hb"], 1: V[p + "post_attention_norm"], 2: S["staged"], 3: S["factor"]}, [H, M], [s.eps]),
                       T(N.TASK_STAGED_GATEUP, l, {0: S["staged"], 1: S["factor"], 2: self.W[p + "gateup"], 4: S["act"]}, [H, I, M, N.ACT_SWIGLU])]
             tasks += product(l, S["act"], 0, I, self.W[p + "down"], H, S["x"], S["hb"])
-        final = (M - 1) // self.rows * self.rows if last else M
-        for r0 in list(range(0, final, self.HEAD_ROWS)) + ([final] if last else []):
-            m = min(self.HEAD_ROWS, final - r0) if r0 < final else M - final
+        final, most = (M - 1) // self.rows * self.rows if last else M, min(self.HEAD_ROWS, self.most[1])
+        for r0 in list(range(0, final, most)) + ([final] if last else []):
+            m = min(most, final - r0) if r0 < final else M - final
             out = S["logits"] if r0 < final else self.logits
             tasks += product(-1, S["x"], V["final_norm"], H, self.W["lm_head"], s.vocab, out, at=r0, m=m)
             tasks.append(T(N.TASK_ARGMAX_PROMPT, -1, {0: out, 1: S["greedy"] + r0 * 4}, [s.vocab, m]))
@@ -257,7 +258,7 @@ class PrefillEngine(BatchDecodeEngine):
         ids = np.array(toks, np.uint32)
         if ids.max() >= self.spec.vocab:
             raise N.FusekitError(f"token id {int(ids[ids >= self.spec.vocab][0])} is outside the embedding table ({self.spec.vocab} rows)")
-        most = min(self.PORTION, self.capacity) // M * M
+        most = max(M, min(self.PORTION, self.most[0]) // M * M)
         for c0 in range(0, n, most):
             part = ids[c0:c0 + most]
             key = (len(part), c0 + most >= n)

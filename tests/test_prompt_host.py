@@ -1,0 +1,82 @@
+"""Host side of whole prompts (PrefillEngine) against a runtime that only keeps books: what is allocated, and which buffers and weights
+the launched tasks name."""
+from dataclasses import replace
+from types import SimpleNamespace
+
+import numpy as np
+
+from fusekit_b200 import _native as N
+from fusekit_b200.batch import PrefillEngine
+from fusekit_b200.model_spec import CONFIGS
+
+
+class Books:
+    def __init__(self):
+        self.next, self.weights, self.sizes, self.launched, self.h = 1 << 20, 0, {}, [], 0
+        self.L = SimpleNamespace(fk_launch_batch=self._launch, fk_graph_capture=self._capture)
+
+    def _launch(self, h, arr, n):
+        self.launched.append([(t.kind, list(t.buf), list(t.iarg)) for t in arr[:n]])
+        return 0
+
+    def _capture(self, h, arr, n, out):
+        out._obj.value = 1
+        return 0
+
+    def info(self):
+        return {"sm": 148}
+
+    def alloc(self, n):
+        p = self.next
+        self.next += -(-n // 256) * 256 + 256
+        self.sizes[p] = n
+        return p
+
+    def weight_alloc(self, n, k, bits):
+        self.weights += 1
+        return self.weights
+
+    def weight_pair(self, gate, up):
+        return self.weight_alloc(0, 0, 4)
+
+    def download(self, p, shape, dtype):
+        return np.zeros(shape, dtype)
+
+    def state_get(self):
+        return 0, 0, 0
+
+    def __getattr__(self, name):                    # uploads, synthetic values, state: nothing to do
+        return lambda *a: None
+
+
+def _engine(rows=4, capacity=400, **kw):
+    eng = PrefillEngine(replace(CONFIGS["tiny-qwen"], n_layers=2), capacity, rows, runtime=Books(), **kw)
+    eng.load_synthetic()
+    eng.capture()
+    return eng
+
+
+def _inside(rt, p, n):
+    """Bytes [p, p + n) lie in one allocation."""
+    return any(q <= p and p + n <= q + size for q, size in rt.sizes.items())
+
+
+def test_prompt_scratch_holds_what_the_tasks_write_whatever_the_portion_is_set_to_later():
+    eng = _engine()
+    rt, s = eng.rt, eng.spec
+    eng.PORTION, eng.HEAD_ROWS = 64, 16
+    eng.prefill([1] * 200)
+    eng.PORTION, eng.HEAD_ROWS = 4096, 4096
+    eng.prefill([1] * 399)
+    eng.PORTION, eng.HEAD_ROWS = 24, 7
+    eng.prefill([1] * 90)
+    seen = 0
+    for tasks in rt.launched:
+        for kind, buf, i in tasks:
+            out = {N.TASK_EMBED_PROMPT: (buf[1], i[0] * i[1] * 2), N.TASK_STAGE_ROWS: (buf[2], i[1] * -(-i[0] // 512) * 1152),
+                   N.TASK_STAGED_LINEAR: (buf[4], i[1] * i[2] * 2), N.TASK_STAGED_GATEUP: (buf[4], i[1] * i[2] * 2),
+                   N.TASK_ROPE_STORE_PROMPT: (buf[1], i[0] * i[2] * i[4] * 2), N.TASK_ATTENTION_ROWS: (buf[3], i[0] * i[3] * i[5] * 2),
+                   N.TASK_ARGMAX_PROMPT: (buf[1], i[1] * 4)}[kind]
+            seen += 1
+            assert _inside(rt, *out), (kind, i[:6])
+    assert seen > 100 and s.n_layers == 2
