@@ -65,6 +65,7 @@ class BatchDecodeEngine:
         self.scratch: dict[str, int] = {}       # of whole prompts (PrefillEngine)
         self.most = (0, 0)                      # positions of a portion and rows of logits that it holds
         self.portions: dict[tuple, object] = {}     # task lists by (rows, last portion)
+        self.bound: tuple[dict, dict] = ({}, {})    # weights and vectors that the captured step names
 
     def x_ptr(self, l): return self.X + l * self.rows * self.spec.hidden * 2
     def hb_ptr(self, l): return self.HB + l * self.rows * self.spec.hidden * 2
@@ -222,12 +223,14 @@ class PrefillEngine(BatchDecodeEngine):
             self.scratch = {k: rt.alloc(n) for k, n in {
                 "tokens": P * 4, "greedy": P * 4, "x": P * H * 2, "hb": P * H * 2, "qkv": P * self.nqkv * 2, "q": P * A * 2, "att": P * A * 2, "act": P * s.inter * 2,
                 "staged": P * max(-(-k // 512) for k in (H, A, s.inter)) * 1152, "factor": P * 4, "logits": self.most[1] * s.vocab * 2}.items()}
+        self.bound = dict(self.W), dict(self.V)     # prompts of any length name what the step's graph names,
+        self.portions.clear()                       # also after other weights were loaded
         return super().capture()
 
     def prompt_dispatches(self, rows: int, last: bool) -> list:
         """One portion of a prompt, positions offset .. offset + rows - 1; with `last` the logits of its last step of `self.rows`
         positions (counted from the prompt's start: portions before are whole steps) end up where a step leaves them."""
-        s, M, H, hd, I, S, V = self.spec, rows, self.spec.hidden, self.spec.head_dim, self.spec.inter, self.scratch, self.V
+        s, M, H, hd, I, S, (W, V) = self.spec, rows, self.spec.hidden, self.spec.head_dim, self.spec.inter, self.scratch, self.bound
         T, A = N.Task.make, self.spec.n_q * self.spec.head_dim
 
         def product(l, src, norm, k, weight, n, out, residual=0, one=0, at=0, m=M):
@@ -237,18 +240,18 @@ class PrefillEngine(BatchDecodeEngine):
         tasks = [T(N.TASK_EMBED_PROMPT, -1, {0: V["embed_tokens"], 1: S["x"], 2: S["tokens"]}, [H, M, s.vocab])]
         for l in range(s.n_layers):
             (ck, cv), p = self.cache[l], f"layers.{l}."
-            tasks += product(l, S["x"], V[p + "input_norm"], H, self.W[p + "qkv"], self.nqkv, S["qkv"], V[p + "qkv_bias_rows"], 1)
+            tasks += product(l, S["x"], V[p + "input_norm"], H, W[p + "qkv"], self.nqkv, S["qkv"], V[p + "qkv_bias_rows"], 1)
             tasks += [T(N.TASK_ROPE_STORE_PROMPT, l, {0: S["qkv"], 1: S["q"], 5: ck, 6: cv}, [s.n_q, s.n_kv, hd, self.capacity, M], [0.0, s.theta]),
                       T(N.TASK_ATTENTION_ROWS, l, {0: S["q"], 1: ck, 2: cv, 3: S["att"]}, [s.n_q, s.n_kv, hd, hd, self.capacity, M, 1 << 8], [1.0 / math.sqrt(hd)])]
-            tasks += product(l, S["att"], 0, A, self.W[p + "o"], H, S["hb"], S["x"])
+            tasks += product(l, S["att"], 0, A, W[p + "o"], H, S["hb"], S["x"])
             tasks += [T(N.TASK_STAGE_ROWS, l, {0: S["hb"], 1: V[p + "post_attention_norm"], 2: S["staged"], 3: S["factor"]}, [H, M], [s.eps]),
-                      T(N.TASK_STAGED_GATEUP, l, {0: S["staged"], 1: S["factor"], 2: self.W[p + "gateup"], 4: S["act"]}, [H, I, M, N.ACT_SWIGLU])]
-            tasks += product(l, S["act"], 0, I, self.W[p + "down"], H, S["x"], S["hb"])
+                      T(N.TASK_STAGED_GATEUP, l, {0: S["staged"], 1: S["factor"], 2: W[p + "gateup"], 4: S["act"]}, [H, I, M, N.ACT_SWIGLU])]
+            tasks += product(l, S["act"], 0, I, W[p + "down"], H, S["x"], S["hb"])
         final, most = (M - 1) // self.rows * self.rows if last else M, min(self.HEAD_ROWS, self.most[1])
         for r0 in list(range(0, final, most)) + ([final] if last else []):
             m = min(most, final - r0) if r0 < final else M - final
             out = S["logits"] if r0 < final else self.logits
-            tasks += product(-1, S["x"], V["final_norm"], H, self.W["lm_head"], s.vocab, out, at=r0, m=m)
+            tasks += product(-1, S["x"], V["final_norm"], H, W["lm_head"], s.vocab, out, at=r0, m=m)
             tasks.append(T(N.TASK_ARGMAX_PROMPT, -1, {0: out, 1: S["greedy"] + r0 * 4}, [s.vocab, m]))
         return tasks
 

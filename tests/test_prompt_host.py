@@ -80,3 +80,22 @@ def test_prompt_scratch_holds_what_the_tasks_write_whatever_the_portion_is_set_t
             seen += 1
             assert _inside(rt, *out), (kind, i[:6])
     assert seen > 100 and s.n_layers == 2
+
+
+def test_prompts_follow_the_weights_of_the_captured_step():
+    eng = _engine()
+    rt = eng.rt
+
+    def weights(count):
+        rt.launched.clear()
+        eng.prefill([1] * count)
+        return {buf[2] for tasks in rt.launched for kind, buf, _ in tasks if kind in (N.TASK_STAGED_LINEAR, N.TASK_STAGED_GATEUP)}, {
+            buf[1] for tasks in rt.launched for kind, buf, _ in tasks if kind == N.TASK_STAGE_ROWS} - {0}
+
+    first = weights(30)
+    assert first[0] == set(eng.W.values())
+    eng.load_synthetic()                            # a step still replays the graph of the weights before
+    assert weights(30) == first and weights(31) == first
+    eng.capture()
+    again = weights(30)
+    assert again == weights(31) and again[0] == set(eng.W.values()) and not (again[0] | again[1]) & (first[0] | first[1])
