@@ -323,7 +323,10 @@ __global__ void __launch_bounds__(FKQ_THREADS, 1) k_qgemm(FkState *st, const __g
             auto store = [&](int c, int f0, float factor, auto &acc, const uint32_t *r) {
                 constexpr int NM = sizeof(acc) / 4;
 #pragma unroll
-                for (int i = 0; i < NM; ++i) acc[i] = acc[i] * __shfl_sync(0xffffffffu, factor, f0 + i) * rmul;
+                for (int i = 0; i < NM; ++i) {          // the smaller power of two first: no overflow on the way to a result in range
+                    const float f = __shfl_sync(0xffffffffu, factor, f0 + i);
+                    acc[i] = acc[i] * fminf(f, rmul) * fmaxf(f, rmul);
+                }
                 if (GATEUP) {
                     // lanes 0-7 / 16-23 hold gate rows, 8-15 / 24-31 the up rows of the same outputs: the lower half takes the even row of X of a
                     // pair, the upper half the odd one

@@ -91,6 +91,26 @@ def test_staged_linear_against_64_bits(runtime, m, k, n, wide):
         N.check(rt.L.fk_free(rt.h, p), "fk_free")
 
 
+# rows of X and weights at opposite ends of the range, and both large or small: every result is in range, the factors' order decides
+@pytest.mark.parametrize("xs,ws", [(2.0 ** 116, 2.0 ** -30), (2.0 ** 120, 2.0 ** -100), (2.0 ** -110, 2.0 ** 100), (2.0 ** 60, 2.0 ** 50), (2.0 ** -60, 2.0 ** -40)])
+@pytest.mark.parametrize("m,k,n", [(5, 1024, 272), (200, 896, 304)])
+def test_staged_linear_at_the_ends_of_the_range(runtime, m, k, n, xs, ws):
+    rt = runtime
+    w = _gen(f"staged.ends.{k}.{n}", n, k)
+    w.scales, w.biases = (O.f32_to_bf16(O.bf16_to_f32(a) * np.float32(ws)) for a in (w.scales, w.biases))
+    x = O.f32_to_bf16(O.bf16_to_f32(_rows(m, k, 11)) * np.float32(xs))
+    wid = _weight(rt, w); rt.weight_finalize(wid)
+    xd, yd = rt.to_device(x), rt.alloc(m * n * 2)
+    staged, factor = _stage(rt, xd, m, k)
+    rt.launch(T(N.TASK_STAGED_LINEAR, -1, {0: staged, 1: factor, 2: wid, 4: yd}, [k, n, m, 0]))
+    got = O.bf16_to_f32(rt.download(yd, (m, n), np.uint16)).astype(np.float64)
+    V, X = _values(w), O.bf16_to_f32(x).astype(np.float64)
+    assert np.abs(X @ V.T).max() < 2.0 ** 127
+    _check(got, X @ V.T, np.abs(X) @ np.abs(V).T, (m, k, n, xs, ws))
+    for p in (xd, yd, staged, factor):
+        N.check(rt.L.fk_free(rt.h, p), "fk_free")
+
+
 def test_staged_linear_keeps_infinities_and_nan_in_their_rows(runtime):
     rt = runtime
     m, k, n = 20, 576, 300
