@@ -438,15 +438,16 @@ __global__ void __launch_bounds__(256) k_row_factors(const uint4 *units, float *
         const uint32_t s[2] = {v.x, v.y}, b[2] = {v.z, v.w};
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-            const float c[4] = {1024.0f * fabsf(bf_lo(s[h])), 1024.0f * fabsf(bf_hi(s[h])), fabsf(fmaf(8.0f, bf_lo(s[h]), bf_lo(b[h]))), fabsf(fmaf(8.0f, bf_hi(s[h]), bf_hi(b[h])))};
+            // a 1024th of both, which is finite wherever s and b are
+            const float t = 0.0009765625f, c[4] = {fabsf(bf_lo(s[h])), fabsf(bf_hi(s[h])), fabsf(fmaf(8.0f * t, bf_lo(s[h]), t * bf_lo(b[h]))), fabsf(fmaf(8.0f * t, bf_hi(s[h]), t * bf_hi(b[h])))};
 #pragma unroll
-            for (int j = 0; j < 4; ++j) if (c[j] <= 3.0e38f) top[h] = fmaxf(top[h], c[j]);
+            for (int j = 0; j < 4; ++j) if (c[j] < INFINITY) top[h] = fmaxf(top[h], c[j]);
         }
     }
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
         top[h] = fmaxf(top[h], __shfl_xor_sync(0xffffffffu, top[h], 1)); top[h] = fmaxf(top[h], __shfl_xor_sync(0xffffffffu, top[h], 2));
-        int e = top[h] > 0.0f ? (int)(__float_as_uint(top[h]) >> 23) - 127 : 14;
+        int e = top[h] > 0.0f ? (int)(__float_as_uint(top[h]) >> 23) - 117 : 14;
         e = e < -110 ? -110 : e;                        // factor and inverse stay normal numbers
         if ((lane & 3) == 0) mul[tile * 16 + h * 8 + (lane >> 2)] = __uint_as_float((uint32_t)(127 + 14 - e) << 23);
     }

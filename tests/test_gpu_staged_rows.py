@@ -92,7 +92,8 @@ def test_staged_linear_against_64_bits(runtime, m, k, n, wide):
 
 
 # rows of X and weights at opposite ends of the range, and both large or small: every result is in range, the factors' order decides
-@pytest.mark.parametrize("xs,ws", [(2.0 ** 116, 2.0 ** -30), (2.0 ** 120, 2.0 ** -100), (2.0 ** -110, 2.0 ** 100), (2.0 ** 60, 2.0 ** 50), (2.0 ** -60, 2.0 ** -40)])
+@pytest.mark.parametrize("xs,ws", [(2.0 ** 116, 2.0 ** -30), (2.0 ** 120, 2.0 ** -100), (2.0 ** -110, 2.0 ** 100), (2.0 ** 60, 2.0 ** 50), (2.0 ** -60, 2.0 ** -40),
+                                   (2.0 ** -100, 2.0 ** 126)])
 @pytest.mark.parametrize("m,k,n", [(5, 1024, 272), (200, 896, 304)])
 def test_staged_linear_at_the_ends_of_the_range(runtime, m, k, n, xs, ws):
     rt = runtime
