@@ -73,6 +73,7 @@ template <int BN, bool GATEUP>
 __global__ void __launch_bounds__(FKQ_THREADS, 1) k_qgemm(FkState *st, const __grid_constant__ CUtensorMap mx, QGemmArgs a) {
     using T = QgTile<BN>;
     constexpr int XS = T::XS, XG = T::XG, NBUF = T::NBUF, AS = T::AS;
+    constexpr bool SPLIT = BN <= FKQ_SPLIT_ROWS;        // tiles that are split over K
     extern __shared__ unsigned char qg_smem[];
     __shared__ __align__(8) uint64_t bars[FKQ_DEQ * FK_STAGES + 2 * XS + 2 * AS + 2 * NBUF + 2];
     __shared__ uint32_t tmem_slot;
@@ -296,7 +297,7 @@ __global__ void __launch_bounds__(FKQ_THREADS, 1) k_qgemm(FkState *st, const __g
         };
         ok = fkq_pieces(a.whole, a.tiles, nsb, me, G, [&](int v, const QWork &w) {
             const int d = v % NBUF, rt = w.tile / a.mtiles, m0 = (w.tile - rt * a.mtiles) * BN, row0 = rt * FKQ_ROWS + sub * 128 + q * 32, n = row0 + lane;
-            const bool part = fkq_part(w, nsb);
+            const bool part = SPLIT && fkq_part(w, nsb);
             const int rows = min(BN, a.m - m0);         // of X that there are
             uint32_t res[16];                           // residual pairs of 32 rows of X on their way
             auto fetch = [&](int c, auto &r) {
@@ -375,7 +376,7 @@ __global__ void __launch_bounds__(FKQ_THREADS, 1) k_qgemm(FkState *st, const __g
                         }
                     }
                 }
-            } else {
+            } else if constexpr (SPLIT) {
                 float *mine = a.scratch + (size_t)fkq_slot(a.tiles, nsb, G, me, w.tile) * fkq_part_floats(BN) + sub * 128 + q * 32 + lane;
 #pragma unroll 1
                 for (int c = 0; c < rows; c += 16) {
@@ -418,7 +419,7 @@ __global__ void __launch_bounds__(FKQ_THREADS, 1) k_qgemm(FkState *st, const __g
             __syncwarp();
             if (lane == 0) tc_arrive(dempty + 8 * d);
             return true;
-        }, [&](const QWork &w) { count(w.tile); });
+        }, [&](const QWork &w) { if constexpr (SPLIT) count(w.tile); });
         if (!ok && lane == 0) atomicOr(&st->error, FKQ_ERR_WAIT);
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");

@@ -9,6 +9,7 @@
 #endif
 #define FKQ_EPI 8                       // storing warps of a block
 #define FKQ_ROWS 256                    // weight rows of a block
+#define FKQ_SPLIT_ROWS 32               // rows of X of the widest tile that is split over K
 #define FKQ_COUNTERS 65536              // ticket words: 8 per tile that is split
 FKQ_HD inline size_t fkq_part_floats(int bn) { return (size_t)bn * FKQ_ROWS; }
 
@@ -49,8 +50,8 @@ template <typename Take, typename Skip> FKQ_HD inline bool fkq_pieces(int whole,
 }
 
 // Rows of X per tile, blocks and split of a product of m rows: the widest tile that the rows fill, a narrower one while that gives more
-// blocks a tile of their own (a step costs a block the same up to 64 rows); up to 32 rows the steps are dealt in equal runs (a part's
-// sums are small, and the product is bound by the weights), from 33 on only while less than half of the blocks have a tile.
+// blocks a tile of their own (a step costs a block the same up to 64 rows).  Tiles of up to 32 rows are dealt in equal runs of steps (a
+// part's sums are small, and the product is bound by the weights), wider ones whole.
 // Measured: 100 rows, 896 -> 1152: 11 us with tiles of 16 rows, 31 with one tile of 128 split over K (its fold passes 128 rows through memory);
 // 4864 -> 896: 19 against 63.
 struct QPlan { int bn, mtiles, tiles, grid, whole; };
@@ -60,11 +61,6 @@ inline QPlan fkq_plan(int m, int ntiles, int nsb, int sm) {
     while (p.bn > 16 && (ntiles + 15) / 16 * ((m + p.bn / 2 - 1) / (p.bn / 2)) <= sm) p.bn /= 2;
     p.mtiles = (m + p.bn - 1) / p.bn; p.tiles = (ntiles + 15) / 16 * p.mtiles; p.whole = 1; p.grid = p.tiles < sm ? p.tiles : sm;
     if (p.tiles > FKQ_COUNTERS / FKQ_EPI) return p;
-    if (p.bn <= 32) {
-        if (p.tiles % sm) { const long long steps = (long long)p.tiles * nsb; p.whole = 0; p.grid = steps < sm ? (int)steps : sm; }
-    } else if (2 * p.tiles <= sm && nsb > 1) {
-        const int parts = sm / p.tiles < nsb ? sm / p.tiles : nsb;
-        p.whole = 0; p.grid = p.tiles * parts;
-    }
+    if (p.bn <= FKQ_SPLIT_ROWS && p.tiles % sm) { const long long steps = (long long)p.tiles * nsb; p.whole = 0; p.grid = steps < sm ? (int)steps : sm; }
     return p;
 }

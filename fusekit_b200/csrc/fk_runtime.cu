@@ -139,7 +139,7 @@ extern "C" fk_status fk_open(int device, fk_handle *out) {
     c->hist_cap = FK_HIST_CAP;
     CU(cudaMalloc(&c->qmm_scratch, sizeof(float) * 2 * c->sm_count * FK_QMM_PART_FLOATS));
     CU(cudaMalloc(&c->qmm_counters, sizeof(unsigned int) * 2 * c->sm_count)); CU(cudaMemset(c->qmm_counters, 0, sizeof(unsigned int) * 2 * c->sm_count));
-    CU(cudaMalloc(&c->qg_scratch, sizeof(float) * 2 * c->sm_count * fkq_part_floats(128)));
+    CU(cudaMalloc(&c->qg_scratch, sizeof(float) * 2 * c->sm_count * fkq_part_floats(FKQ_SPLIT_ROWS)));
     CU(cudaMalloc(&c->qg_counters, sizeof(unsigned int) * FKQ_COUNTERS)); CU(cudaMemset(c->qg_counters, 0, sizeof(unsigned int) * FKQ_COUNTERS));
     CU(cudaMalloc(&c->history, sizeof(uint32_t) * c->hist_cap)); CU(cudaMemset(c->history, 0, sizeof(uint32_t) * c->hist_cap));
     CU(cudaMallocHost(&c->pinned, sizeof(uint32_t) * (c->hist_cap + 64)));

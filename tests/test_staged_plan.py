@@ -40,9 +40,34 @@ static int tickets(int m, int nt, int nsb, int sm, int share) {
     return 0;
 }
 
+// every step of every tile is dealt once; only tiles of up to FKQ_SPLIT_ROWS rows in parts, two of them a block at most, each in a slot of its own
+static int cover(int m, int nt, int nsb, int sm) {
+    const QPlan p = fkq_plan(m, nt, nsb, sm);
+    CHECK(p.bn >= 16 && p.bn <= 128 && p.grid >= 1 && p.grid <= sm && (p.whole || p.bn <= FKQ_SPLIT_ROWS));
+    CHECK(p.whole || p.tiles <= FKQ_COUNTERS / FKQ_EPI);
+    std::vector<int> next(p.tiles, 0), slot(2 * p.grid, 0), parts(p.tiles, 0);
+    for (int b = 0; b < p.grid; ++b) {
+        QWork w;
+        for (int v = 0; fkq_work(p.whole, p.tiles, nsb, b, p.grid, v, w); ++v) {
+            CHECK(w.tile >= 0 && w.tile < p.tiles && w.k0 < w.k1 && next[w.tile] == w.k0);
+            next[w.tile] = w.k1;
+            if (!fkq_part(w, nsb)) continue;
+            const int s = fkq_slot(p.tiles, nsb, p.grid, b, w.tile);
+            CHECK(!p.whole && s >= 0 && s < 2 * p.grid && slot[s]++ == 0 && fkq_owner(p.tiles, nsb, p.grid, w.tile * nsb) + parts[w.tile]++ == b);
+        }
+    }
+    for (int t = 0; t < p.tiles; ++t) CHECK(next[t] == nsb && (parts[t] == 0 || parts[t] == fkq_parts(p.tiles, nsb, p.grid, t)));
+    return 0;
+}
+
 int main(int argc, char **argv) {
     srand(7);
     const int sms[] = {132, 148, 160}, ms[] = {1, 5, 16, 17, 32, 33, 100, 1000};
+    if (argc > 1) {
+        for (int sm : sms) for (int m : ms) for (int i = 0; i < 400; ++i) if (cover(m, 1 + rand() % (i % 2 ? 2600 : 160), 1 + rand() % 64, sm)) return 1;
+        printf("ok\n");
+        return 0;
+    }
     for (int sm : sms) for (int m : ms) for (int i = 0; i < 150; ++i) {
         const int nt = 1 + rand() % 2600, nsb = 1 + rand() % 64;
         for (int share : {0, 3, 100}) if (tickets(m, nt, nsb, sm, share)) return 1;
@@ -65,4 +90,9 @@ def driver(tmp_path_factory):
 def test_ticket_words_are_zero_after_every_launch(driver):
     """Also after one in which storing warps gave up: the next product would otherwise take old parts for its own."""
     p = subprocess.run([driver], capture_output=True, text=True, timeout=300)
+    assert p.returncode == 0 and p.stdout == "ok\n", p.stdout
+
+
+def test_every_step_is_dealt_once_and_parts_are_narrow(driver):
+    p = subprocess.run([driver, "cover"], capture_output=True, text=True, timeout=300)
     assert p.returncode == 0 and p.stdout == "ok\n", p.stdout
