@@ -1,7 +1,7 @@
 // Quantised matrix product on the 5th-generation tensor cores for any number of rows: Y[M, N] = T(X[M, K] . dequant(W)^T + residual)
 // or the gated activation of gate/up pairs, 4-bit weights in the streaming layout (units of 16 rows x 8 groups, fk_stream.cuh).
 //
-// Arithmetic: one pass of kind::f16 (fp16 operands, fp32 accumulation over all of K in tensor memory), with operands that are exact.
+// Arithmetic: one pass of kind::f16 (fp16 operands, fp32 accumulation in tensor memory), with operands that are exact within these limits.
 //   * A weight is (q - 8) s + e, e = b + 8 s, after a power of two per weight row (k_row_factors: the larger of 1024 |s| and |e| lands in
 //     [2^14, 2^15)).  A nibble in the low bits of 0x6400 is 1024 + q, so one fused multiply-add gives (1024 + q) s + c; with c = -1032 s
 //     rounded towards zero to fp16, c = -1032 s + d, the result (q - 8) s + d is a multiple of s's last place below 2^11 of them, hence exact,
@@ -21,6 +21,9 @@
 //
 // Bound by the issue of the dequantising warps (538 instructions a k-block and scheduler, 72 % of its slots): 1000 rows, 3584 -> 2 x 18944, 292 us =
 // 931 TFLOP/s; 16 rows, 5120 -> 2 x 27648, 65 us = 2.45 TB/s of weights (k_qmm4 98 us; 20 -> 22 us at 5120 -> 5120, where start-up counts).
+//
+// Sums are kept in tensor memory over at most 5120 columns (fkq_stretch); longer ones are added up in the scratch area by the warp that
+// stores them.
 //
 // Work split: `whole` = tiles dealt whole in turn, else all (tile, super-block) steps dealt in equal runs; a run that covers part of a
 // tile leaves fp32 sums in the scratch area, and of the warps that hold the same rows the last to arrive adds the parts in K order.
@@ -62,6 +65,11 @@ __device__ __forceinline__ void qg_st16(uint32_t addr, const uint32_t (&r)[16]) 
                  ::"r"(addr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
                    "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
 }
+__device__ __forceinline__ void qg_put16(uint32_t addr, const uint32_t (&d)[16]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+                 ::"r"(addr), "r"(d[0]), "r"(d[1]), "r"(d[2]), "r"(d[3]), "r"(d[4]), "r"(d[5]), "r"(d[6]), "r"(d[7]),
+                   "r"(d[8]), "r"(d[9]), "r"(d[10]), "r"(d[11]), "r"(d[12]), "r"(d[13]), "r"(d[14]), "r"(d[15]) : "memory");
+}
 __device__ __forceinline__ void qg_ld16(uint32_t (&d)[16], uint32_t addr) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
                  : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]), "=r"(d[4]), "=r"(d[5]), "=r"(d[6]), "=r"(d[7]),
@@ -69,7 +77,7 @@ __device__ __forceinline__ void qg_ld16(uint32_t (&d)[16], uint32_t addr) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
-template <int BN, bool GATEUP>
+template <int BN, bool GATEUP, bool LONG>              // LONG: more than FKQ_SUM_STEPS super-blocks of columns
 __global__ void __launch_bounds__(FKQ_THREADS, 1) k_qgemm(FkState *st, const __grid_constant__ CUtensorMap mx, QGemmArgs a) {
     using T = QgTile<BN>;
     constexpr int XS = T::XS, XG = T::XG, NBUF = T::NBUF, AS = T::AS;
@@ -246,12 +254,15 @@ __global__ void __launch_bounds__(FKQ_THREADS, 1) k_qgemm(FkState *st, const __g
         int s = 0, as = 0;
         uint32_t xph = 0, aph = 0;
         bool xready = false, aready = false;
-        for (int v = 0; ok && fkq_work(a.whole, a.tiles, nsb, me, G, v, w); ++v) {
-            const int d = v % NBUF;
-            if (v >= NBUF && !tc_wait_warp(dempty + 8 * d, (uint32_t)(v / NBUF - 1) & 1u, a.limit)) { ok = false; break; }
+        int sums = 0;                                   // handed to the storing warps so far
+        for (int v = 0; ok && fkq_work(a.whole, a.tiles, nsb, me, G, v, w); ++v)
+        for (int c0 = w.k0, c1; ok && c0 < w.k1; c0 = c1, ++sums) {
+            c1 = LONG ? fkq_stretch(w, c0) : w.k1;
+            const int d = sums % NBUF;
+            if (sums >= NBUF && !tc_wait_warp(dempty + 8 * d, (uint32_t)(sums / NBUF - 1) & 1u, a.limit)) { ok = false; break; }
             const uint32_t dd = tm + (uint32_t)((d * 2 + sub) * BN);
-            uint32_t again = 0;                         // 0: the tile's first MMA overwrites
-            for (int sb = w.k0; sb < w.k1 && ok; ++sb)
+            uint32_t again = 0;                         // 0: the first MMA overwrites
+            for (int sb = c0; sb < c1 && ok; ++sb)
 #pragma unroll 1
                 for (int kk = 0, g = 0; kk < 9; ++kk) {
                     if ((g == 0 && !xready && !tc_wait_warp(xfull + 8 * s, xph, a.limit)) || (!aready && !tc_wait_warp(afull + 8 * as, aph, a.limit))) { ok = false; break; }
@@ -295,8 +306,10 @@ __global__ void __launch_bounds__(FKQ_THREADS, 1) k_qgemm(FkState *st, const __g
             }
             return __shfl_sync(0xffffffffu, ticket, 0) == most;
         };
-        ok = fkq_pieces(a.whole, a.tiles, nsb, me, G, [&](int v, const QWork &w) {
-            const int d = v % NBUF, rt = w.tile / a.mtiles, m0 = (w.tile - rt * a.mtiles) * BN, row0 = rt * FKQ_ROWS + sub * 128 + q * 32, n = row0 + lane;
+        int sums = 0;                                   // taken over so far
+        uint32_t src = 0;
+        ok = fkq_pieces(a.whole, a.tiles, nsb, me, G, [&](int, const QWork &w) {
+            const int rt = w.tile / a.mtiles, m0 = (w.tile - rt * a.mtiles) * BN, row0 = rt * FKQ_ROWS + sub * 128 + q * 32, n = row0 + lane;
             const bool part = SPLIT && fkq_part(w, nsb);
             const int rows = min(BN, a.m - m0);         // of X that there are
             uint32_t res[16];                           // residual pairs of 32 rows of X on their way
@@ -316,10 +329,52 @@ __global__ void __launch_bounds__(FKQ_THREADS, 1) k_qgemm(FkState *st, const __g
                 return f;
             };
             const float rmul = row0 + lane < a.W.ntiles * 16 ? __uint_as_float(0x7F000000u - __float_as_uint(__ldg(a.rowmul + row0 + lane))) : 0.0f;       // 2^-k of 2^k
-            if (!GATEUP && !part) fetch(0, res);        // under the tile's MMAs
-            if (!tc_wait_warp(dfull + 8 * d, (uint32_t)(v / NBUF) & 1u, a.limit)) return false;
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t src = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)((d * 2 + sub) * BN);
+            // waits for the next sums in tensor memory
+            auto next = [&]() {
+                const int d = sums % NBUF;
+                if (!tc_wait_warp(dfull + 8 * d, (uint32_t)(sums / NBUF) & 1u, a.limit)) return false;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                src = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)((d * 2 + sub) * BN);
+                return true;
+            };
+            auto taken = [&]() {                        // they are read: the MMAs may go on
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) tc_arrive(dempty + 8 * (sums % NBUF));
+                ++sums;
+            };
+            // Parts of tiles and stretches that others follow leave their sums in the scratch area, added to those of the stretches before; a tile's last
+            // stretch adds those to its own in tensor memory.  Sums that are added are requested 16 columns ahead.
+            const bool long_sum = LONG && fkq_stretch(w, w.k0) < w.k1;
+            for (int c0 = w.k0, c1;; c0 = c1) {
+                c1 = LONG ? fkq_stretch(w, c0) : w.k1;
+                const bool last = !LONG || c1 == w.k1, add = LONG && c0 > w.k0;
+                if (!GATEUP && !part && !long_sum) fetch(0, res);      // under the MMAs
+                if (!next()) return false;
+                if constexpr (SPLIT || LONG) if (part || long_sum) {
+                    float *mine = a.scratch + (size_t)(a.whole ? me : fkq_slot(a.tiles, nsb, G, me, w.tile)) * fkq_part_floats(BN) + sub * 128 + q * 32 + lane;
+                    float p[16];
+                    auto before = [&](int c) {
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) p[i] = add && c < rows ? __ldcg(mine + (size_t)(c + i) * FKQ_ROWS) : 0.0f;
+                    };
+                    before(0);
+#pragma unroll 1
+                    for (int c = 0; c < rows; c += 16) {
+                        uint32_t r[16]; qg_ld16(r, src + (uint32_t)c);
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) if (add) r[i] = __float_as_uint(__uint_as_float(r[i]) + p[i]);
+                        before(c + 16);
+                        if (last && !part) { qg_put16(src + (uint32_t)c, r); continue; }
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) __stcg(mine + (size_t)(c + i) * FKQ_ROWS, __uint_as_float(r[i]));
+                    }
+                    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                }
+                if (!GATEUP && last && !part && long_sum) fetch(0, res);
+                if (last) break;
+                taken();
+            }
             // rows c .. of X, whose factors lanes f0 .. hold; r: their residual pairs
             auto store = [&](int c, int f0, float factor, auto &acc, const uint32_t *r) {
                 constexpr int NM = sizeof(acc) / 4;
@@ -377,13 +432,6 @@ __global__ void __launch_bounds__(FKQ_THREADS, 1) k_qgemm(FkState *st, const __g
                     }
                 }
             } else if constexpr (SPLIT) {
-                float *mine = a.scratch + (size_t)fkq_slot(a.tiles, nsb, G, me, w.tile) * fkq_part_floats(BN) + sub * 128 + q * 32 + lane;
-#pragma unroll 1
-                for (int c = 0; c < rows; c += 16) {
-                    uint32_t r[16]; qg_ld16(r, src + (uint32_t)c);
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) __stcg(mine + (size_t)(c + i) * FKQ_ROWS, __uint_as_float(r[i]));
-                }
                 const int first = fkq_owner(a.tiles, nsb, G, w.tile * nsb), last = first + fkq_parts(a.tiles, nsb, G, w.tile) - 1;
                 __threadfence();
                 __syncwarp();
@@ -415,9 +463,7 @@ __global__ void __launch_bounds__(FKQ_THREADS, 1) k_qgemm(FkState *st, const __g
                     }
                 }
             }
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) tc_arrive(dempty + 8 * d);
+            taken();
             return true;
         }, [&](const QWork &w) { if constexpr (SPLIT) count(w.tile); });
         if (!ok && lane == 0) atomicOr(&st->error, FKQ_ERR_WAIT);

@@ -9,7 +9,9 @@
 #endif
 #define FKQ_EPI 8                       // storing warps of a block
 #define FKQ_ROWS 256                    // weight rows of a block
-#define FKQ_SPLIT_ROWS 32               // rows of X of the widest tile that is split over K
+#define FKQ_MOST_ROWS 128               // rows of X of the widest tile
+#define FKQ_SPLIT_ROWS 32               // .. that is split over K (two parts of a block take no more scratch than a widest tile)
+#define FKQ_SUM_STEPS 10                // super-blocks (of 512 columns) summed in one go in tensor memory
 #define FKQ_COUNTERS 65536              // ticket words: 8 per tile that is split
 FKQ_HD inline size_t fkq_part_floats(int bn) { return (size_t)bn * FKQ_ROWS; }
 
@@ -33,6 +35,14 @@ FKQ_HD inline int fkq_slot(int tiles, int nsb, int G, int b, int tile) { return 
 // rows the one that counts the last of the tile's parts adds them up and sets the ticket word to zero.
 FKQ_HD inline bool fkq_part(const QWork &w, int nsb) { return w.k0 != 0 || w.k1 != nsb; }
 FKQ_HD inline int fkq_parts(int tiles, int nsb, int G, int tile) { return fkq_owner(tiles, nsb, G, (tile + 1) * nsb - 1) - fkq_owner(tiles, nsb, G, tile * nsb) + 1; }
+// Where the sums of a piece that begin at super-block `at` end: stretches of at most FKQ_SUM_STEPS, about equally long.  The MMAs cut what an
+// accumulator cannot hold (towards zero) where an addition rounds, so a sum drifts by about 6e-10 of itself per column.  Results on the
+// wrong side of their rounding, gated activations, 3584 rows: over 18944 columns in one go 0.67 % (k_qmm4 0.34 %), in stretches 0.29 %; over
+// 5120 columns 0.22 % (0.32 %).  The storing warps add stretches in fp32, rounded, while the MMAs wait: 1000 rows, 18944 -> 3584, 149 -> 175 us.
+FKQ_HD inline int fkq_stretch(const QWork &w, int at) {
+    const int n = w.k1 - w.k0, parts = (n + FKQ_SUM_STEPS - 1) / FKQ_SUM_STEPS, each = (n + parts - 1) / parts;
+    return at + each < w.k1 ? at + each : w.k1;
+}
 // The pieces of block b in the hands of one storing warp.  take(v, w) waits for the piece and stores it (counting its ticket if it is a part); it
 // returns false, with nothing counted, when the wait runs out.  From then on nothing is taken, but skip(w) still counts the
 // ticket of every part: the ticket words are zero again after every launch, also after one that gave up.

@@ -122,6 +122,11 @@ template <typename K> static cudaError_t big_smem(K kern) {
     return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - (int)fa.sharedSizeBytes);
 }
 
+template <int BN, bool GATEUP> static cudaError_t init_qgemm() {
+    cudaError_t e = cudaFuncSetAttribute(k_qgemm<BN, GATEUP, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)QgTile<BN>::SMEM);
+    return e != cudaSuccess ? e : cudaFuncSetAttribute(k_qgemm<BN, GATEUP, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)QgTile<BN>::SMEM);
+}
+
 extern "C" const char *fk_last_error(void) { return g_err; }
 extern "C" const char *fk_version(void) { return "fusekit-b200 0.1 (sm_100a)"; }
 
@@ -139,7 +144,7 @@ extern "C" fk_status fk_open(int device, fk_handle *out) {
     c->hist_cap = FK_HIST_CAP;
     CU(cudaMalloc(&c->qmm_scratch, sizeof(float) * 2 * c->sm_count * FK_QMM_PART_FLOATS));
     CU(cudaMalloc(&c->qmm_counters, sizeof(unsigned int) * 2 * c->sm_count)); CU(cudaMemset(c->qmm_counters, 0, sizeof(unsigned int) * 2 * c->sm_count));
-    CU(cudaMalloc(&c->qg_scratch, sizeof(float) * 2 * c->sm_count * fkq_part_floats(FKQ_SPLIT_ROWS)));
+    CU(cudaMalloc(&c->qg_scratch, sizeof(float) * c->sm_count * fkq_part_floats(FKQ_MOST_ROWS)));
     CU(cudaMalloc(&c->qg_counters, sizeof(unsigned int) * FKQ_COUNTERS)); CU(cudaMemset(c->qg_counters, 0, sizeof(unsigned int) * FKQ_COUNTERS));
     CU(cudaMalloc(&c->history, sizeof(uint32_t) * c->hist_cap)); CU(cudaMemset(c->history, 0, sizeof(uint32_t) * c->hist_cap));
     CU(cudaMallocHost(&c->pinned, sizeof(uint32_t) * (c->hist_cap + 64)));
@@ -173,7 +178,7 @@ extern "C" fk_status fk_open(int device, fk_handle *out) {
     CU(big_smem(k_linear_residual<4>)); CU(big_smem(k_linear_residual<8>)); CU(big_smem(k_linear_residual<16>));
     CU(big_smem(k_rmsnorm_gateup_act<4>)); CU(big_smem(k_rmsnorm_gateup_act<8>)); CU(big_smem(k_rmsnorm_gateup_act<16>));
     CU(big_smem(k_final_head<4>)); CU(big_smem(k_final_head<8>)); CU(big_smem(k_final_head<16>));
-#define QG(BN) CU(cudaFuncSetAttribute(k_qgemm<BN, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)QgTile<BN>::SMEM)); CU(cudaFuncSetAttribute(k_qgemm<BN, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)QgTile<BN>::SMEM))
+#define QG(BN) CU((init_qgemm<BN, false>())); CU((init_qgemm<BN, true>()))
     QG(16); QG(32); QG(64); QG(128);
 #undef QG
     CU(fkl_init());
@@ -459,9 +464,12 @@ static cudaError_t launch_qmm(Ctx *c, const Weight *w, QmmArgs &qa, bool gateup)
     if (gateup) return launch(c, k_qmm4<true>, dim3(qg), dim3(FK_QMM_WARPS * 32), qmm_smem_bytes(), c->state, qa);
     return launch(c, k_qmm4<false>, dim3(qg), dim3(FK_QMM_WARPS * 32), qmm_smem_bytes(), c->state, qa);
 }
+template <int BN, bool GATEUP> static cudaError_t launch_qgemm(Ctx *c, const QPlan &p, const CUtensorMap &mx, const QGemmArgs &a) {
+    if (a.W.nsb > FKQ_SUM_STEPS) return launch(c, k_qgemm<BN, GATEUP, true>, dim3(p.grid), dim3(FKQ_THREADS), QgTile<BN>::SMEM, c->state, mx, a);
+    return launch(c, k_qgemm<BN, GATEUP, false>, dim3(p.grid), dim3(FKQ_THREADS), QgTile<BN>::SMEM, c->state, mx, a);
+}
 template <int BN> static cudaError_t launch_qgemm(Ctx *c, const QPlan &p, bool gateup, const CUtensorMap &mx, const QGemmArgs &a) {
-    if (gateup) return launch(c, k_qgemm<BN, true>, dim3(p.grid), dim3(FKQ_THREADS), QgTile<BN>::SMEM, c->state, mx, a);
-    return launch(c, k_qgemm<BN, false>, dim3(p.grid), dim3(FKQ_THREADS), QgTile<BN>::SMEM, c->state, mx, a);
+    return gateup ? launch_qgemm<BN, true>(c, p, mx, a) : launch_qgemm<BN, false>(c, p, mx, a);
 }
 // a product of staged rows (fk_qgemm.cuh): plain rows with a residual, or gate/up pairs with the activation
 static fk_status run_staged(Ctx *c, const Weight *w, bool gateup, const void *xs, const float *xscale, const uint16_t *residual, int ldr, uint16_t *y, int k, int n, int m, int act, cudaError_t *e) {

@@ -112,6 +112,29 @@ def test_staged_linear_at_the_ends_of_the_range(runtime, m, k, n, xs, ws):
         N.check(rt.L.fk_free(rt.h, p), "fk_free")
 
 
+@pytest.mark.parametrize("m,k,n", [(12, 32768, 272), (40, 18944, 512), (16, 5632, 38400), (30, 5632, 38400), (520, 10752, 4096), (1000, 12288, 3584)])
+def test_long_sums_are_added_in_stretches(runtime, m, k, n):
+    """The residual takes the leading digits away, so that the result shows the sum's last ones (to 2^-18 of it, in either direction).  Sums over all
+    columns in tensor memory lean towards zero by 5e-10 to 6e-10 of themselves per column (1.1e-5 at 18944); stretches of at most 5120 columns by
+    3e-6 at most.  Tiles of every width: in parts, whole with several a block, and the last rows of X of a tile missing."""
+    rt = runtime
+    w = _gen(f"staged.long.{k}.{n}", n, k)
+    x = _rows(m, k, k + n)
+    want = O.bf16_to_f32(x).astype(np.float64) @ _values(w).T
+    res = O.f32_to_bf16(-want.astype(np.float32))
+    wid = _weight(rt, w); rt.weight_finalize(wid)
+    xd, rd, yd = rt.to_device(x), rt.to_device(res), rt.alloc(m * n * 2)
+    staged, factor = _stage(rt, xd, m, k)
+    for _ in range(2):
+        rt.launch(T(N.TASK_STAGED_LINEAR, -1, {0: staged, 1: factor, 2: wid, 3: rd, 4: yd}, [k, n, m, 0]))
+    err = O.bf16_to_f32(rt.download(yd, (m, n), np.uint16)).astype(np.float64) - (want + O.bf16_to_f32(res).astype(np.float64))
+    assert rt.state_get()[2] == 0
+    lean, size = (err * np.sign(want)).sum() / np.abs(want).sum(), np.sqrt((err ** 2).sum() / (want ** 2).sum())
+    assert abs(lean) <= 4.5e-6 and size <= 6e-6, (m, k, n, lean, size)
+    for p in (xd, rd, yd, staged, factor):
+        N.check(rt.L.fk_free(rt.h, p), "fk_free")
+
+
 def test_staged_linear_keeps_infinities_and_nan_in_their_rows(runtime):
     rt = runtime
     m, k, n = 20, 576, 300
