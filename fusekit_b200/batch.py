@@ -216,13 +216,15 @@ class PrefillEngine(BatchDecodeEngine):
         s = self.spec
         return self.qmm == 0 and s.head_dim % 64 == 0 and s.vocab % 8 == 0 and s.hidden % 64 == 0 and s.inter % 64 == 0 and max(s.hidden, s.inter, s.n_q * s.head_dim) <= 32768
 
+    def _allocate(self):
+        """Buffers of a portion, before the first prompt that is longer than a step (some 200 MB for the 7B shape)."""
+        s, P, rt = self.spec, max(self.rows, min(self.PORTION, self.capacity)), self.rt
+        H, A, self.most = s.hidden, s.n_q * s.head_dim, (P, min(P, self.HEAD_ROWS))
+        self.scratch = {k: rt.alloc(n) for k, n in {
+            "tokens": P * 4, "greedy": P * 4, "x": P * H * 2, "hb": P * H * 2, "qkv": P * self.nqkv * 2, "q": P * A * 2, "att": P * A * 2, "act": P * s.inter * 2,
+            "staged": P * max(-(-k // 512) for k in (H, A, s.inter)) * 1152, "factor": P * 4, "logits": self.most[1] * s.vocab * 2}.items()}
+
     def capture(self) -> int:
-        if self._staged and not self.scratch and self.capacity > self.rows:
-            s, P, rt = self.spec, max(self.rows, min(self.PORTION, self.capacity)), self.rt
-            H, A, self.most = s.hidden, s.n_q * s.head_dim, (P, min(P, self.HEAD_ROWS))
-            self.scratch = {k: rt.alloc(n) for k, n in {
-                "tokens": P * 4, "greedy": P * 4, "x": P * H * 2, "hb": P * H * 2, "qkv": P * self.nqkv * 2, "q": P * A * 2, "att": P * A * 2, "act": P * s.inter * 2,
-                "staged": P * max(-(-k // 512) for k in (H, A, s.inter)) * 1152, "factor": P * 4, "logits": self.most[1] * s.vocab * 2}.items()}
         self.bound = dict(self.W), dict(self.V)     # prompts of any length name what the step's graph names,
         self.portions.clear()                       # also after other weights were loaded
         return super().capture()
@@ -261,6 +263,8 @@ class PrefillEngine(BatchDecodeEngine):
         ids = np.array(toks, np.uint32)
         if ids.max() >= self.spec.vocab:
             raise N.FusekitError(f"token id {int(ids[ids >= self.spec.vocab][0])} is outside the embedding table ({self.spec.vocab} rows)")
+        if not self.scratch:
+            self._allocate()
         most = max(M, min(self.PORTION, self.most[0]) // M * M)
         for c0 in range(0, n, most):
             part = ids[c0:c0 + most]

@@ -144,8 +144,6 @@ extern "C" fk_status fk_open(int device, fk_handle *out) {
     c->hist_cap = FK_HIST_CAP;
     CU(cudaMalloc(&c->qmm_scratch, sizeof(float) * 2 * c->sm_count * FK_QMM_PART_FLOATS));
     CU(cudaMalloc(&c->qmm_counters, sizeof(unsigned int) * 2 * c->sm_count)); CU(cudaMemset(c->qmm_counters, 0, sizeof(unsigned int) * 2 * c->sm_count));
-    CU(cudaMalloc(&c->qg_scratch, sizeof(float) * c->sm_count * fkq_part_floats(FKQ_MOST_ROWS)));
-    CU(cudaMalloc(&c->qg_counters, sizeof(unsigned int) * FKQ_COUNTERS)); CU(cudaMemset(c->qg_counters, 0, sizeof(unsigned int) * FKQ_COUNTERS));
     CU(cudaMalloc(&c->history, sizeof(uint32_t) * c->hist_cap)); CU(cudaMemset(c->history, 0, sizeof(uint32_t) * c->hist_cap));
     CU(cudaMallocHost(&c->pinned, sizeof(uint32_t) * (c->hist_cap + 64)));
     const char *e = getenv("FK_PDL"); if (e && e[0] == '0') c->pdl = false;
@@ -471,12 +469,25 @@ template <int BN, bool GATEUP> static cudaError_t launch_qgemm(Ctx *c, const QPl
 template <int BN> static cudaError_t launch_qgemm(Ctx *c, const QPlan &p, bool gateup, const CUtensorMap &mx, const QGemmArgs &a) {
     return gateup ? launch_qgemm<BN, true>(c, p, mx, a) : launch_qgemm<BN, false>(c, p, mx, a);
 }
+// Sums and tickets of staged products that are split over K or long (20 MB): allocated before the first such product, or before a graph with
+// staged products is captured.
+static fk_status staged_scratch(Ctx *c) {
+    if (c->qg_scratch) return FK_OK;
+    unsigned int *counters = nullptr; float *scratch = nullptr;
+    CU(cudaMalloc(&counters, sizeof(unsigned int) * FKQ_COUNTERS));
+    cudaError_t e = cudaMemsetAsync(counters, 0, sizeof(unsigned int) * FKQ_COUNTERS, c->stream);
+    if (e == cudaSuccess) e = cudaMalloc(&scratch, sizeof(float) * c->sm_count * fkq_part_floats(FKQ_MOST_ROWS));
+    if (e != cudaSuccess) { cudaFree(counters); CU(e); }
+    c->qg_counters = counters; c->qg_scratch = scratch;
+    return FK_OK;
+}
 // a product of staged rows (fk_qgemm.cuh): plain rows with a residual, or gate/up pairs with the activation
 static fk_status run_staged(Ctx *c, const Weight *w, bool gateup, const void *xs, const float *xscale, const uint16_t *residual, int ldr, uint16_t *y, int k, int n, int m, int act, cudaError_t *e) {
     if (!w || !w->finalized || !w->tiled || w->bits != 4 || w->rows_kind != (gateup ? FK_ROWS_GATE_UP : FK_ROWS_PLAIN)) return fail(FK_ERR_VALUE, "staged product: takes streamed 4-bit weights (plain rows, or gate/up pairs)");
     if (w->k != k || w->n != (gateup ? 2LL : 1LL) * n || m <= 0 || !xs || !xscale || !y || ((uintptr_t)xs & 15)) return fail(FK_ERR_VALUE, "staged product: shape mismatch");
     if (k > FKQ_MAX_K) return fail(FK_ERR_VALUE, "staged product: at most %d columns", FKQ_MAX_K);
     const QPlan p = fkq_plan(m, w->ntiles, w->nsb, c->sm_count);
+    if (!p.whole || w->nsb > FKQ_SUM_STEPS) { fk_status s = staged_scratch(c); if (s) return s; }
     QGemmArgs a{w->tview(), xscale, residual, y, c->qg_scratch, c->qg_counters, w->rowmul, m, n, ldr, act, p.whole, p.mtiles, p.tiles, c->wait_limit};
     CUtensorMap mx;
     if (!fkl_tensor_map(&mx, xs, m, (long long)w->nsb * FKQ_SB, (long long)w->nsb * FKQ_SB, p.bn, true)) return fail(FK_ERR_VALUE, "staged product: tensor map refused");
@@ -1023,6 +1034,8 @@ extern "C" fk_status fk_graph_capture(fk_handle h, const fk_task *tasks, int n, 
     CTX(h);
     if (!tasks || n <= 0 || !out) return fail(FK_ERR_VALUE, "empty task list");
     Graph g; g.tasks.assign(tasks, tasks + n);
+    for (int j = 0; j < n; ++j)
+        if (tasks[j].kind == FK_TASK_STAGED_LINEAR || tasks[j].kind == FK_TASK_STAGED_GATEUP) { fk_status s = staged_scratch(c); if (s) return s; }
     CU(cudaStreamSynchronize(c->stream));
     CU(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
     fk_status s = FK_OK;

@@ -231,3 +231,40 @@ def test_prompt_positions_past_the_capacity_are_reported(runtime, offset, rows):
     assert err == 0 and (got["k"].reshape(nkv, cap, hd)[:, cap - m:] != 0x3f3f).any(2).all()
     for p in [qkv, *buf.values()]:
         N.check(rt.L.fk_free(rt.h, p), "fk_free")
+
+
+def test_split_sums_are_allocated_by_the_product_or_the_graph_that_needs_them():
+    import ctypes as C
+    import torch
+    from fusekit_b200.runtime import Runtime
+
+    def free():
+        torch.cuda.synchronize()
+        return torch.cuda.mem_get_info()[0]
+
+    for graph in (False, True):
+        rt = Runtime(0)
+        try:
+            tasks, outs = [], []
+            for m, k, n in ((40, 512, 37888), (16, 4096, 304), (1000, 5632, 3584)):         # whole tiles; parts; whole tiles and long sums
+                wid, x = rt.weight_alloc(n, k, 4), rt.to_device(_rows(m, k, 3))
+                rt.weight_synth_rows(wid, 0, n, 77, 0.02, k, 0, 0); rt.weight_finalize(wid)
+                (staged, factor), y = _stage(rt, x, m, k), rt.alloc(m * n * 2)
+                tasks.append(T(N.TASK_STAGED_LINEAR, -1, {0: staged, 1: factor, 2: wid, 4: y}, [k, n, m, 0])); outs.append((y, m * n))
+            start = free()
+            if graph:
+                arr, g = (N.Task * 3)(*tasks), C.c_uint64()
+                N.check(rt.L.fk_graph_capture(rt.h, arr, 3, C.byref(g)), "fk_graph_capture")
+                assert start - free() >= 19 << 20
+                N.check(rt.L.fk_graph_launch(rt.h, g.value, None), "fk_graph_launch")
+            else:
+                rt.launch(tasks[0])
+                assert start - free() < 4 << 20
+                rt.launch(tasks[1]); rt.launch(tasks[2])
+                assert 19 << 20 <= start - free() < 26 << 20
+            got = [rt.download(p, (c,), np.uint16) for p, c in outs]
+            assert rt.state_get()[2] == 0 and all(a.any() for a in got)
+            want = got if not graph else want
+            assert all(np.array_equal(a, b) for a, b in zip(got, want))
+        finally:
+            rt.close()

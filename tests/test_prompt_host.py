@@ -99,3 +99,18 @@ def test_prompts_follow_the_weights_of_the_captured_step():
     eng.capture()
     again = weights(30)
     assert again == weights(31) and again[0] == set(eng.W.values()) and not (again[0] | again[1]) & (first[0] | first[1])
+
+
+def test_prompt_scratch_comes_with_the_first_prompt_longer_than_a_step():
+    eng = _engine(rows=8)
+    eng.decode_chunk = lambda base, seeds, count: (np.zeros((count, eng.rows), np.uint32), 0.0)
+    before = dict(eng.rt.sizes)
+    eng.prefill([1] * 8)                            # verifying drafts, say
+    assert eng.rt.sizes == before
+    eng.prefill([1] * 20)
+    scratch = dict(eng.rt.sizes)
+    assert len(scratch) > len(before)
+    eng.prefill([1] * 300)
+    eng.capture()
+    eng.prefill([1] * 20)
+    assert eng.rt.sizes == scratch
