@@ -230,26 +230,28 @@ class PrefillEngine(BatchDecodeEngine):
         return super().capture()
 
     def prompt_dispatches(self, rows: int, last: bool) -> list:
-        """One portion of a prompt, positions offset .. offset + rows - 1; with `last` the logits of its last step of `self.rows`
-        positions (counted from the prompt's start: portions before are whole steps) end up where a step leaves them."""
+        """One portion of a prompt, positions offset .. offset + rows - 1; with `last` the logits and the residual stream of its last step
+        of `self.rows` positions (counted from the prompt's start: portions before are whole steps) end up where a step leaves them."""
         s, M, H, hd, I, S, (W, V) = self.spec, rows, self.spec.hidden, self.spec.head_dim, self.spec.inter, self.scratch, self.bound
         T, A = N.Task.make, self.spec.n_q * self.spec.head_dim
 
-        def product(l, src, norm, k, weight, n, out, residual=0, one=0, at=0, m=M):
-            return [T(N.TASK_STAGE_ROWS, l, {0: src + at * k * 2, 1: norm, 2: S["staged"], 3: S["factor"]}, [k, m], [s.eps]),
-                    T(N.TASK_STAGED_LINEAR, l, {0: S["staged"], 1: S["factor"], 2: weight, 3: residual, 4: out}, [k, n, m, one])]
+        final = (M - 1) // self.rows * self.rows if last else M
 
-        tasks = [T(N.TASK_EMBED_PROMPT, -1, {0: V["embed_tokens"], 1: S["x"], 2: S["tokens"]}, [H, M, s.vocab])]
+        def product(l, src, norm, k, weight, n, out, residual=0, one=0, at=0, m=M, tail=0):
+            return [T(N.TASK_STAGE_ROWS, l, {0: src + at * k * 2, 1: norm, 2: S["staged"], 3: S["factor"]}, [k, m], [s.eps]),
+                    T(N.TASK_STAGED_LINEAR, l, {0: S["staged"], 1: S["factor"], 2: weight, 3: residual, 4: out, 5: tail if last else 0}, [k, n, m, one, final])]
+
+        tasks = [T(N.TASK_EMBED_PROMPT, -1, {0: V["embed_tokens"], 1: S["x"], 2: S["tokens"], 3: self.x_ptr(0) if last else 0}, [H, M, s.vocab, final])]
         for l in range(s.n_layers):
             (ck, cv), p = self.cache[l], f"layers.{l}."
             tasks += product(l, S["x"], V[p + "input_norm"], H, W[p + "qkv"], self.nqkv, S["qkv"], V[p + "qkv_bias_rows"], 1)
             tasks += [T(N.TASK_ROPE_STORE_PROMPT, l, {0: S["qkv"], 1: S["q"], 5: ck, 6: cv}, [s.n_q, s.n_kv, hd, self.capacity, M], [0.0, s.theta]),
                       T(N.TASK_ATTENTION_ROWS, l, {0: S["q"], 1: ck, 2: cv, 3: S["att"]}, [s.n_q, s.n_kv, hd, hd, self.capacity, M, 1 << 8], [1.0 / math.sqrt(hd)])]
-            tasks += product(l, S["att"], 0, A, W[p + "o"], H, S["hb"], S["x"])
+            tasks += product(l, S["att"], 0, A, W[p + "o"], H, S["hb"], S["x"], tail=self.hb_ptr(l))
             tasks += [T(N.TASK_STAGE_ROWS, l, {0: S["hb"], 1: V[p + "post_attention_norm"], 2: S["staged"], 3: S["factor"]}, [H, M], [s.eps]),
                       T(N.TASK_STAGED_GATEUP, l, {0: S["staged"], 1: S["factor"], 2: W[p + "gateup"], 4: S["act"]}, [H, I, M, N.ACT_SWIGLU])]
-            tasks += product(l, S["act"], 0, I, W[p + "down"], H, S["x"], S["hb"])
-        final, most = (M - 1) // self.rows * self.rows if last else M, min(self.HEAD_ROWS, self.most[1])
+            tasks += product(l, S["act"], 0, I, W[p + "down"], H, S["x"], S["hb"], tail=self.x_ptr(l + 1))
+        most = min(self.HEAD_ROWS, self.most[1])
         for r0 in list(range(0, final, most)) + ([final] if last else []):
             m = min(most, final - r0) if r0 < final else M - final
             out = S["logits"] if r0 < final else self.logits

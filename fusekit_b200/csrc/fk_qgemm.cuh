@@ -45,7 +45,7 @@ template <int BN> struct QgTile {
     static constexpr size_t SMEM = 1024 + (size_t)XS * XG * XBYTES + (size_t)FKQ_DEQ * FK_STAGES * FK_UNIT_BYTES;
 };
 
-struct QGemmArgs { TiledW W; const float *xscale; const uint16_t *residual; uint16_t *y; float *scratch; unsigned int *counters; const float *rowmul; int m, n, ldr, act, whole, mtiles, tiles; uint32_t limit; };
+struct QGemmArgs { TiledW W; const float *xscale; const uint16_t *residual; uint16_t *y; float *scratch; unsigned int *counters; const float *rowmul; int m, n, ldr, act, whole, mtiles, tiles; uint32_t limit; uint16_t *tail; int from; };      // tail: plain rows of y from `from` on once more
 
 // D += A B^T: A (128 rows, 16 halves) in tensor memory, B (the descriptor's rows) in shared memory; more = 0 overwrites D
 __device__ __forceinline__ void qg_mma(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t more) {
@@ -294,7 +294,7 @@ __global__ void __launch_bounds__(FKQ_THREADS, 1) k_qgemm(FkState *st, const __g
         const int ew = wid - FKQ_DEQ, q = ew & 3, sub = ew >> 2, odd = lane & 1;
         // plain rows in pairs: neighbouring lanes trade so that each holds two weight rows of one row of X (even lanes the even one), and
         // loads and stores are 4 bytes wide
-        const bool pairs = !GATEUP && !(a.n & 1) && !(a.ldr & 1) && !(((uintptr_t)a.y | (uintptr_t)a.residual) & 3);
+        const bool pairs = !GATEUP && !(a.n & 1) && !(a.ldr & 1) && !(((uintptr_t)a.y | (uintptr_t)a.residual | (uintptr_t)a.tail) & 3);
         // counts a part of a tile; true for the last one
         auto count = [&](int tile) {
             const unsigned int most = (unsigned int)fkq_parts(a.tiles, nsb, G, tile) - 1u;
@@ -401,13 +401,19 @@ __global__ void __launch_bounds__(FKQ_THREADS, 1) k_qgemm(FkState *st, const __g
                         const float other = __shfl_xor_sync(0xffffffffu, odd ? acc[i] : acc[i + 1], 1);
                         const float lo = (odd ? other : acc[i]) + bf_lo(r[i >> 1]), hi = (odd ? acc[i + 1] : other) + bf_hi(r[i >> 1]);
                         const int m = c + i + odd;
-                        if (m < rows && n - odd < a.n) *reinterpret_cast<uint32_t *>(a.y + (size_t)(m0 + m) * a.n + n - odd) = (uint32_t)f2bf(lo) | ((uint32_t)f2bf(hi) << 16);
+                        if (m < rows && n - odd < a.n) {
+                            const uint32_t v = (uint32_t)f2bf(lo) | ((uint32_t)f2bf(hi) << 16);
+                            *reinterpret_cast<uint32_t *>(a.y + (size_t)(m0 + m) * a.n + n - odd) = v;
+                            if (a.tail && m0 + m >= a.from) *reinterpret_cast<uint32_t *>(a.tail + (size_t)(m0 + m - a.from) * a.n + n - odd) = v;
+                        }
                     }
                 } else if (n < a.n) {
 #pragma unroll
                     for (int i = 0; i < NM; ++i) if (c + i < rows) {
                         const float add = a.residual ? bf2f(__ldcg(a.residual + (size_t)(m0 + c + i) * a.ldr + n)) : 0.0f;
-                        a.y[(size_t)(m0 + c + i) * a.n + n] = f2bf(acc[i] + add);
+                        const uint16_t v = f2bf(acc[i] + add);
+                        a.y[(size_t)(m0 + c + i) * a.n + n] = v;
+                        if (a.tail && m0 + c + i >= a.from) a.tail[(size_t)(m0 + c + i - a.from) * a.n + n] = v;
                     }
                 }
                 __syncwarp();
@@ -582,14 +588,15 @@ __global__ void __launch_bounds__(NT) k_stage_rows(const FkState *st, StageRowsA
 }
 
 // ---------------------------------------------------------------- the other kernels of a prompt
-struct EmbedPromptArgs { const uint16_t *table; uint16_t *x; const uint32_t *tokens; int h, vocab; };
+struct EmbedPromptArgs { const uint16_t *table; uint16_t *x; const uint32_t *tokens; int h, vocab; uint16_t *tail; int from; };
 __global__ void __launch_bounds__(256) k_embed_prompt(FkState *st, EmbedPromptArgs a) {        // rows of h (a multiple of 8) values
     pdl_wait(); pdl_launch_dependents();
     uint32_t tok = __ldcg(a.tokens + blockIdx.x);
     if (tok >= (uint32_t)a.vocab) { if (threadIdx.x == 0) atomicOr(&st->error, FKL_ERR_TOKEN); tok = 0; }
     const uint4 *src = reinterpret_cast<const uint4 *>(a.table + (size_t)tok * a.h);
     uint4 *dst = reinterpret_cast<uint4 *>(a.x + (size_t)blockIdx.x * a.h);
-    for (int i = threadIdx.x; i < a.h / 8; i += blockDim.x) dst[i] = __ldg(src + i);
+    uint4 *tail = a.tail && (int)blockIdx.x >= a.from ? reinterpret_cast<uint4 *>(a.tail + (size_t)(blockIdx.x - a.from) * a.h) : nullptr;
+    for (int i = threadIdx.x; i < a.h / 8; i += blockDim.x) { const uint4 v = __ldg(src + i); dst[i] = v; if (tail) tail[i] = v; }
 }
 // greedy token after every row, ties to the lowest index; eight logits per load (v a multiple of 8)
 __global__ void __launch_bounds__(512) k_argmax_prompt(const FkState *st, const uint16_t *logits, uint32_t *out, int v) {

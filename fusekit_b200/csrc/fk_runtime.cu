@@ -482,13 +482,13 @@ static fk_status staged_scratch(Ctx *c) {
     return FK_OK;
 }
 // a product of staged rows (fk_qgemm.cuh): plain rows with a residual, or gate/up pairs with the activation
-static fk_status run_staged(Ctx *c, const Weight *w, bool gateup, const void *xs, const float *xscale, const uint16_t *residual, int ldr, uint16_t *y, int k, int n, int m, int act, cudaError_t *e) {
+static fk_status run_staged(Ctx *c, const Weight *w, bool gateup, const void *xs, const float *xscale, const uint16_t *residual, int ldr, uint16_t *y, int k, int n, int m, int act, cudaError_t *e, uint16_t *tail = nullptr, int from = 0) {
     if (!w || !w->finalized || !w->tiled || w->bits != 4 || w->rows_kind != (gateup ? FK_ROWS_GATE_UP : FK_ROWS_PLAIN)) return fail(FK_ERR_VALUE, "staged product: takes streamed 4-bit weights (plain rows, or gate/up pairs)");
     if (w->k != k || w->n != (gateup ? 2LL : 1LL) * n || m <= 0 || !xs || !xscale || !y || ((uintptr_t)xs & 15)) return fail(FK_ERR_VALUE, "staged product: shape mismatch");
     if (k > FKQ_MAX_K) return fail(FK_ERR_VALUE, "staged product: at most %d columns", FKQ_MAX_K);
     const QPlan p = fkq_plan(m, w->ntiles, w->nsb, c->sm_count);
     if (!p.whole || w->nsb > FKQ_SUM_STEPS) { fk_status s = staged_scratch(c); if (s) return s; }
-    QGemmArgs a{w->tview(), xscale, residual, y, c->qg_scratch, c->qg_counters, w->rowmul, m, n, ldr, act, p.whole, p.mtiles, p.tiles, c->wait_limit};
+    QGemmArgs a{w->tview(), xscale, residual, y, c->qg_scratch, c->qg_counters, w->rowmul, m, n, ldr, act, p.whole, p.mtiles, p.tiles, c->wait_limit, tail, from};
     CUtensorMap mx;
     if (!fkl_tensor_map(&mx, xs, m, (long long)w->nsb * FKQ_SB, (long long)w->nsb * FKQ_SB, p.bn, true)) return fail(FK_ERR_VALUE, "staged product: tensor map refused");
     *e = p.bn == 16 ? launch_qgemm<16>(c, p, gateup, mx, a) : p.bn == 32 ? launch_qgemm<32>(c, p, gateup, mx, a) : p.bn == 64 ? launch_qgemm<64>(c, p, gateup, mx, a) : launch_qgemm<128>(c, p, gateup, mx, a);
@@ -897,7 +897,8 @@ static fk_status run_task(Ctx *c, const fk_task &t, const Weight *nextw = nullpt
         break;
     }
     case FK_TASK_STAGED_LINEAR: {
-        fk_status s = run_staged(c, get_w(c, b[2]), false, (const void *)b[0], (const float *)b[1], (const uint16_t *)b[3], i[3] ? 0 : i[1], (uint16_t *)b[4], i[0], i[1], i[2], 0, &e);
+        if (b[5] && i[4] < 0) return fail(FK_ERR_VALUE, "staged product: the repeated rows begin at a row");
+        fk_status s = run_staged(c, get_w(c, b[2]), false, (const void *)b[0], (const float *)b[1], (const uint16_t *)b[3], i[3] ? 0 : i[1], (uint16_t *)b[4], i[0], i[1], i[2], 0, &e, (uint16_t *)b[5], i[4]);
         if (s) return s;
         break;
     }
@@ -908,8 +909,8 @@ static fk_status run_task(Ctx *c, const fk_task &t, const Weight *nextw = nullpt
         break;
     }
     case FK_TASK_EMBED_PROMPT: {
-        if (!b[0] || !b[1] || !b[2] || i[0] <= 0 || i[0] % 8 || i[1] <= 0 || i[2] <= 0 || ((b[0] | b[1]) & 15)) return fail(FK_ERR_VALUE, "embed_prompt: bad arguments");
-        EmbedPromptArgs a{(const uint16_t *)b[0], (uint16_t *)b[1], (const uint32_t *)b[2], i[0], i[2]};
+        if (!b[0] || !b[1] || !b[2] || i[0] <= 0 || i[0] % 8 || i[1] <= 0 || i[2] <= 0 || ((b[0] | b[1] | b[3]) & 15) || (b[3] && i[3] < 0)) return fail(FK_ERR_VALUE, "embed_prompt: bad arguments");
+        EmbedPromptArgs a{(const uint16_t *)b[0], (uint16_t *)b[1], (const uint32_t *)b[2], i[0], i[2], (uint16_t *)b[3], i[3]};
         e = launch(c, k_embed_prompt, dim3(i[1]), dim3(256), 0, c->state, a);
         break;
     }

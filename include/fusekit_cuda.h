@@ -235,8 +235,10 @@ enum { FK_ACT_NONE = 0, FK_ACT_RELU_SQUARED = 2, FK_ACT_SILU = 3 };
  *                      buf3 row factors f32[M]   i0 K (a multiple of 64, at most 32768)  i1 M   f0 eps
  * STAGED_LINEAR        buf0 staged rows  buf1 row factors  buf2 weight (streamed 4-bit, plain rows)  buf3 residual T[M, N]|0  buf4 y T[M, N]
  *                      i0 K  i1 N  i2 M (any number)  i3 = 1: one residual row T[N] for all.  Row m is LINEAR_RESIDUAL's for x[m]
+ *                      buf5 T[M - i4, N]|0: the rows from i4 on once more
  * STAGED_GATEUP        buf0 staged rows  buf1 row factors  buf2 weight (fk_weight_pair)  buf4 act_out T[M, I]   i0 H  i1 I  i2 M  i3 act
- * EMBED_PROMPT         buf0 table T[V, H]  buf1 x T[M, H]  buf2 token ids u32[M] (a device buffer)   i0 H  i1 M  i2 V
+ * EMBED_PROMPT         buf0 table T[V, H]  buf1 x T[M, H]  buf2 token ids u32[M] (a device buffer)  buf3 T[M - i3, H]|0: the rows from i3 on once
+ *                      more   i0 H  i1 M  i2 V
  * ROPE_STORE_PROMPT    ROPE_STORE_ROWS for any number of consecutive positions (head_dim a multiple of 8, at most 512), without its wrap: past the
  *                      capacity nothing is stored and the error word gets 0x100000
  * ARGMAX_PROMPT        buf0 logits T[M, V]  buf1 greedy ids u32[M]   i0 V (a multiple of 8)  i1 M; the decode state is left alone

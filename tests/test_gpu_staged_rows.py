@@ -268,3 +268,44 @@ def test_split_sums_are_allocated_by_the_product_or_the_graph_that_needs_them():
             assert all(np.array_equal(a, b) for a, b in zip(got, want))
         finally:
             rt.close()
+
+
+@pytest.mark.parametrize("rows,count", [(16, 90), (4, 7), (5, 23), (16, 33)])
+def test_whole_prompts_leave_the_residual_stream_of_their_last_step(rows, count):
+    """``x_ptr`` / ``hb_ptr`` of the last step's positions, after prompts taken whole (in one portion and in several) as after steps."""
+    from fusekit_b200.batch import PrefillEngine
+    from fusekit_b200.model_spec import CONFIGS, stream_id
+    spec, got = CONFIGS["tiny-qwen"], {}
+    prompt = [O.uniform_u32(stream_id(spec.seed, "prompt"), i, spec.vocab) for i in range(count)]
+    n, L, H = (count - 1) % rows + 1, spec.n_layers, spec.hidden
+    for name, qmm, portion in (("steps", 2, 1024), ("whole", 0, 1024), ("portions", 0, 32)):
+        eng = PrefillEngine(spec, 192, rows, qmm=qmm)
+        try:
+            eng.PORTION = portion
+            eng.load_synthetic()
+            eng.prefill(prompt[:rows])                  # what an earlier step left
+            eng.prefill(prompt)
+            x = eng.rt.download(eng.x_ptr(0), (L + 1, rows, H), np.uint16)[:, :n]
+            hb = eng.rt.download(eng.hb_ptr(0), (L, rows, H), np.uint16)[:, :n]
+            got[name] = O.bf16_to_f32(np.concatenate([x, hb])).astype(np.float64)
+        finally:
+            eng.close()
+    for name in ("whole", "portions"):
+        assert np.array_equal(got[name][0], got["steps"][0])        # embedding rows
+        for a, b in zip(got[name], got["steps"]):
+            assert np.sqrt(np.mean((a - b) ** 2)) <= 8e-3 * np.sqrt(np.mean(b ** 2)), name
+
+
+@pytest.mark.parametrize("m,k,n,at", [(20, 512, 256, 16), (20, 512, 255, 3), (300, 896, 1152, 288), (40, 512, 40000, 0), (5, 4096, 304, 4)])
+def test_staged_rows_are_repeated_from_a_row_on(runtime, m, k, n, at):
+    rt = runtime
+    w = _gen(f"staged.tail.{k}.{n}", n, k)
+    wid = _weight(rt, w); rt.weight_finalize(wid)
+    xd, yd, td = rt.to_device(_rows(m, k, 5)), rt.alloc(m * n * 2), rt.alloc((m - at + 1) * n * 2)
+    N.check(rt.L.fk_memset(rt.h, td, 0x3f, (m - at + 1) * n * 2), "fk_memset")
+    staged, factor = _stage(rt, xd, m, k)
+    rt.launch(T(N.TASK_STAGED_LINEAR, -1, {0: staged, 1: factor, 2: wid, 4: yd, 5: td}, [k, n, m, 0, at]))
+    y, tail = rt.download(yd, (m, n), np.uint16), rt.download(td, (m - at + 1, n), np.uint16)
+    assert np.array_equal(tail[:-1], y[at:]) and (tail[-1] == 0x3f3f).all()
+    for p in (xd, yd, td, staged, factor):
+        N.check(rt.L.fk_free(rt.h, p), "fk_free")

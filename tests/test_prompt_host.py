@@ -79,6 +79,8 @@ def test_prompt_scratch_holds_what_the_tasks_write_whatever_the_portion_is_set_t
                    N.TASK_ARGMAX_PROMPT: (buf[1], i[1] * 4)}[kind]
             seen += 1
             assert _inside(rt, *out), (kind, i[:6])
+            if kind == N.TASK_STAGED_LINEAR and buf[5]:
+                assert 0 < i[2] - i[4] <= eng.rows and _inside(rt, buf[5], (i[2] - i[4]) * i[1] * 2)
     assert seen > 100 and s.n_layers == 2
 
 
