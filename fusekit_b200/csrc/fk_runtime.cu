@@ -944,10 +944,11 @@ static fk_status run_task(Ctx *c, const fk_task &t, const Weight *nextw = nullpt
                     (const uint16_t *)b[8], (const uint16_t *)b[9], (uint16_t *)b[3], (float *)b[4], (uint32_t *)b[5], nq, nkv, hd, cap, chunks, f[0]};
         const size_t smem = sdpa_smem_bytes(G, hd, chunks);
         if (smem > 200 * 1024) return fail(FK_ERR_VALUE, "sdpa_decode_quant: capacity too large for the merge table");
-        // a cluster per kv head, keys split over its CTAs: 16 for caches of 1024 rows and more while all are resident at once, 8 for shorter
-        // ones; more than two heads of 256 dimensions a kv head do not fit its registers (nor more than 8 heads): global partials
+        // a cluster per kv head, keys split over its CTAs: 16 for caches of 1024 rows and more while the clusters fill no more than half of the SMs
+        // (4 heads of 128, 8 bits: 9.1 us against 8.6 with 8 CTAs at 200 keys, 9.8 / 10.7 at 800, 18.4 / 29.2 at 4000; 8 such clusters are not
+        // resident at once: 16.2 / 7.9 and 33.4 / 26.7), else 8; more than two heads of 256 dimensions a kv head do not fit its registers (nor more than 8 heads): global partials
         if (c->sdpa_cluster && G <= 8 && (hd < 256 || G <= 2) && !((b[1] | b[2]) & 15)) {
-            const int cl = cap >= 1024 && nkv * FK_SDPA_CLMAX <= c->sm_count ? FK_SDPA_CLMAX : FK_SDPA_CL;
+            const int cl = cap >= 1024 && nkv * FK_SDPA_CLMAX <= c->sm_count / 2 ? FK_SDPA_CLMAX : FK_SDPA_CL;
             const dim3 cgrid(cl, nkv), cblock(FK_SDPA_CW * 32);
             const size_t csmem = sdpa_cl_smem_bytes(G, hd);
 #define SQ(B) (hd == 64 ? launch_cluster(c, k_sdpa_cluster_q<B, 64, 8>, cgrid, cblock, csmem, cl, (const FkState *)c->state, a) \
