@@ -22,7 +22,7 @@ from .model_spec import ModelSpec, stream_id, tensor_name
 from .runtime import Runtime
 
 
-STAGED_STEPS = 10                # steps of 256 x 512 weights a block from which a batch's gate/up rows go through the staged product
+STAGED_STEPS = 14                # steps of 256 x 512 weights a block from which a batch's gate/up rows go through the staged product
 
 
 class BatchDecodeEngine:
@@ -156,8 +156,10 @@ class BatchDecodeEngine:
 
     def _gate_up(self, l: int, M: int, H: int, I: int) -> list:
         """Norm, gate/up product and activation of the rows.  The staged product streams weights faster than the register-operand one (16 rows,
-        5120 -> 2 x 27648: 65 against 98 us) but starts slower: a step of the 32B shape gains 12 % (15 steps a block; 6 % with 6 rows), one of the
-        7B shape loses 5 % (7 steps), one of the 0.5B shape 12 %."""
+        5120 -> 2 x 27648: 65 against 98 us) but starts slower.  A layer's time by it and by the other, in us, 6 and 16 rows: 8192 -> 2 x 28672 (24 steps a
+        block) 205 / 224 and 227 / 268; 6144 -> 2 x 24576 (15.6) 148 / 151 and 165 / 182; the 32B shape's 5120 -> 2 x 27648 (14.6) 143 / 152 and 158 / 182;
+        8192 -> 2 x 16384 (13.8) 148 / 146 and 168 / 173; 6144 -> 2 x 18432 (11.7) 129 / 121 and 147 / 143; 5120 -> 2 x 18944 (10) 115 / 111 and
+        129 / 130; the 7B shape's (7) 94 / 89 and 105 / 104.  Between 10 and 14 steps it depends on how the other's last wave falls."""
         T, norm, w = N.Task.make, self.V[f"layers.{l}.post_attention_norm"], self.W[f"layers.{l}.gateup"]
         if self.qmm == 0 and H % 64 == 0 and H <= 32768 and -(-2 * I // 256) * -(-H // 512) >= STAGED_STEPS * self.sm:
             return [T(N.TASK_STAGE_ROWS, l, {0: self.hb_ptr(l), 1: norm, 2: self.staged, 3: self.factor}, [H, M], [self.spec.eps]),

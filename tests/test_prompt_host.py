@@ -4,9 +4,10 @@ from dataclasses import replace
 from types import SimpleNamespace
 
 import numpy as np
+import pytest
 
 from fusekit_b200 import _native as N
-from fusekit_b200.batch import PrefillEngine
+from fusekit_b200.batch import BatchDecodeEngine, PrefillEngine
 from fusekit_b200.model_spec import CONFIGS
 
 
@@ -116,3 +117,12 @@ def test_prompt_scratch_comes_with_the_first_prompt_longer_than_a_step():
     eng.capture()
     eng.prefill([1] * 20)
     assert eng.rt.sizes == scratch
+
+
+@pytest.mark.parametrize("hidden,inter,staged", [(5120, 27648, True), (6144, 24576, True), (8192, 28672, True), (8192, 16384, False), (6144, 18432, False),
+                                                 (5120, 18944, False), (3584, 18944, False), (896, 4864, False)])
+def test_batches_take_the_staged_product_only_where_it_was_faster_with_any_number_of_rows(hidden, inter, staged):
+    eng = BatchDecodeEngine(replace(CONFIGS["tiny-qwen"], n_layers=1, hidden=hidden, inter=inter), 64, 6, runtime=Books())
+    eng.load_synthetic()
+    eng.capture()
+    assert (N.TASK_STAGED_GATEUP in [t.kind for t in eng.tasks]) == staged
