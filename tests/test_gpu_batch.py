@@ -1,5 +1,7 @@
 """Batch decode of M independent sequences against M batch-1 oracle runs (the reference has no batch of sequences:
 python/fusekit_runtime/dispatch.py:2268-2289; each row is defined as what the one-row path gives for that sequence)."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -42,6 +44,28 @@ def test_batch_decode_rows_match_batch1_oracle_runs(rows, qmm):
             assert not mism and len(ties) <= 2, (m, mism, ties)
             model.close()
         assert len({tuple(allt[:, m]) for m in range(rows)}) > 1         # the sequences really differ
+    finally:
+        eng.close()
+
+
+@pytest.mark.parametrize("rows", [2, 5, 16])
+def test_batches_through_the_staged_product_match_batch1_oracle_runs(rows, monkeypatch):
+    """The gate/up form of large shapes (rows staged, product on tcgen05, captured in the step's graph), asked for on the toy."""
+    from fusekit_b200 import _native as N, batch
+    monkeypatch.setattr(batch, "STAGED_STEPS", 0)
+    spec, ctx, steps, cap = CONFIGS["tiny-qwen"], 20, 12, 64
+    eng = BatchDecodeEngine(spec, cap, rows)
+    try:
+        eng.load_synthetic(); eng.prefill_kv_synthetic(ctx)
+        seeds = np.array([3 + 7 * m for m in range(rows)], np.uint32)
+        toks, _ = eng.decode_chunk(ctx, seeds, steps)
+        kinds = [t.kind for t in eng.tasks]
+        assert kinds.count(N.TASK_STAGED_GATEUP) == spec.n_layers and N.TASK_RMSNORM_GATEUP_ACT not in kinds
+        for m in range(rows):
+            model = oracle_for_sequence(spec, cap, ctx, m)
+            mism, ties = compare_greedy(toks[:, m], model, int(seeds[m]), ctx, tie_ulps=4.0)
+            assert not mism and len(ties) <= 2, (m, mism, ties)
+            model.close()
     finally:
         eng.close()
 
@@ -106,8 +130,13 @@ def test_greedy_tokens_of_rows(runtime, vocab):
     f = O.bf16_to_f32(x)
     logits, counter, preds = rt.to_device(x), rt.to_device(np.zeros(1, np.uint32)), rt.alloc(rows * 4)
     rt.state_set(0, 7)
-    rt.launch(N.Task.make(N.TASK_ARGMAX_ROWS, -1, {0: logits, 5: counter}, [vocab, rows, 1]))
+    task = N.Task.make(N.TASK_ARGMAX_ROWS, -1, {0: logits, 5: counter}, [vocab, rows, 1])
+    rt.launch(task)
     assert rt.state_get()[:2] == (int(f[0].argmax()), 8)
+    g, got, seeds = C.c_uint64(), np.zeros((2, rows), np.uint32), np.zeros(rows, np.uint32)
+    N.check(rt.L.fk_graph_capture(rt.h, (N.Task * 1)(task), 1, C.byref(g)), "fk_graph_capture")
+    N.check(rt.L.fk_decode_chunk_rows(rt.h, g.value, 7, seeds.ctypes.data, rows, 2, got.ctypes.data, None), "fk_decode_chunk_rows")
+    assert (got == f.argmax(1)).all(), (got, f.argmax(1))
     if vocab % 8 == 0:
         rt.launch(N.Task.make(N.TASK_ARGMAX_PROMPT, -1, {0: logits, 1: preds}, [vocab, rows]))
         assert list(rt.download(preds, (rows,), np.uint32)) == list(f.argmax(1))

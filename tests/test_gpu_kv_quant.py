@@ -108,10 +108,10 @@ def test_quantised_attention_matches_the_oracle(runtime, bits, nq, nkv, hd, pos,
 @pytest.mark.gpu
 @pytest.mark.parametrize("bits", [4, 8])
 @pytest.mark.parametrize("nq,nkv,hd", [(4, 2, 64), (28, 4, 128), (40, 8, 128), (8, 4, 256), (8, 2, 256), (8, 1, 128)])
-@pytest.mark.parametrize("pos,cap", [(5, 1024), (1023, 1024), (2047, 2304), (2048, 2304), (2200, 2304)])
+@pytest.mark.parametrize("pos,cap", [(5, 1024), (1023, 1024), (2047, 2304), (2048, 2304), (2200, 2304), (1500, 1024), (5000, 2304)])
 def test_quantised_attention_over_long_caches(runtime, bits, nq, nkv, hd, pos, cap):
-    """Clusters of 16 CTAs (caches of 1024 rows and more; 8 kv heads take 8) with idle CTAs, one round of their warps and the next, a wrapped cache's whole
-    length; four heads of 256 dimensions a kv head take the kernel with global partials."""
+    """Clusters of 16 CTAs (caches of 1024 rows and more; 8 kv heads take 8) with idle CTAs, one round of their warps and the next, caches that have wrapped (the
+    newest row in the middle, left out of the early loads); four heads of 256 dimensions a kv head take the kernel with global partials."""
     test_quantised_attention_matches_the_oracle(runtime, bits, nq, nkv, hd, pos, cap)
 
 

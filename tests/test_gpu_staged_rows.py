@@ -185,7 +185,7 @@ def test_whole_prompts_match_the_steps(rows, count):
     for name, qmm, portion in (("steps", 2, 1024), ("whole", 0, 1024), ("portions", 0, 32)):
         eng = PrefillEngine(spec, cap, rows, qmm=qmm)
         try:
-            eng.PORTION = portion
+            eng.PORTION, eng.HEAD_ROWS = portion, 32    # several slices of logits
             eng.load_synthetic()
             eng.prefill(prompt[:base])
             preds = eng.prefill(prompt[base:], base)
@@ -308,4 +308,52 @@ def test_staged_rows_are_repeated_from_a_row_on(runtime, m, k, n, at):
     y, tail = rt.download(yd, (m, n), np.uint16), rt.download(td, (m - at + 1, n), np.uint16)
     assert np.array_equal(tail[:-1], y[at:]) and (tail[-1] == 0x3f3f).all()
     for p in (xd, yd, td, staged, factor):
+        N.check(rt.L.fk_free(rt.h, p), "fk_free")
+
+
+@pytest.mark.parametrize("nq,nkv,hd", [(14, 2, 64), (28, 4, 128), (8, 4, 256), (3, 3, 8), (2, 1, 512)])
+def test_prompt_positions_are_turned_and_stored(runtime, nq, nkv, hd):
+    """RoPE and the cache store of 70 positions past position 0 against the oracle, position by position: keys and queries within one bf16 step where the
+    device's sine differs from libm's in the last bit (at most 2^-7 of the pair's length), values to the bit."""
+    rt, rows, cap, at, theta = runtime, 70, 300, 131, 1e6
+    W = nq + 2 * nkv
+    qkv = _rows(rows, W * hd, hd + nq)
+    xd, sizes = rt.to_device(qkv), {"q": rows * nq * hd, "k": nkv * cap * hd, "v": nkv * cap * hd}
+    buf = {n: rt.alloc(s * 2) for n, s in sizes.items()}
+    for n, s in sizes.items():
+        N.check(rt.L.fk_memset(rt.h, buf[n], 0x3f, s * 2), "fk_memset")
+    rt.state_set(0, at)
+    rt.launch(T(N.TASK_ROPE_STORE_PROMPT, 0, {0: xd, 1: buf["q"], 5: buf["k"], 6: buf["v"]}, [nq, nkv, hd, cap, rows], [0.0, theta]))
+    assert rt.state_get()[1:] == (at, 0)
+    q = rt.download(buf["q"], (rows, nq, hd), np.uint16)
+    k, v = (rt.download(buf[n], (nkv, cap, hd), np.uint16) for n in "kv")
+    x = qkv.reshape(rows, W, hd)
+    for m in range(rows):
+        want = O.bf16_to_f32(O.rope(x[m, :nq + nkv].reshape(-1), nq + nkv, hd, at + m, theta)).reshape(nq + nkv, hd)
+        f = O.bf16_to_f32(x[m, :nq + nkv]).reshape(nq + nkv, 2, hd // 2)
+        length = np.tile(np.hypot(f[:, 0], f[:, 1]), 2)
+        got = O.bf16_to_f32(np.concatenate([q[m], k[:, at + m]]))
+        assert (np.abs(got - want) <= 2.0 ** -7 * length).all(), (m, np.abs(got - want).max())
+        assert np.array_equal(v[:, at + m], x[m, nq + nkv:])
+    outside = np.ones(cap, bool); outside[at:at + rows] = False
+    assert (k[:, outside] == 0x3f3f).all() and (v[:, outside] == 0x3f3f).all()
+    for p in [xd, *buf.values()]:
+        N.check(rt.L.fk_free(rt.h, p), "fk_free")
+
+
+@pytest.mark.parametrize("h,rows,at", [(64, 1, 0), (896, 37, 32), (5120, 200, 0)])
+def test_embedding_rows_of_a_prompt(runtime, h, rows, at):
+    rt, vocab = runtime, 50
+    table = np.random.default_rng(h).integers(0, 1 << 16, (vocab, h)).astype(np.uint16)
+    ids = np.random.default_rng(rows).integers(0, vocab, rows).astype(np.uint32)
+    td, idd, xd, sd = rt.to_device(table), rt.to_device(ids), rt.alloc(rows * h * 2), rt.alloc((rows - at) * h * 2)
+    task = T(N.TASK_EMBED_PROMPT, -1, {0: td, 1: xd, 2: idd, 3: sd}, [h, rows, vocab, at])
+    rt.state_set(0, 0)
+    rt.launch(task)
+    assert rt.state_get()[2] == 0 and np.array_equal(rt.download(xd, (rows, h), np.uint16), table[ids]) and np.array_equal(rt.download(sd, (rows - at, h), np.uint16), table[ids[at:]])
+    rt.upload(idd, np.where(np.arange(rows) == rows - 1, vocab, ids).astype(np.uint32))
+    rt.launch(task)                                     # an id outside the table: the error bit, and row 0
+    assert rt.state_get()[2] == 0x20000 and np.array_equal(rt.download(xd, (rows, h), np.uint16)[-1], table[0])
+    rt.state_set(0, 0)
+    for p in (td, idd, xd, sd):
         N.check(rt.L.fk_free(rt.h, p), "fk_free")
