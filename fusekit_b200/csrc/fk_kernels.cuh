@@ -1428,17 +1428,11 @@ __global__ void k_rope_store_rows(const FkState *st, RopeRowsArgs a) {
         dst[d] = src[d]; dst[d + half] = src[d + half];
     }
 }
-struct ArgmaxRowsArgs { const uint16_t *logits; uint32_t *counter, *history; int v, rows, advance; };
-// greedy token of every sequence from its T-rounded logits, ties to the lowest index (argmax_logits_scan.rs:83-124); the
-// block that finishes last advances the shared position.  history[step * rows + m] receives sequence m's token.
-__global__ void __launch_bounds__(1024) k_argmax_rows(FkState *st, ArgmaxRowsArgs a) {
-    __shared__ unsigned long long wbest[32];
-    pdl_wait(); pdl_launch_dependents();
-    const int m = blockIdx.x, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const uint16_t *lg = a.logits + (size_t)m * a.v;
+// A thread's share of the largest key among v logits; eight per load where `wide` (16-byte aligned, v a multiple of 8: a 2-byte load each took
+// 148 rounds for a vocabulary of 151936).
+__device__ __forceinline__ unsigned long long argmax_share(const uint16_t *lg, int v, bool wide) {
     unsigned long long best = 0ull;
-    // eight logits per load where the rows are 16-byte aligned (a 2-byte load each took 148 rounds for a vocabulary of 151936)
-    const int nv = (a.v & 7) || ((uintptr_t)a.logits & 15) ? 0 : a.v / 8;
+    const int nv = wide ? v / 8 : 0;
     for (int i = threadIdx.x; i < nv; i += blockDim.x) {
         const uint4 p = __ldcg(reinterpret_cast<const uint4 *>(lg) + i);
         const uint32_t h[4] = {p.x, p.y, p.z, p.w};
@@ -1448,7 +1442,17 @@ __global__ void __launch_bounds__(1024) k_argmax_rows(FkState *st, ArgmaxRowsArg
             best = k0 > best ? k0 : best; best = k1 > best ? k1 : best;
         }
     }
-    for (int i = nv * 8 + threadIdx.x; i < a.v; i += blockDim.x) { const unsigned long long key = argmax_key(__ldcg(lg + i), (uint32_t)i); best = key > best ? key : best; }
+    for (int i = nv * 8 + threadIdx.x; i < v; i += blockDim.x) { const unsigned long long key = argmax_key(__ldcg(lg + i), (uint32_t)i); best = key > best ? key : best; }
+    return best;
+}
+struct ArgmaxRowsArgs { const uint16_t *logits; uint32_t *counter, *history; int v, rows, advance; };
+// greedy token of every sequence from its T-rounded logits, ties to the lowest index (argmax_logits_scan.rs:83-124); the
+// block that finishes last advances the shared position.  history[step * rows + m] receives sequence m's token.
+__global__ void __launch_bounds__(1024) k_argmax_rows(FkState *st, ArgmaxRowsArgs a) {
+    __shared__ unsigned long long wbest[32];
+    pdl_wait(); pdl_launch_dependents();
+    const int m = blockIdx.x, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    unsigned long long best = argmax_share(a.logits + (size_t)m * a.v, a.v, !((a.v & 7) || ((uintptr_t)a.logits & 15)));
     best = warp_max_u64(best);
     if (lane == 0) wbest[wid] = best;
     __syncthreads();

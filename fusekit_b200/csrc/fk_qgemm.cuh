@@ -3,7 +3,8 @@
 //
 // Arithmetic: one pass of kind::f16 (fp16 operands, fp32 accumulation in tensor memory), with operands that are exact within these limits.
 //   * A weight is (q - 8) s + e, e = b + 8 s, after a power of two per weight row (k_row_factors: the larger of 1024 |s| and |e| lands in
-//     [2^14, 2^15)).  A nibble in the low bits of 0x6400 is 1024 + q, so one fused multiply-add gives (1024 + q) s + c; with c = -1032 s
+//     [2^14, 2^15)).  A nibble in the low bits of 0x6400 is 1024 + q (published: arXiv
+//     2211.10017; the upper nibble of a byte comes by 1/16), so one fused multiply-add gives (1024 + q) s + c; with c = -1032 s
 //     rounded towards zero to fp16, c = -1032 s + d, the result (q - 8) s + d is a multiple of s's last place below 2^11 of them, hence exact,
 //     and d (the same for all nibbles of a group: c + 960 s, the constant of nibbles 4 bits up, is exact too) is taken off e.
 //     Scales down to 2^-18 of the row's largest are exact, smaller ones carry an error of 2^-23 of the row's largest weight.
@@ -598,21 +599,11 @@ __global__ void __launch_bounds__(256) k_embed_prompt(FkState *st, EmbedPromptAr
     uint4 *tail = a.tail && (int)blockIdx.x >= a.from ? reinterpret_cast<uint4 *>(a.tail + (size_t)(blockIdx.x - a.from) * a.h) : nullptr;
     for (int i = threadIdx.x; i < a.h / 8; i += blockDim.x) { const uint4 v = __ldg(src + i); dst[i] = v; if (tail) tail[i] = v; }
 }
-// greedy token after every row, ties to the lowest index; eight logits per load (v a multiple of 8)
+// greedy token after every row, ties to the lowest index (v a multiple of 8)
 __global__ void __launch_bounds__(512) k_argmax_prompt(const FkState *st, const uint16_t *logits, uint32_t *out, int v) {
     __shared__ unsigned long long best_of[16];
     pdl_wait(); pdl_launch_dependents();
-    const uint4 *lg = reinterpret_cast<const uint4 *>(logits + (size_t)blockIdx.x * v);
-    unsigned long long best = 0ull;
-    for (int i = threadIdx.x; i < v / 8; i += blockDim.x) {
-        const uint4 p = __ldcg(lg + i);
-        const uint32_t h[4] = {p.x, p.y, p.z, p.w};
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const unsigned long long k0 = argmax_key((uint16_t)(h[j] & 0xffffu), (uint32_t)(i * 8 + 2 * j)), k1 = argmax_key((uint16_t)(h[j] >> 16), (uint32_t)(i * 8 + 2 * j + 1));
-            best = k0 > best ? k0 : best; best = k1 > best ? k1 : best;
-        }
-    }
+    unsigned long long best = argmax_share(logits + (size_t)blockIdx.x * v, v, true);
     best = warp_max_u64(best);
     if ((threadIdx.x & 31) == 0) best_of[threadIdx.x >> 5] = best;
     __syncthreads();
