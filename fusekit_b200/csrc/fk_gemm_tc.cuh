@@ -118,7 +118,7 @@ __global__ void __launch_bounds__(FKL_TC_THREADS, 1) k_gemm_tc(FkState *st, cons
                 const uint64_t off = (uint64_t)(s * (T::STAGE >> 4)), da = da0 + off, db = db0 + off;
                 const uint32_t bar = empty + 8 * s;
                 if (++s == S) { s = 0; ph ^= 1u; }
-                ready = tc_try_warp(full + 8 * s, ph);
+                const bool seen = tc_look(full + 8 * s, ph);
                 if (tc_elect()) {
 #pragma unroll
                     for (int k = 0; k < FKL_TC_BK / 16; ++k)
@@ -127,7 +127,7 @@ __global__ void __launch_bounds__(FKL_TC_THREADS, 1) k_gemm_tc(FkState *st, cons
                     tc_commit(bar);
                     if (kb + 1 == a.kblocks) tc_commit(afull + 8 * b);
                 }
-                __syncwarp();
+                ready = tc_all(seen);
             }
         }
         if (!tc_drain_mmas(drained)) ok = false;        // before tensor memory is freed, also where the storing warps gave up

@@ -147,7 +147,7 @@ __global__ void __launch_bounds__(FKQ_THREADS, 1) k_qgemm(FkState *st, const __g
         };
         auto claim = [&](bool free) {                   // the slot `as` may be written; a wait that runs out gives the kernel up
             announce();
-            if (!free && !tc_wait_warp(aempty + 8 * as, aph, a.limit)) ok = false;
+            if (!tc_all(free) && !tc_wait_warp(aempty + 8 * as, aph, a.limit)) ok = false;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         };
         auto taken = [&]() { pend = afull + 8 * as; if (++as == AS) { as = 0; aph ^= 1u; } };
@@ -178,7 +178,7 @@ __global__ void __launch_bounds__(FKQ_THREADS, 1) k_qgemm(FkState *st, const __g
 #pragma unroll
                     for (int h = 0; h < 2; ++h) {
                         const uint4 nx = lds128(u + (uint32_t)((2 * j + h + 1) * 512));      // after the last group: the scales, not used
-                        const bool free = tc_try_warp(aempty + 8 * as, aph);
+                        const bool free = tc_look(aempty + 8 * as, aph);
                         const uint32_t sg = __shfl_sync(0xffffffffu, sc[h], src), cg = __shfl_sync(0xffffffffu, cc[h], src);
                         const uint32_t sg8 = __shfl_sync(0xffffffffu, sc[2 + h], src), cg8 = __shfl_sync(0xffffffffu, cc[2 + h], src);
                         // nibbles 4 bits up: (1024 + 16 q) s / 16 + c + 960 s
@@ -200,7 +200,7 @@ __global__ void __launch_bounds__(FKQ_THREADS, 1) k_qgemm(FkState *st, const __g
                 if (!ok) break;
                 stages += 9;
                 {                                       // the sums' slots: columns 8b + 2t (e_hi, e_hi) and 8b + 2t + 1 (e_lo, 0) of group 2t + b
-                    const bool free = tc_try_warp(aempty + 8 * as, aph);
+                    const bool free = tc_look(aempty + 8 * as, aph);
                     uint32_t r[8];
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {       // e[i] is row g + 8 (i / 2), group 2t + (i & 1)
@@ -271,9 +271,10 @@ __global__ void __launch_bounds__(FKQ_THREADS, 1) k_qgemm(FkState *st, const __g
                     const uint64_t db = db0 + (uint64_t)((s * XG + g) * (T::XBYTES >> 4));
                     const uint32_t aa = tma + (uint32_t)(as * 64), xs_bar = xempty + 8 * s, as_bar = aempty + 8 * as;
                     const bool last = ++g == XG;
-                    if (last) { g = 0; if (++s == XS) { s = 0; xph ^= 1u; } xready = tc_try_warp(xfull + 8 * s, xph); }
+                    bool xseen = xready;
+                    if (last) { g = 0; if (++s == XS) { s = 0; xph ^= 1u; } xseen = tc_look(xfull + 8 * s, xph); }
                     if (++as == AS) { as = 0; aph ^= 1u; }
-                    aready = tc_try_warp(afull + 8 * as, aph);
+                    const bool aseen = tc_look(afull + 8 * as, aph);
                     if (tc_elect()) {
                         qg_mma(dd, aa, db, idesc, again);
                         qg_mma(dd, aa + 8, db + 2, idesc, 1u);
@@ -281,7 +282,8 @@ __global__ void __launch_bounds__(FKQ_THREADS, 1) k_qgemm(FkState *st, const __g
                         tc_commit(as_bar);
                         if (last) tc_commit(xs_bar);
                     }
-                    __syncwarp();
+                    aready = tc_all(aseen);
+                    if (last) xready = tc_all(xseen);
                     again = 1;
                 }
             if (ok && tc_elect()) tc_commit(dfull + 8 * d);

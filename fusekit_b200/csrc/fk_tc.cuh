@@ -2,7 +2,7 @@
 //
 // Every wait is bounded: TC_WAIT_LIMIT polls by default (FklEnv::wait_limit), after which the kernel sets an error bit, waits for its own
 // copies and MMAs in flight (TC_DRAIN polls at most, whatever the limit above), frees its tensor memory and returns.  A warp whose
-// lanes go on together decides together: tc_wait_warp and tc_try_warp give all 32 lanes one answer, so that no lane leaves a loop
+// lanes go on together decides together: tc_wait_warp and tc_all give all 32 lanes one answer, so that no lane leaves a loop
 // whose other lanes enter an aligned instruction or a full-mask shuffle.
 #pragma once
 #include "fk_common.cuh"
@@ -27,16 +27,18 @@ __device__ __forceinline__ bool tc_wait(uint32_t bar, uint32_t parity, uint32_t 
     for (uint32_t i = 0; i < limit; ++i) if (tc_poll(bar, parity)) return true;
     return false;
 }
-// a whole warp waits, or looks once without waiting
+// a whole warp waits
 __device__ __forceinline__ bool tc_wait_warp(uint32_t bar, uint32_t parity, uint32_t limit) {
     for (uint32_t i = 0; i < limit; ++i) if (__all_sync(0xffffffffu, tc_poll(bar, parity))) return true;
     return false;
 }
-__device__ __forceinline__ bool tc_try_warp(uint32_t bar, uint32_t parity) {
+// looks once without waiting; the warp takes the answer with a vote where it needs it (a vote right here would wait for the look)
+__device__ __forceinline__ bool tc_look(uint32_t bar, uint32_t parity) {
     uint32_t ok;
     asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-    return __all_sync(0xffffffffu, ok != 0);
+    return ok != 0;
 }
+__device__ __forceinline__ bool tc_all(bool v) { return __all_sync(0xffffffffu, v); }
 // true in one lane of a warp whose lanes are together, the same one every time
 __device__ __forceinline__ bool tc_elect() {
     uint32_t p;
