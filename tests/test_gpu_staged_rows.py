@@ -172,6 +172,28 @@ def test_staged_gateup_matches_the_one_row_kernel(runtime, m, h, inter, act):
         assert np.abs(got[i] - want).max() <= 2.0 ** -5 * max(np.abs(want).max(), rms) and np.sqrt(np.mean((got[i] - want) ** 2)) <= 4e-3 * rms, (m, h, inter, act, i)
 
 
+@pytest.mark.parametrize("m,h,inter", [(2, 896, 4864), (16, 5120, 2000), (33, 512, 137), (130, 1088, 512), (20, 5632, 520)])
+def test_staged_gateup_against_64_bits(runtime, m, h, inter):
+    """silu(gate) up in 64 bits: gate and up are rounded to bf16 (2^-8 of each, 2^-19 of the sum of magnitudes before that), silu's slope is at most
+    1.1, and the result is rounded once more."""
+    rt = runtime
+    g, u = _gen(f"staged.g{h}.{inter}", inter, h), _gen(f"staged.u{h}.{inter}", inter, h)
+    pair = rt.weight_pair(_weight(rt, g), _weight(rt, u))
+    x = _rows(m, h, m * h)
+    xd, yd = rt.to_device(x), rt.alloc(m * inter * 2)
+    staged, factor = _stage(rt, xd, m, h)
+    rt.launch(T(N.TASK_STAGED_GATEUP, -1, {0: staged, 1: factor, 2: pair, 4: yd}, [h, inter, m, N.ACT_SWIGLU]))
+    got = O.bf16_to_f32(rt.download(yd, (m, inter), np.uint16)).astype(np.float64)
+    X, G, U = O.bf16_to_f32(x).astype(np.float64), _values(g), _values(u)
+    gate, up = X @ G.T, X @ U.T
+    silu = gate / (1 + np.exp(-gate))
+    dg, du = (2.0 ** -8 * np.abs(v) + 2.0 ** -19 * (np.abs(X) @ np.abs(W).T) for v, W in ((gate, G), (up, U)))
+    bound = 1.02 * (1.1 * dg * (np.abs(up) + du) + np.abs(silu) * du + 2.0 ** -8 * np.abs(silu * up))
+    assert (np.abs(got - silu * up) <= bound).all(), np.max(np.abs(got - silu * up) / bound)
+    for p in (xd, yd, staged, factor):
+        N.check(rt.L.fk_free(rt.h, p), "fk_free")
+
+
 @pytest.mark.parametrize("rows,count", [(16, 17), (16, 90), (4, 5), (4, 7), (5, 23), (16, 150)])
 def test_whole_prompts_match_the_steps(rows, count):
     """A prompt through the kernels of whole prompts against the same engine stepping it (the mma.sync kernels asked for by name): caches
