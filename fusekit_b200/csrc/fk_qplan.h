@@ -38,7 +38,7 @@ FKQ_HD inline int fkq_parts(int tiles, int nsb, int G, int tile) { return fkq_ow
 // Where the sums of a piece that begin at super-block `at` end: stretches of at most FKQ_SUM_STEPS, about equally long.  The MMAs cut what an
 // accumulator cannot hold (towards zero) where an addition rounds, so a sum drifts by about 6e-10 of itself per column.  Results on the
 // wrong side of their rounding, gated activations, 3584 rows: over 18944 columns in one go 0.67 % (k_qmm4 0.34 %), in stretches 0.29 %; over
-// 5120 columns 0.22 % (0.32 %).  The storing warps add stretches in fp32, rounded, while the MMAs wait: 1000 rows, 18944 -> 3584, 152 -> 166 us.
+// 5120 columns 0.22 % (0.32 %).  The storing warps add stretches in fp32, rounded, while the MMAs wait: 1000 rows, 18944 -> 3584, 152 -> 157 us.
 FKQ_HD inline int fkq_stretch(const QWork &w, int at) {
     const int n = w.k1 - w.k0, parts = (n + FKQ_SUM_STEPS - 1) / FKQ_SUM_STEPS, each = (n + parts - 1) / parts;
     return at + each < w.k1 ? at + each : w.k1;
