@@ -19,75 +19,6 @@ template <int BN> struct TcTile {
 };
 struct TcGemmArgs { void *y; const int *offsets; int m, n, kblocks, row0, ldy, act, out_f32, experts; float scale; BlockCols b; uint32_t limit; };       // b: BLOCK form
 
-// A warp stores 32 rows (lane = row) of a finished accumulator of BN columns: `src` its lanes' part of tensor memory, rows from mend on are not stored.
-template <int BN, bool BLOCK> __device__ __forceinline__ void tc_store_row(const TcGemmArgs &a, uint32_t src, int row, int mend, int n0) {
-#pragma unroll 1
-    for (int c = 0; c < BN; c += 32) {
-        __syncwarp();
-        uint32_t d[32];
-        asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-                     : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]), "=r"(d[4]), "=r"(d[5]), "=r"(d[6]), "=r"(d[7]), "=r"(d[8]), "=r"(d[9]), "=r"(d[10]),
-                       "=r"(d[11]), "=r"(d[12]), "=r"(d[13]), "=r"(d[14]), "=r"(d[15]), "=r"(d[16]), "=r"(d[17]), "=r"(d[18]), "=r"(d[19]), "=r"(d[20]), "=r"(d[21]),
-                       "=r"(d[22]), "=r"(d[23]), "=r"(d[24]), "=r"(d[25]), "=r"(d[26]), "=r"(d[27]), "=r"(d[28]), "=r"(d[29]), "=r"(d[30]), "=r"(d[31])
-                     : "r"(src + (uint32_t)c));
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        const int col = n0 + c;
-        if (row >= mend || col >= a.n) continue;
-        if (BLOCK && col >= a.b.exact) {            // 16 (gate, up) pairs
-            uint16_t *y = (uint16_t *)a.b.y3 + (size_t)row * a.b.ld3 + (col - a.b.exact) / 2;
-            float v[16];
-#pragma unroll
-            for (int i = 0; i < 16; ++i) v[i] = clamped_glu(__uint_as_float(d[2 * i]), __uint_as_float(d[2 * i + 1]), a.b.limit);
-            if (col + 32 <= a.n) {
-#pragma unroll
-                for (int i = 0; i < 4; ++i) st4(y + 4 * i, make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]));
-            } else {
-#pragma unroll
-                for (int i = 0; i < 16; ++i) if (col + 2 * i < a.n) y[i] = f2bf(v[i]);
-            }
-            continue;
-        }
-        if (BLOCK) {
-            if (col < a.b.silu) {
-#pragma unroll
-                for (int i = 0; i < 32; ++i) if (col + i < a.b.silu) d[i] = __float_as_uint(act_apply(__uint_as_float(d[i]), FKL_ACT_SILU));
-            }
-        } else {
-#pragma unroll
-            for (int i = 0; i < 32; ++i) d[i] = __float_as_uint(act_apply(__uint_as_float(d[i]), a.act) * a.scale);
-        }
-        const bool whole = col + 32 <= a.n, exact = BLOCK && col >= a.b.plain;
-        if (a.out_f32 || exact) {
-            const int ld = exact ? a.b.exact - a.b.plain : a.ldy;
-            float *y = exact ? a.b.y2 + (size_t)row * ld + col - a.b.plain : (float *)a.y + (size_t)row * ld + col;
-            if (whole && (ld & 3) == 0) {
-#pragma unroll
-                for (int i = 0; i < 8; ++i) reinterpret_cast<uint4 *>(y)[i] = make_uint4(d[4 * i], d[4 * i + 1], d[4 * i + 2], d[4 * i + 3]);
-            } else {
-#pragma unroll
-                for (int i = 0; i < 32; ++i) if (col + i < a.n) y[i] = __uint_as_float(d[i]);
-            }
-        } else {
-            uint16_t *y = (uint16_t *)a.y + (size_t)row * a.ldy + col;
-            if (whole && (a.ldy & 7) == 0) {
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    uint32_t w[4];
-#pragma unroll
-                    for (int p = 0; p < 4; ++p) {
-                        const __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(d[8 * i + 2 * p]), __uint_as_float(d[8 * i + 2 * p + 1]));
-                        w[p] = *reinterpret_cast<const uint32_t *>(&h);
-                    }
-                    reinterpret_cast<uint4 *>(y)[i] = make_uint4(w[0], w[1], w[2], w[3]);
-                }
-            } else {
-#pragma unroll
-                for (int i = 0; i < 32; ++i) if (col + i < a.n) y[i] = f2bf(__uint_as_float(d[i]));
-            }
-        }
-    }
-}
-
 template <int BN, bool BLOCK>
 __global__ void __launch_bounds__(FKL_TC_THREADS, 1) k_gemm_tc(FkState *st, const __grid_constant__ CUtensorMap mx, const __grid_constant__ CUtensorMap mw, TcGemmArgs a) {
     using T = TcTile<BN>;
@@ -209,7 +140,71 @@ __global__ void __launch_bounds__(FKL_TC_THREADS, 1) k_gemm_tc(FkState *st, cons
             const int b = j & 1, row = m0 + q * 32 + lane;
             if (!tc_wait_warp(afull + 8 * b, (uint32_t)(j / 2) & 1u, a.limit)) { ok = false; break; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            tc_store_row<BN, BLOCK>(a, tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * BN), row, mend, n0);
+#pragma unroll 1
+            for (int c = 0; c < BN; c += 32) {
+                __syncwarp();
+                uint32_t d[32];
+                asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+                             : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]), "=r"(d[4]), "=r"(d[5]), "=r"(d[6]), "=r"(d[7]), "=r"(d[8]), "=r"(d[9]), "=r"(d[10]),
+                               "=r"(d[11]), "=r"(d[12]), "=r"(d[13]), "=r"(d[14]), "=r"(d[15]), "=r"(d[16]), "=r"(d[17]), "=r"(d[18]), "=r"(d[19]), "=r"(d[20]), "=r"(d[21]),
+                               "=r"(d[22]), "=r"(d[23]), "=r"(d[24]), "=r"(d[25]), "=r"(d[26]), "=r"(d[27]), "=r"(d[28]), "=r"(d[29]), "=r"(d[30]), "=r"(d[31])
+                             : "r"(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * BN + c)));
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                const int col = n0 + c;
+                if (row >= mend || col >= a.n) continue;
+                if (BLOCK && col >= a.b.exact) {            // 16 (gate, up) pairs
+                    uint16_t *y = (uint16_t *)a.b.y3 + (size_t)row * a.b.ld3 + (col - a.b.exact) / 2;
+                    float v[16];
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) v[i] = clamped_glu(__uint_as_float(d[2 * i]), __uint_as_float(d[2 * i + 1]), a.b.limit);
+                    if (col + 32 <= a.n) {
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) st4(y + 4 * i, make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]));
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) if (col + 2 * i < a.n) y[i] = f2bf(v[i]);
+                    }
+                    continue;
+                }
+                if (BLOCK) {
+                    if (col < a.b.silu) {
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) if (col + i < a.b.silu) d[i] = __float_as_uint(act_apply(__uint_as_float(d[i]), FKL_ACT_SILU));
+                    }
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) d[i] = __float_as_uint(act_apply(__uint_as_float(d[i]), a.act) * a.scale);
+                }
+                const bool whole = col + 32 <= a.n, exact = BLOCK && col >= a.b.plain;
+                if (a.out_f32 || exact) {
+                    const int ld = exact ? a.b.exact - a.b.plain : a.ldy;
+                    float *y = exact ? a.b.y2 + (size_t)row * ld + col - a.b.plain : (float *)a.y + (size_t)row * ld + col;
+                    if (whole && (ld & 3) == 0) {
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) reinterpret_cast<uint4 *>(y)[i] = make_uint4(d[4 * i], d[4 * i + 1], d[4 * i + 2], d[4 * i + 3]);
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) if (col + i < a.n) y[i] = __uint_as_float(d[i]);
+                    }
+                } else {
+                    uint16_t *y = (uint16_t *)a.y + (size_t)row * a.ldy + col;
+                    if (whole && (a.ldy & 7) == 0) {
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            uint32_t w[4];
+#pragma unroll
+                            for (int p = 0; p < 4; ++p) {
+                                const __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(d[8 * i + 2 * p]), __uint_as_float(d[8 * i + 2 * p + 1]));
+                                w[p] = *reinterpret_cast<const uint32_t *>(&h);
+                            }
+                            reinterpret_cast<uint4 *>(y)[i] = make_uint4(w[0], w[1], w[2], w[3]);
+                        }
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) if (col + i < a.n) y[i] = f2bf(__uint_as_float(d[i]));
+                    }
+                }
+            }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) tc_arrive(aempty + 8 * b);
@@ -220,123 +215,4 @@ __global__ void __launch_bounds__(FKL_TC_THREADS, 1) k_gemm_tc(FkState *st, cons
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     if (wid == 2) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)T::COLS) : "memory");
-}
-
-// ---------------------------------------------------------------- two SMs on one tile
-// The same product for many rows, not grouped: the two blocks of a cluster share a tile of 256 rows of X by 256 rows of W (cta_group::2).  Each holds its
-// 128 rows of X and half of the rows of W, so a slice of 64 costs an SM 32 KB of loads where a 128 x 256 tile of its own costs 48, and every
-// operand row crosses shared memory for twice as many products: the single-SM form stops at 1.1 PFLOP/s on that traffic.  Both blocks'
-// loads count on the first block's barrier; its MMA warp issues for both, and commits free the stages (announce the accumulators) in both.
-// Accumulators: 128 rows x 256 columns in each block's tensor memory, two of them.
-#define FKL_TC2_STAGES 6
-#define FKL_TC2_STAGE (2 * 128 * FKL_TC_BK * 2)
-#define FKL_TC2_SMEM ((size_t)FKL_TC2_STAGES * FKL_TC2_STAGE + 1024)
-template <bool BLOCK>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(FKL_TC_THREADS, 1) k_gemm_pair(FkState *st, const __grid_constant__ CUtensorMap mx, const __grid_constant__ CUtensorMap mw, TcGemmArgs a) {
-    constexpr int S = FKL_TC2_STAGES, STAGE = FKL_TC2_STAGE;
-    extern __shared__ unsigned char smem_raw[];
-    __shared__ __align__(8) uint64_t bars[2 * S + 5];
-    __shared__ uint32_t tmem_slot;
-    const int tid = threadIdx.x, lane = tid & 31, wid = __shfl_sync(0xffffffffu, tid >> 5, 0);
-    uint32_t rank; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
-    const uint32_t base = (tc_smem(smem_raw) + 1023u) & ~1023u;
-    const uint32_t full = tc_smem(bars), empty = full + 8 * S, afull = empty + 8 * S, aempty = afull + 16, drained = aempty + 16;       // full, aempty: the first block's count
-    if (tid == 0) {
-        for (int s = 0; s < S; ++s) { tc_init(full + 8 * s, 1); tc_init(empty + 8 * s, 1); }
-        for (int s = 0; s < 2; ++s) { tc_init(afull + 8 * s, 1); tc_init(aempty + 8 * s, 8); }
-        tc_init(drained, 1);
-        tc_init_fence();
-    }
-    if (wid == 2) {
-        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc_smem(&tmem_slot)), "r"(512u) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    tc_cluster_sync();                  // both blocks' barriers are up, their tensor memory is allocated
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    pdl_launch_dependents();
-    pdl_wait();
-    const uint32_t tmem = tmem_slot;
-    const int mtiles = (a.m + 255) / 256, total = mtiles * ((a.n + 255) / 256), pair = (int)blockIdx.x >> 1, pairs = (int)gridDim.x >> 1;
-    auto place = [&](int t, int &m0, int &n0) { const int nt = t / mtiles; m0 = (t - nt * mtiles) * 256 + (int)rank * 128; n0 = nt * 256; };
-    bool ok = true;
-    if (wid == 0) {
-        if (lane == 0) {
-            const uint32_t counted = tc_remote(full, 0);
-            int it = 0;
-            for (int t = pair; t < total && ok; t += pairs) {
-                int m0, n0; place(t, m0, n0);
-                for (int kb = 0; kb < a.kblocks; ++kb, ++it) {
-                    const int s = it % S;
-                    if (it >= S && !tc_wait(empty + 8 * s, (uint32_t)(it / S - 1) & 1u, a.limit)) { ok = false; break; }
-                    if (rank == 0) tc_expect(full + 8 * s, 2u * STAGE);
-                    tc_load_pair(base + s * STAGE, &mx, kb * FKL_TC_BK, m0, counted + 8 * s);
-                    tc_load_pair(base + s * STAGE + STAGE / 2, &mw, kb * FKL_TC_BK, a.row0 + n0 + (int)rank * 128, counted + 8 * s);
-                }
-            }
-            // the last stages have landed and, unless a wait ran out, are multiplied before the block may leave (what this block's loads filled, the
-            // first block's barrier says, and both blocks leave together)
-            for (int j = it > S ? it - S : 0; j < it; ++j) {
-                if (rank == 0 && !tc_wait(full + 8 * (j % S), (uint32_t)(j / S) & 1u, TC_DRAIN)) ok = false;
-                if (ok && !tc_wait(empty + 8 * (j % S), (uint32_t)(j / S) & 1u, a.limit)) ok = false;
-            }
-            if (!ok) atomicOr(&st->error, FKL_ERR_TC_WAIT);
-        }
-    } else if (wid == 1) {
-        if (rank == 0) {
-            const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((256u >> 3) << 17) | ((256u >> 4) << 24);
-            const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
-            const uint64_t da0 = tc_desc(base), db0 = tc_desc(base + STAGE / 2);
-            int s = 0, j = 0;
-            uint32_t ph = 0;
-            bool ready = false;
-            for (int t = pair; t < total && ok; t += pairs, ++j) {
-                const int b = j & 1;
-                if (j >= 2 && !tc_wait_warp_cluster(aempty + 8 * b, (uint32_t)(j / 2 - 1) & 1u, a.limit)) { ok = false; break; }
-                const uint32_t d = tm + (uint32_t)(b * 256);
-                for (int kb = 0; kb < a.kblocks; ++kb) {
-                    if (!ready && !tc_wait_warp_cluster(full + 8 * s, ph, a.limit)) { ok = false; break; }
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint64_t off = (uint64_t)(s * (STAGE >> 4)), da = da0 + off, db = db0 + off;
-                    const uint32_t bar = empty + 8 * s;
-                    if (++s == S) { s = 0; ph ^= 1u; }
-                    const bool seen = tc_poll_cluster_look(full + 8 * s, ph);
-                    if (tc_elect()) {
-#pragma unroll
-                        for (int k = 0; k < FKL_TC_BK / 16; ++k)
-                            asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-                                         ::"r"(d), "l"(da + (uint64_t)(k * 2)), "l"(db + (uint64_t)(k * 2)), "r"(idesc), "r"(kb | k) : "memory");
-                        tc_commit_pair(bar);
-                        if (kb + 1 == a.kblocks) tc_commit_pair(afull + 8 * b);
-                    }
-                    ready = tc_all(seen);
-                }
-            }
-            if (tc_elect()) asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(drained) : "memory");
-            __syncwarp();
-            if (!tc_wait_warp(drained, 0u, TC_DRAIN)) ok = false;      // before tensor memory is freed, also where the storing warps gave up
-            if (!ok && lane == 0) atomicOr(&st->error, FKL_ERR_TC_WAIT);
-        }
-    } else if (wid >= 4) {
-        const int q = wid - 4;
-        const uint32_t freed = tc_remote(aempty, 0);
-        int j = 0;
-        for (int t = pair; t < total && ok; t += pairs, ++j) {
-            int m0, n0; place(t, m0, n0);
-            const int b = j & 1, row = m0 + q * 32 + lane;
-            if (!tc_wait_warp_cluster(afull + 8 * b, (uint32_t)(j / 2) & 1u, a.limit)) { ok = false; break; }
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            tc_store_row<256, BLOCK>(a, tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * 256), row, a.m, n0);
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) tc_arrive_remote(freed + 8 * b);
-        }
-        if (!ok && lane == 0) atomicOr(&st->error, FKL_ERR_TC_WAIT);
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    tc_cluster_sync();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (wid == 2) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
 }

@@ -31,7 +31,6 @@ cudaError_t fkl_init() {
     TRY(cudaFuncSetAttribute(k_gemm_tc<64, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TcTile<64>::SMEM)); TRY(cudaFuncSetAttribute(k_gemm_tc<64, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TcTile<64>::SMEM));
     TRY(cudaFuncSetAttribute(k_gemm_tc<128, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TcTile<128>::SMEM)); TRY(cudaFuncSetAttribute(k_gemm_tc<128, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TcTile<128>::SMEM));
     TRY(cudaFuncSetAttribute(k_gemm_tc<256, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TcTile<256>::SMEM)); TRY(cudaFuncSetAttribute(k_gemm_tc<256, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TcTile<256>::SMEM));
-    TRY(cudaFuncSetAttribute(k_gemm_pair<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FKL_TC2_SMEM)); TRY(cudaFuncSetAttribute(k_gemm_pair<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FKL_TC2_SMEM));
 #define FL(KD, W) TRY(big_smem(k_flash_rows<KD, 64, W>)); TRY(big_smem(k_flash_rows<KD, 128, W>)); TRY(big_smem(k_flash_rows<KD, 256, W>))
     FL(32, false); FL(64, false); FL(128, false); FL(32, true); FL(64, true); FL(128, true);
 #undef FL
@@ -189,15 +188,6 @@ fk_status fkl_run(FklEnv &c, const fk_task &t, char *err, size_t ecap) {
             const long long tiles = mt * ((N + bn - 1) / bn);
             const int grid = tiles < c.sm_count ? (int)tiles : c.sm_count;
             CUtensorMap mx, mw;
-            // Two SMs a tile where that needs no more rounds of tiles (a pair's round takes 0.9 of a single's, so a last round it adds does not
-            // pay): 1500 rows of kakunex-5120 7.83 ms a prompt for 8.44, 300 rows of kakunex-3584, five rounds for four, 3.21 for 3.15.
-            const long long pt = (long long)((M + 255) / 256) * ((N + 255) / 256), pairs = c.sm_count / 2;
-            if (bn == 256 && !groups && M > 128 && (pt + pairs - 1) / pairs <= (tiles + c.sm_count - 1) / c.sm_count) {
-                const int pg = pt * 2 < c.sm_count ? (int)pt * 2 : c.sm_count / 2 * 2;
-                if (!fkl_tensor_map(&mx, (const void *)b[0], M, w.k, ldx, 128) || !fkl_tensor_map(&mw, w.rows, w.n, w.k, w.k, 128)) return bad(err, ecap, "linear_rows: tensor map refused");
-                e = block ? launch(c, k_gemm_pair<true>, dim3(pg), dim3(FKL_TC_THREADS), FKL_TC2_SMEM, c.state, mx, mw, a) : launch(c, k_gemm_pair<false>, dim3(pg), dim3(FKL_TC_THREADS), FKL_TC2_SMEM, c.state, mx, mw, a);
-                break;
-            }
             if (!fkl_tensor_map(&mx, (const void *)b[0], M, w.k, ldx, 128) || !fkl_tensor_map(&mw, w.rows, w.n, w.k, w.k, bn)) return bad(err, ecap, "linear_rows: tensor map refused");
             if (block) e = bn == 256 ? launch_tc<256, true>(c, grid, mx, mw, a) : bn == 128 ? launch_tc<128, true>(c, grid, mx, mw, a) : launch_tc<64, true>(c, grid, mx, mw, a);
             else e = bn == 256 ? launch_tc<256, false>(c, grid, mx, mw, a) : bn == 128 ? launch_tc<128, false>(c, grid, mx, mw, a) : launch_tc<64, false>(c, grid, mx, mw, a);

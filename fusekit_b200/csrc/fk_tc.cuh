@@ -62,27 +62,3 @@ __device__ __forceinline__ uint64_t tc_desc(uint32_t addr) {
 // an address of this block's shared memory in block `rank` of the cluster; a barrier of all threads of the cluster's blocks
 __device__ __forceinline__ uint32_t tc_remote(uint32_t addr, uint32_t rank) { uint32_t r; asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank)); return r; }
 __device__ __forceinline__ void tc_cluster_sync() { asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory"); }
-// two blocks on one tile (cta_group::2)
-__device__ __forceinline__ void tc_arrive_remote(uint32_t bar) { asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory"); }
-__device__ __forceinline__ void tc_commit_pair(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((uint16_t)3) : "memory");
-}
-// this block's tile, counted on a barrier of the pair's first block
-__device__ __forceinline__ void tc_load_pair(uint32_t dst, const CUtensorMap *map, int k, int row, uint32_t bar) {
-    asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-                 ::"r"(dst), "l"(map), "r"(k), "r"(row), "r"(bar) : "memory");
-}
-__device__ __forceinline__ bool tc_poll_cluster(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-    return ok != 0;
-}
-__device__ __forceinline__ bool tc_poll_cluster_look(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-    return ok != 0;
-}
-__device__ __forceinline__ bool tc_wait_warp_cluster(uint32_t bar, uint32_t parity, uint32_t limit) {
-    for (uint32_t i = 0; i < limit; ++i) if (__all_sync(0xffffffffu, tc_poll_cluster(bar, parity))) return true;
-    return false;
-}
