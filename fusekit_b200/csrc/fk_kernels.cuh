@@ -9,6 +9,7 @@
 // position and prefetch old cache rows ahead of their own wait.
 #pragma once
 #include "fk_common.cuh"
+#include "fk_sdpa_layout.h"
 #include <cooperative_groups.h>
 namespace cg = cooperative_groups;
 
@@ -641,8 +642,6 @@ __global__ void __launch_bounds__(FK_SDPA_THREADS) k_sdpa_decode_q(const FkState
 
 // ---------------------------------------------------------------- cluster SDPA
 #define FK_SDPA_CL 8            // CTAs per kv head (portable cluster size); they split the keys
-#define FK_SDPA_CLMAX 16        // the tensor-core kernel also runs as a cluster of 16 (non-portable size) when few kv heads leave SMs idle
-#define FK_SDPA_CW 16           // warps per CTA
 #define FK_SDPA_KPW 8           // keys per warp iteration (4 lanes per key)
 __host__ __device__ inline size_t sdpa_cl_smem_bytes(int G, int hd) {
     return sizeof(float) * (size_t)(G * (hd + 16) + FK_SDPA_CW * G * (hd + 2) + G * (hd + 2) + FK_SDPA_CW * G + G + 16);
@@ -833,24 +832,11 @@ __global__ void __launch_bounds__(FK_SDPA_CW * 32) k_sdpa_cluster(const FkState 
 //                                  exactly the layout S came out in; p is split into two bf16 terms (hi + lo), so the
 //                                  products carry 16 significant bits of p (sdpa_decode.rs:697-715 accumulates p*v in fp32)
 // A lane then handles one head instead of looping over the group: ~150 instructions per 16 keys instead of ~2200.
-#define FK_SDPA_MK 16
 __device__ __forceinline__ void mma_bf16_f32(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) { return (uint32_t)f2bf(lo) | ((uint32_t)f2bf(hi) << 16); }
-template <int HD, int CW = FK_SDPA_CW> struct SdpaMmaLayout {
-    static constexpr int QSTRIDE = HD * 2 + 16;                  // bytes per q row (bf16)
-    static constexpr int VSTRIDE = HD * 2 + 16;                  // bytes per V tile row: ldmatrix rows hit distinct banks
-    static constexpr int WTILE = FK_SDPA_MK * VSTRIDE;           // bytes of a warp's V tile; later its [G][HD+2] fp32 partial
-    __host__ __device__ static constexpr int q() { return 0; }
-    __host__ __device__ static constexpr int tiles() { return 8 * QSTRIDE; }
-    __host__ __device__ static constexpr int cpart() { return tiles() + CW * WTILE; }
-    __host__ __device__ static constexpr int wexp(int G) { return cpart() + (G * HD + FK_SDPA_CLMAX) * 4; }      // after the received o slices
-    __host__ __device__ static constexpr int fexp(int G) { return wexp(G) + FK_SDPA_CLMAX * G * 2 * 4; }              // [16][G] factors + [G] maxima + [G] 1 / l
-    __host__ __device__ static constexpr int bytes(int G) { return fexp(G) + (16 * G + 2 * G) * 4 + 64; }
-};
-template <int CW> __host__ __device__ inline size_t sdpa_mma_smem_bytes(int G, int hd) { return hd == 256 ? SdpaMmaLayout<256, CW>::bytes(G) : hd == 128 ? SdpaMmaLayout<128, CW>::bytes(G) : SdpaMmaLayout<64, CW>::bytes(G); }
 // The end of a cluster attention kernel whose warps left (m, l, o[HD]) per head where their tiles were.
 template <int HD, int CW, typename Barrier>
 __device__ __forceinline__ void sdpa_push_fold(cg::cluster_group &cluster, Barrier &&started, unsigned char *smem_att, int G, int kvh, int k_begin, int k_end, uint16_t *out, unsigned long long *tl) {
@@ -1129,7 +1115,7 @@ __global__ void __launch_bounds__(256, HD <= 128 ? 2 : 1) k_sdpa_mma_q(const FkS
     cg::cluster_group cluster = cg::this_cluster();
     const int G = a.n_q / a.n_kv, kvh = blockIdx.y, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, g = lane >> 2, t = lane & 3;
     const int rank = (int)cluster.block_rank(), CL = (int)cluster.num_blocks(), stride = HD + 2;
-    float *qsum = reinterpret_cast<float *>(smem_att + L::cpart());          // [8][NG], then [8] inverse scales: until the fold
+    float *qsum = reinterpret_cast<float *>(smem_att + L::qsum(G));          // [8][NG], then [8] inverse scales
     constexpr float OFF = BITS == 8 ? 128.0f : 8.0f;
     pdl_launch_dependents();
     auto started = cluster.barrier_arrive();

@@ -1,5 +1,5 @@
 """Attention over quantised caches with the codes as matrix operands: queries at the ends of their range (a power of two per head brings them into
-fp16), and scales that lie on odd addresses, which the kernel with global partials takes."""
+fp16), scales that lie on odd addresses, which the kernel with global partials takes, and blocks of a cluster that are done before others."""
 import math
 
 import numpy as np
@@ -14,7 +14,7 @@ pytestmark = pytest.mark.gpu
 T = N.Task.make
 
 
-def case(rt, bits, nq, nkv, hd, cap, pos, up, odd):
+def case(rt, bits, nq, nkv, hd, cap, pos, up, odd, again=0):
     """Queries times 2^up with keys' scales and biases times 2^-up: the scores stay as they are."""
     rows, per, ng = nkv * cap, 32 // bits, hd // 64
     rng = np.random.default_rng(hd + bits + pos)
@@ -29,8 +29,12 @@ def case(rt, bits, nq, nkv, hd, cap, pos, up, odd):
             6: put(ks), 7: put(kb), 8: put(vs), 9: put(vb)}
     rt.state_set(0, pos)
     rt.launch(T(N.TASK_SDPA_DECODE_QUANT, 0, bufs, [nq, nkv, hd, cap, bits], [1.0 / math.sqrt(hd)]))
+    first = rt.download(bufs[3], (nq * hd,), np.uint16)
+    for _ in range(again):
+        rt.launch(T(N.TASK_SDPA_DECODE_QUANT, 0, bufs, [nq, nkv, hd, cap, bits], [1.0 / math.sqrt(hd)]))
+        assert np.array_equal(rt.download(bufs[3], (nq * hd,), np.uint16), first)
     want = O.sdpa_decode_quant(q, kp, ks, kb, vp, vs, vb, nq, nkv, hd, cap, min(pos + 1, cap), 1.0 / math.sqrt(hd), bits)
-    assert_close_bf16(rt.download(bufs[3], (nq * hd,), np.uint16), want, f"q{bits}")
+    assert_close_bf16(first, want, f"q{bits}")
     for i, p in bufs.items():
         N.check(rt.L.fk_free(rt.h, p - 2 if odd and i >= 6 else p), "fk_free")
 
@@ -47,3 +51,13 @@ def test_queries_of_any_size(runtime, bits, nq, nkv, hd, up):
 @pytest.mark.parametrize("nq,nkv,hd", [(14, 2, 64), (28, 4, 128)])
 def test_scales_on_odd_addresses(runtime, bits, nq, nkv, hd):
     case(runtime, bits, nq, nkv, hd, 201, 150, 0, True)
+
+
+@pytest.mark.parametrize("bits", [4, 8])
+@pytest.mark.parametrize("nq,nkv,hd,cap", [(1, 1, 64, 2048), (14, 2, 64, 2048), (28, 4, 128, 2048), (4, 2, 256, 2048), (56, 8, 128, 512)])
+def test_blocks_of_a_cluster_that_finish_first(runtime, bits, nq, nkv, hd, cap):
+    """Blocks without a key, or with fewer rounds of them, hand their share over while others of the cluster (16 blocks, or 8) still read their
+    queries: every launch gives the same bits, those of the oracle's grade (``case``)."""
+    rt = runtime
+    for pos in (0, 17, 300, cap - 1):
+        case(rt, bits, nq, nkv, hd, cap, pos, 0, False, again=60)
