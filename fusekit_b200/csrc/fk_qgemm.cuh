@@ -101,7 +101,7 @@ template <int BN, bool GATEUP, bool LONG, bool CLUSTER>
 __global__ void __launch_bounds__(FKQ_THREADS, 1) k_qgemm(FkState *st, const __grid_constant__ CUtensorMap mx, QGemmArgs a) {
     using T = QgTile<BN>;
     constexpr int XS = T::XS, XG = T::XG, NBUF = T::NBUF, AS = T::AS;
-    constexpr bool SPLIT = !CLUSTER && (BN <= FKQ_SPLIT_ROWS || (LONG && BN == FKQ_MOST_ROWS));        // tiles whose parts meet in memory
+    constexpr bool SPLIT = !CLUSTER && BN <= FKQ_SPLIT_ROWS;        // tiles whose parts meet in memory
     constexpr bool LINES = !CLUSTER && T::BOX > 0;                  // .. that are stored by whole lines
     extern __shared__ unsigned char qg_smem[];
     __shared__ __align__(8) uint64_t bars[FKQ_DEQ * FK_STAGES + 2 * XS + 2 * AS + 2 * NBUF + 2];
@@ -573,43 +573,40 @@ __global__ void __launch_bounds__(FKQ_THREADS, 1) k_qgemm(FkState *st, const __g
                     }
                     store(c, c & 31, factors(c), acc, r2);
                 }
+            } else if constexpr (LINES) {
+                if (!qg_all(1 + sub, good)) return false;              // the four warps of an accumulator meet below: all of them or none
+                // 16 rows of X at a time cross shared memory, gate rows before up rows, those 16 banks on
+                float *box = reinterpret_cast<float *>(qg_smem + (ring + (uint32_t)(FKQ_DEQ * FK_STAGES * FK_UNIT_BYTES) - smem_u32(qg_smem))) + sub * 2048;
+                const int t = q * 32 + lane, up = (t >> 3) & 1, at = GATEUP ? up * 64 + (((t >> 4) * 8 + (t & 7)) ^ (up * 16)) : t;
+#pragma unroll 1
+                for (int c = 0; c < rows; c += 16) {
+                    uint32_t r[16]; qg_ld16(r, src + (uint32_t)c);
+                    asm volatile("bar.sync %0, 128;" ::"r"(1 + sub) : "memory");      // the 16 rows before are read
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) box[i * 128 + at] = __uint_as_float(r[i]);
+                    asm volatile("bar.sync %0, 128;" ::"r"(1 + sub) : "memory");
+                    lines(c, box);
+                }
             } else if (!part) {
-                if constexpr (LINES) {
-                    if (!qg_all(1 + sub, good)) return false;              // the four warps of an accumulator meet below: all of them or none
-                    // 16 rows of X at a time cross shared memory, gate rows before up rows, those 16 banks on
-                    float *box = reinterpret_cast<float *>(qg_smem + (ring + (uint32_t)(FKQ_DEQ * FK_STAGES * FK_UNIT_BYTES) - smem_u32(qg_smem))) + sub * 2048;
-                    const int t = q * 32 + lane, up = (t >> 3) & 1, at = GATEUP ? up * 64 + (((t >> 4) * 8 + (t & 7)) ^ (up * 16)) : t;
 #pragma unroll 1
-                    for (int c = 0; c < rows; c += 16) {
+                for (int cc = 0; cc < rows; cc += 32) {
+                    const float f = factors(cc);
+#pragma unroll
+                    for (int h = 0; h < (BN > 16 ? 2 : 1); ++h) {
+                        const int c = cc + 16 * h;
                         uint32_t r[16]; qg_ld16(r, src + (uint32_t)c);
-                        asm volatile("bar.sync %0, 128;" ::"r"(1 + sub) : "memory");      // the 16 rows before are read
+                        float acc[16];
 #pragma unroll
-                        for (int i = 0; i < 16; ++i) box[i * 128 + at] = __uint_as_float(r[i]);
-                        asm volatile("bar.sync %0, 128;" ::"r"(1 + sub) : "memory");
-                        lines(c, box);
-                    }
-                } else {
-#pragma unroll 1
-                    for (int cc = 0; cc < rows; cc += 32) {
-                        const float f = factors(cc);
+                        for (int i = 0; i < 16; ++i) acc[i] = __uint_as_float(r[i]);
+                        store(c, 16 * h, f, acc, res + 8 * h);
+                        if (!GATEUP) {
+                            uint32_t nx[8]; fetch(c + 32, nx);
 #pragma unroll
-                        for (int h = 0; h < (BN > 16 ? 2 : 1); ++h) {
-                            const int c = cc + 16 * h;
-                            uint32_t r[16]; qg_ld16(r, src + (uint32_t)c);
-                            float acc[16];
-#pragma unroll
-                            for (int i = 0; i < 16; ++i) acc[i] = __uint_as_float(r[i]);
-                            store(c, 16 * h, f, acc, res + 8 * h);
-                            if (!GATEUP) {
-                                uint32_t nx[8]; fetch(c + 32, nx);
-#pragma unroll
-                                for (int i = 0; i < 8; ++i) res[8 * h + i] = nx[i];
-                            }
+                            for (int i = 0; i < 8; ++i) res[8 * h + i] = nx[i];
                         }
                     }
                 }
             } else if constexpr (SPLIT) {
-                if (!good) return false;
                 const int first = fkq_owner(a.tiles, nsb, G, w.tile * nsb), last = first + fkq_parts(a.tiles, nsb, G, w.tile) - 1;
                 __threadfence();
                 __syncwarp();

@@ -75,13 +75,6 @@ inline QPlan fkq_plan(int m, int ntiles, int nsb, int sm) {
     return p;
 }
 
-// Wide tiles of long sums are dealt in equal runs of steps too where the last wave leaves blocks idle for longer than what parts that meet in memory
-// cost, three and a half steps (7B shape, 18944 -> 3584, 1000 rows: 112 tiles of 37 steps on 148 SMs, 28 steps a block).
-inline void fkq_level(QPlan &p, int nsb, int sm) {
-    if (p.whole != 1 || p.bn != FKQ_MOST_ROWS || nsb <= FKQ_SUM_STEPS || p.tiles > FKQ_COUNTERS / FKQ_EPI) return;
-    if ((double)p.tiles * nsb / sm + 3.5 < (double)((p.tiles + sm - 1) / sm) * nsb) { p.whole = 0; p.grid = (long long)p.tiles * nsb < sm ? p.tiles * nsb : sm; }
-}
-
 // A cluster of S blocks shares a tile and splits its super-blocks (grid = tiles * S, whole = -S in a plan).
 FKQ_HD inline bool fkq_cluster_work(int S, int tiles, int nsb, int b, int v, QWork &w) {      // one piece a block
     const int part = b % S;
@@ -111,4 +104,10 @@ inline bool fkq_cluster_plan(int m, int ntiles, int nsb, int sm, const int (&mos
         }
     }
     return found;
+}
+// What a product runs as.  Only tiles of up to FKQ_SPLIT_ROWS rows have parts that meet in memory: the storing warps of an accumulator give up one by one
+// there, and the four of a tile that is stored by whole lines meet at a barrier of the block.
+inline QPlan fkq_choose(int m, int ntiles, int nsb, int sm, const int (&most)[3]) {
+    QPlan p;
+    return fkq_cluster_plan(m, ntiles, nsb, sm, most, p) ? p : fkq_plan(m, ntiles, nsb, sm);
 }

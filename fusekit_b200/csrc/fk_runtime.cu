@@ -90,7 +90,7 @@ struct Ctx {
     uint32_t *pinned = nullptr;                 // host staging for state / history
     std::vector<Weight> weights; std::vector<Graph> graphs; std::vector<void *> allocs;
     bool pending = false; bool pdl = true; int sm_count = 148;
-    float *qg_scratch = nullptr, *qg_wide = nullptr; unsigned int *qg_counters = nullptr;      // of the staged products
+    float *qg_scratch = nullptr; unsigned int *qg_counters = nullptr;      // of the staged products
     float *qmm_scratch = nullptr; unsigned int *qmm_counters = nullptr;   // K-split partial sums and tickets of the several-row projection
     bool use_tiled = true; int stages = FK_STAGES; int force_warps = 0; int force_split = -1; bool qmm_tc = false; int wide_upto = 3; bool sdpa_cluster = true; bool sdpa_mma = true; int sdpa_cl = 0;
     int qg_clusters[3] = {0, 0, 0};         // of 2, 4 and 8 blocks of a staged product that are resident at once
@@ -210,7 +210,7 @@ extern "C" fk_status fk_close(fk_handle h) {
     for (unsigned char *p : c->loop_arenas) cudaFree(p);
     if (c->arena) cudaFree(c->arena);
     c->ipc_open.clear(); c->loop_arenas.clear(); c->arena = nullptr; c->peer_ready = false; c->comm = nullptr;
-    cudaFree(c->qg_scratch); cudaFree(c->qg_wide); cudaFree(c->qg_counters);
+    cudaFree(c->qg_scratch); cudaFree(c->qg_counters);
     cudaFree(c->qmm_scratch); cudaFree(c->qmm_counters);
     cudaFree(c->state); cudaFree(c->history); cudaFreeHost(c->pinned);
     cudaEventDestroy(c->ev0); cudaEventDestroy(c->ev1); cudaStreamDestroy(c->stream);
@@ -491,9 +491,8 @@ template <int BN> static cudaError_t launch_qgemm(Ctx *c, const QPlan &p, bool g
     return gateup ? launch_qgemm<BN, true>(c, p, mx, a) : launch_qgemm<BN, false>(c, p, mx, a);
 }
 // Sums and tickets of staged products that are split over K or long (20 MB): allocated before the first such product, or before a graph with
-// staged products is captured.  wide: two parts of a widest tile a block (39 MB), for products that fkq_level deals.
-static fk_status staged_scratch(Ctx *c, bool wide) {
-    if (wide && !c->qg_wide) CU(cudaMalloc(&c->qg_wide, sizeof(float) * 2 * c->sm_count * fkq_part_floats(FKQ_MOST_ROWS)));
+// staged products is captured.
+static fk_status staged_scratch(Ctx *c) {
     if (c->qg_scratch) return FK_OK;
     unsigned int *counters = nullptr; float *scratch = nullptr;
     CU(cudaMalloc(&counters, sizeof(unsigned int) * FKQ_COUNTERS));
@@ -503,20 +502,14 @@ static fk_status staged_scratch(Ctx *c, bool wide) {
     c->qg_counters = counters; c->qg_scratch = scratch;
     return FK_OK;
 }
-static QPlan staged_plan(Ctx *c, const Weight *w, int m) {
-    QPlan p;
-    if (!fkq_cluster_plan(m, w->ntiles, w->nsb, c->sm_count, c->qg_clusters, p)) { p = fkq_plan(m, w->ntiles, w->nsb, c->sm_count); fkq_level(p, w->nsb, c->sm_count); }
-    return p;
-}
-static bool staged_wide(const QPlan &p) { return !p.whole && p.bn > FKQ_SPLIT_ROWS; }
 // a product of staged rows (fk_qgemm.cuh): plain rows with a residual, or gate/up pairs with the activation
 static fk_status run_staged(Ctx *c, const Weight *w, bool gateup, const void *xs, const float *xscale, const uint16_t *residual, int ldr, uint16_t *y, int k, int n, int m, int act, cudaError_t *e, uint16_t *tail = nullptr, int from = 0) {
     if (!w || !w->finalized || !w->tiled || w->bits != 4 || w->rows_kind != (gateup ? FK_ROWS_GATE_UP : FK_ROWS_PLAIN)) return fail(FK_ERR_VALUE, "staged product: takes streamed 4-bit weights (plain rows, or gate/up pairs)");
     if (w->k != k || w->n != (gateup ? 2LL : 1LL) * n || m <= 0 || !xs || !xscale || !y || ((uintptr_t)xs & 15)) return fail(FK_ERR_VALUE, "staged product: shape mismatch");
     if (k > FKQ_MAX_K) return fail(FK_ERR_VALUE, "staged product: at most %d columns", FKQ_MAX_K);
-    const QPlan p = staged_plan(c, w, m);
-    if (!p.whole || (p.whole > 0 && w->nsb > FKQ_SUM_STEPS)) { fk_status s = staged_scratch(c, staged_wide(p)); if (s) return s; }
-    QGemmArgs a{w->tview(), xscale, residual, y, staged_wide(p) ? c->qg_wide : c->qg_scratch, c->qg_counters, w->rowmul, m, n, ldr, act, p.whole, p.mtiles, p.tiles, c->wait_limit, tail, from};
+    const QPlan p = fkq_choose(m, w->ntiles, w->nsb, c->sm_count, c->qg_clusters);
+    if (!p.whole || (p.whole > 0 && w->nsb > FKQ_SUM_STEPS)) { fk_status s = staged_scratch(c); if (s) return s; }
+    QGemmArgs a{w->tview(), xscale, residual, y, c->qg_scratch, c->qg_counters, w->rowmul, m, n, ldr, act, p.whole, p.mtiles, p.tiles, c->wait_limit, tail, from};
     CUtensorMap mx;
     if (!fkl_tensor_map(&mx, xs, m, (long long)w->nsb * FKQ_SB, (long long)w->nsb * FKQ_SB, p.bn, true)) return fail(FK_ERR_VALUE, "staged product: tensor map refused");
     *e = p.bn == 16 ? launch_qgemm<16>(c, p, gateup, mx, a) : p.bn == 32 ? launch_qgemm<32>(c, p, gateup, mx, a) : p.bn == 64 ? launch_qgemm<64>(c, p, gateup, mx, a) : launch_qgemm<128>(c, p, gateup, mx, a);
@@ -1092,12 +1085,7 @@ extern "C" fk_status fk_graph_capture(fk_handle h, const fk_task *tasks, int n, 
     if (!tasks || n <= 0 || !out) return fail(FK_ERR_VALUE, "empty task list");
     Graph g; g.tasks.assign(tasks, tasks + n);
     for (int j = 0; j < n; ++j)
-        if (tasks[j].kind == FK_TASK_STAGED_LINEAR || tasks[j].kind == FK_TASK_STAGED_GATEUP) {
-            const Weight *w = get_w(c, tasks[j].buf[2]);
-            const int m = tasks[j].iarg[2];
-            fk_status s = staged_scratch(c, w && w->finalized && m > 0 && staged_wide(staged_plan(c, w, m)));
-            if (s) return s;
-        }
+        if (tasks[j].kind == FK_TASK_STAGED_LINEAR || tasks[j].kind == FK_TASK_STAGED_GATEUP) { fk_status s = staged_scratch(c); if (s) return s; }
     CU(cudaStreamSynchronize(c->stream));
     CU(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
     fk_status s = FK_OK;

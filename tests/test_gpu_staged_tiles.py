@@ -1,4 +1,4 @@
-"""Wide tiles of staged products: stored by whole lines (results at any alignment, last rows of a tile missing), and long sums dealt in equal runs of steps."""
+"""Wide tiles of staged products: stored by whole lines (results at any alignment, last rows of a tile missing), and long sums (in stretches, or split over a cluster)."""
 import pytest
 
 from tests import test_gpu_staged_rows as R
@@ -17,11 +17,11 @@ def test_lines_of_gated_rows(runtime, m, inter):
     R.test_staged_gateup_against_64_bits(runtime, m, 512, inter)
 
 
-# 100 tiles of 11 steps, 112 of 24 (parts of one step among them), 40 of 37 over more SMs than tiles
-@pytest.mark.parametrize("m,k,n", [(200, 5632, 12800), (1000, 12288, 3584), (620, 18944, 2048)])
-def test_long_sums_in_equal_runs(runtime, m, k, n):
+# 100 tiles of 11 steps and 112 of 24, whole, in two and three stretches; 40 of 37, whose steps a cluster splits; 184 of 21 on fewer SMs
+@pytest.mark.parametrize("m,k,n", [(200, 5632, 12800), (1000, 12288, 3584), (620, 18944, 2048), (1018, 10752, 5888)])
+def test_long_sums(runtime, m, k, n):
     R.test_staged_linear_against_64_bits(runtime, m, k, n, False)
 
 
-def test_long_gated_sums_in_equal_runs(runtime):
+def test_long_gated_sums(runtime):
     R.test_staged_gateup_against_64_bits(runtime, 200, 5632, 6400)
