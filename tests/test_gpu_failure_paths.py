@@ -9,6 +9,7 @@ import pytest
 from fusekit_b200 import _native as N
 from fusekit_b200.model_spec import CONFIGS
 from fusekit_b200.runtime import DecodeEngine, Runtime
+from tests.test_staged_forms import FORMS
 
 pytestmark = pytest.mark.gpu
 
@@ -56,28 +57,42 @@ def test_seed_token_outside_the_embedding_table_is_refused_on_the_host():
 
 
 def _tensor_core_products(rt, seed):
-    """Every tcgen05 product once with its tiles whole and once split over K or spread over many blocks: (error word, results)."""
+    """Every tcgen05 product in each of its forms (staged: FORMS; row products in tiles of 64, 128 and 256 columns), and attention of many positions with one map and with
+    two: (error words, results)."""
     T, rng, out = N.Task.make, np.random.default_rng(seed), []
     bf = lambda a: (np.ascontiguousarray(a, np.float32).view(np.uint32) >> 16).astype(np.uint16)                   # noqa: E731
-    rt.state_set(0, 0)
-    for m, k, n in ((40, 1024, 512), (16, 4096, 304), (300, 512, 2560)):
+    errors = []
+
+    def fresh(nbytes):
+        p = rt.alloc(nbytes)
+        N.check(rt.L.fk_memset(rt.h, p, 0, nbytes), "fk_memset")
+        return p
+
+    for m, k, n in FORMS:
+        rt.state_set(0, 0)
         wid, x = rt.weight_alloc(n, k, 4), rt.to_device(bf(rng.normal(size=(m, k))))
         rt.weight_synth_rows(wid, 0, n, 77, 0.02, k, 0, 0); rt.weight_finalize(wid)
-        y, staged, factor = rt.alloc(m * n * 2), rt.alloc(m * -(-k // 512) * 1152), rt.alloc(m * 4)
-        N.check(rt.L.fk_memset(rt.h, y, 0, m * n * 2), "fk_memset")
+        y, staged, factor = fresh(m * n * 2), rt.alloc(m * -(-k // 512) * 1152), rt.alloc(m * 4)
         rt.launch(T(N.TASK_STAGE_ROWS, -1, {0: x, 2: staged, 3: factor}, [k, m], [1e-6]))
         rt.launch(T(N.TASK_STAGED_LINEAR, -1, {0: staged, 1: factor, 2: wid, 4: y}, [k, n, m, 0]))
         out.append(rt.download(y, (m, n), np.uint16))
-    staged_error = rt.state_get()[2]
-    rt.state_set(0, 0)
-    for m, k, n in ((40, 1024, 64), (700, 1024, 2048)):
+        errors.append((rt.state_get()[2], 0x400000))
+    for m, k, n in ((40, 1024, 64), (2048, 1024, 1024), (2048, 1024, 2304)):
+        rt.state_set(0, 0)
         wid, w = rt.weight_alloc(n, k, 16), bf(rng.normal(size=(n, k)))
         rt.weight_upload_rows(wid, 0, w); rt.weight_keep_rows(wid)
-        x, y = rt.to_device(bf(rng.normal(size=(m, k)))), rt.alloc(m * n * 4)
-        N.check(rt.L.fk_memset(rt.h, y, 0, m * n * 4), "fk_memset")
+        x, y = rt.to_device(bf(rng.normal(size=(m, k)))), fresh(m * n * 4)
         rt.launch(T(N.TASK_LINEAR_ROWS, -1, {0: x, 1: wid, 2: y}, [m, 0, n, k, n, 0, 256, 0]))
         out.append(rt.download(y, (m, n), np.float32))
-    return staged_error, rt.state_get()[2], out
+        errors.append((rt.state_get()[2], 0x200000))
+    for maps, H, rows in ((1, 3, 300), (2, 2, 300)):
+        rt.state_set(0, 0)
+        q, ck, cv = (rt.to_device(bf(rng.normal(size=s))) for s in ((rows, H * maps, 64), (maps, rows, 64), (1, rows, 128)))
+        y = fresh(rows * H * 128 * 2)
+        rt.launch(T(N.TASK_ATTENTION_ROWS, 0, {0: q, 1: ck, 2: cv, 3: y}, [H, 1, 64, 128, rows, rows, maps << 8, H], [0.125, 0.3, 0.2, 1e-5]))
+        out.append(rt.download(y, (rows, H * 128), np.uint16))
+        errors.append((rt.state_get()[2], 0x200000))
+    return errors, out
 
 
 def test_tensor_core_products_whose_waits_run_out_report_it_and_end(monkeypatch):
@@ -92,13 +107,13 @@ def test_tensor_core_products_whose_waits_run_out_report_it_and_end(monkeypatch)
         rt = Runtime(0)
         try:
             for _ in range(2):
-                staged, rows, got = _tensor_core_products(rt, 5)
+                errors, got = _tensor_core_products(rt, 5)
                 if limit is None:
-                    assert staged == 0 and rows == 0
+                    assert not any(word for word, _ in errors)
                     want = want or got
                     assert all(np.array_equal(a, b) and a.any() for a, b in zip(got, want))
                 else:
-                    assert staged & 0x400000 and rows & 0x200000
+                    assert all(word & bit for word, bit in errors), errors
                     a = np.arange(256, dtype=np.uint16)
                     assert np.array_equal(rt.smoke(a, a).shape, a.shape)
         finally:
