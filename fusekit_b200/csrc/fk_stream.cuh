@@ -36,6 +36,7 @@
 #pragma once
 #include "fk_common.cuh"
 #include "fk_attend.cuh"
+#include "fk_recip.cuh"
 
 #define FK_UNIT_VEC 288                 // uint4 per unit: 8 groups x 32 lanes + 32 scale/bias vectors (also the ring slot size)
 #define FK_UNIT_BYTES (FK_UNIT_VEC * 16)
@@ -986,19 +987,17 @@ struct SGateUpArgs {
     // copy 3 bytes per activation instead of each converting all of them (2.9 us of staging per layer on the 7B shape)
     uint32_t *dig_out; float2 *dig_xsi;
 };
-// SwiGLU of N pairs.  1 / x, x = 1 + exp(-g) from 1 on, is rounded to nearest as a division rounds it: an approximation and one Newton step in
-// fused multiply-adds (P. Markstein, IBM J. Res. Dev. 34, 1990), the same bits for every x below 2^126 (tests/test_gpu_staged_rows.py); where one of
-// a thread's values is beyond, or none, it divides.  A division has a branch of its own: N of them ran one after the other, 208 cycles each in
-// the storing warps of the staged product.
+// SwiGLU of N pairs.  1 / x, x = 1 + exp(-g) from 1 on, comes without a branch (fk_recip.cuh: the bits of a division below 2^126); where one of a thread's
+// values is beyond, or none, it divides.  A division has a branch of its own: N of them ran one after the other, 208 cycles each in the storing
+// warps of the staged product.
 template <int N> __device__ __forceinline__ void s_act_swiglu(const float (&ga)[N], const float (&ua)[N], uint16_t (&o)[N]) {
     float x[N], r[N];
     bool far = false;
 #pragma unroll
     for (int i = 0; i < N; ++i) {
         x[i] = 1.0f + expf(-rT(ga[i]));
-        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r[i]) : "f"(x[i]));
-        r[i] = fmaf(r[i], fmaf(-x[i], r[i], 1.0f), r[i]);
-        far |= !(x[i] < 8.507059e37f);
+        r[i] = recip_from_one(x[i]);
+        far |= !(x[i] < FK_RECIP_END);
     }
     if (far) {
 #pragma unroll
