@@ -254,7 +254,7 @@ class PrefillEngine(BatchDecodeEngine):
                       T(N.TASK_STAGED_GATEUP, l, {0: S["staged"], 1: S["factor"], 2: W[p + "gateup"], 4: S["act"]}, [H, I, M, N.ACT_SWIGLU])]
             tasks += product(l, S["act"], 0, I, W[p + "down"], H, S["x"], S["hb"], tail=self.x_ptr(l + 1))
         # The head in slices of rows.  The last step's rows are a slice's last ones, whose logits are stored twice (a product of their own reads all of the
-        # head for them: 0.5B shape, 100 positions, 137 -> 78 us).
+        # head for them: 0.5B shape, 100 positions, 110 -> 69 us).
         most = min(self.HEAD_ROWS, self.most[1])
         starts = sorted({final if last and r0 > final else r0 for r0 in range(0, M, most)})
         for r0, r1 in zip(starts, starts[1:] + [M]):

@@ -17,7 +17,9 @@
 //
 // Bound by the special-function unit (an exponential per score: 16 a clock and SM) and about as much by the MMAs, whose value product runs twice
 // for hi + lo.  Prompts, us, k_flash_rows before: fatulix-2048, 2048 positions (two maps of 64, values of 128) 9697 -> 7150; kakunex-5120, 1500 (window of
-// 1024) 8521 -> 8279; the 7B shape, 1000, 20870 -> 20219; the 0.5B shape, 600, 4782 -> 4621.  Errors against 64 bits agree with k_flash_rows to four digits.
+// 1024) 8521 -> 8279; the 7B shape, 1000, 20870 -> 20219; the 0.5B shape, 600, 4782 -> 4621.  Errors against 64 bits agree with k_flash_rows to seven digits,
+// results on the wrong side of their bf16 rounding 0.27 -> 0.29 % (two maps, 2048 positions), 0.22 -> 0.24 % (128 x 128, 1000), 0.82 both (64 x 64 at 6000), 4.45 both (two maps at 60000).
+// Waits: fk_tc.cuh (the eight softmax warps meet at two barriers of their own, which each of them reaches).
 #pragma once
 #include "fk_flash.cuh"
 #include "fk_tc.cuh"

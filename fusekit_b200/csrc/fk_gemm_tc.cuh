@@ -5,7 +5,7 @@
 // TMA (128-byte swizzle) into a ring of shared-memory stages, one thread of warp 1 issues tcgen05.mma (cta_group::1, M = 128,
 // N = BN, K = 16) into one of two accumulators in tensor memory, warps 4 .. 7 read finished accumulators back and store them
 // while the next tile is being multiplied.  Rows past the end of a tile's range are multiplied and not stored (past the end of
-// the tensor TMA delivers zeros).  Every wait is bounded (fk_tc.cuh).
+// the tensor TMA delivers zeros).  Waits: fk_tc.cuh.
 #pragma once
 #include "fk_layers.cuh"
 #include "fk_tc.cuh"

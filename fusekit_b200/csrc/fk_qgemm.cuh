@@ -18,7 +18,7 @@
 // and write it straight into tensor memory as the A operand (tcgen05.st .16x256b: the lane layout of the units is its lane layout; a ring
 // of four to seven k-blocks); through shared memory the expanded operand costs two more crossings of it than the packed weights.  One warp
 // fetches X by TMA (128-byte swizzle), one warp per accumulator issues its MMAs, 8 warps store finished tiles.  Weight rings are filled before
-// griddepcontrol.wait.  Every wait is bounded (fk_tc.cuh).
+// griddepcontrol.wait.  Waits: fk_tc.cuh; a storing warp gives up by itself, the four that store a tile by whole lines do together.
 //
 // Bound by the dequantising warps (a k-block and the latencies around it, 3.1 us a super-block, against 2.9 of MMAs) and by the store between tiles, under
 // which the MMAs wait.  256 x 128 tiles therefore cross shared memory 16 rows of X at a time: a warp stores whole lines of one row, factors are per

@@ -10,7 +10,7 @@
 #define FKQ_EPI 8                       // storing warps of a block
 #define FKQ_ROWS 256                    // weight rows of a block
 #define FKQ_MOST_ROWS 128               // rows of X of the widest tile
-#define FKQ_SPLIT_ROWS 32               // .. that is split over K (two parts of a block take no more scratch than a widest tile)
+#define FKQ_SPLIT_ROWS 32               // .. whose parts meet in memory (two parts of a block take no more scratch than a widest tile)
 #define FKQ_SUM_STEPS 10                // super-blocks (of 512 columns) summed in one go in tensor memory
 #define FKQ_COUNTERS 65536              // ticket words: 8 per tile that is split
 FKQ_HD inline size_t fkq_part_floats(int bn) { return (size_t)bn * FKQ_ROWS; }
@@ -59,7 +59,7 @@ template <typename Take, typename Skip> FKQ_HD inline bool fkq_pieces(int whole,
     return ok;
 }
 
-// Rows of X per tile, blocks and split of a product of m rows: the widest tile that the rows fill, a narrower one while that gives more
+// Rows of X per tile, blocks and split of a product of m rows that no cluster takes (fkq_cluster_plan): the widest tile that the rows fill, a narrower one while that gives more
 // blocks a tile of their own (a step costs a block the same up to 64 rows).  Tiles of up to 32 rows are dealt in equal runs of steps (a
 // part's sums are small, and the product is bound by the weights), wider ones whole.
 // Measured: 100 rows, 896 -> 1152: 11 us with tiles of 16 rows, 31 with one tile of 128 split over K (its fold passes 128 rows through memory);

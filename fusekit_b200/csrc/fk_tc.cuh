@@ -1,9 +1,12 @@
-// Barriers and issue helpers of the warp-specialised tcgen05 kernels (fk_gemm_tc.cuh, fk_qgemm.cuh).
+// Barriers and issue helpers of the warp-specialised tcgen05 kernels (fk_gemm_tc.cuh, fk_flash_tc.cuh, fk_qgemm.cuh).
 //
-// Every wait is bounded: TC_WAIT_LIMIT polls by default (FklEnv::wait_limit), after which the kernel sets an error bit, waits for its own
-// copies and MMAs in flight (TC_DRAIN polls at most, whatever the limit above), frees its tensor memory and returns.  A warp whose
-// lanes go on together decides together: tc_wait_warp and tc_all give all 32 lanes one answer, so that no lane leaves a loop
-// whose other lanes enter an aligned instruction or a full-mask shuffle.
+// Every wait for copies, for MMAs and for what another warp hands over is bounded: TC_WAIT_LIMIT polls by default (FklEnv::wait_limit), after which
+// the kernel sets an error bit, waits for its own copies and MMAs in flight (TC_DRAIN polls at most, whatever the limit above), frees its
+// tensor memory and returns.  A warp whose lanes go on together decides together: tc_wait_warp and tc_all give all 32 lanes one answer, so that no lane
+// leaves a loop whose other lanes enter an aligned instruction or a full-mask shuffle.
+// What cannot be counted: the allocation of tensor memory (it waits for a block on the same SM that holds some to leave, and no such block waits for the one
+// that allocates), barriers of threads of a block or a cluster (every warp reaches each of them, also after it gave up; where some would not,
+// the warps vote first: qg_all), and griddepcontrol.wait.
 #pragma once
 #include "fk_common.cuh"
 #include <cuda.h>

@@ -48,8 +48,9 @@ def test_queries_of_any_size(runtime, bits, nq, nkv, hd, up):
 
 
 @pytest.mark.parametrize("bits", [4, 8])
-@pytest.mark.parametrize("nq,nkv,hd", [(14, 2, 64), (28, 4, 128)])
+@pytest.mark.parametrize("nq,nkv,hd", [(14, 2, 64), (28, 4, 128), (4, 2, 256)])
 def test_scales_on_odd_addresses(runtime, bits, nq, nkv, hd):
+    """Rows of one group (64 dimensions) are read by themselves and may lie anywhere; those of two and four go to the kernel with global partials."""
     case(runtime, bits, nq, nkv, hd, 201, 150, 0, True)
 
 
